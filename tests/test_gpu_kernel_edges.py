@@ -1,0 +1,51 @@
+"""The forms a call is dispatched to by its sizes, at the edges of each form: the one-pass short-sequence kernel (16-key
+steps of its products, 32-column chunks, one and two 128-row tiles, its largest length and the one after it), the mask
+ring of the tensor-core kernels (chunks of 32 keys; rows on 16-byte boundaries or not), the exact kernels' tiles and
+key groups, and the 64-row steps of the tensor-core backward.  Every case against the CPU oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import cosine, from_dev_bf16, max_abs, normal_qkv, sawtooth_mask, to_dev, to_dev_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops(attn_lib):
+    import torch
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device: there is no fallback path to test")
+    from autorust_b200 import ops as _ops
+    return _ops
+
+
+def _bf16(oracle_lib, arrays):
+    return [oracle_lib.f32_to_bf16(x) for x in arrays]
+
+
+@pytest.mark.parametrize("mode,d", [("bf16", 64), ("bf16", 128), ("tf32", 64), ("sage", 128), ("sage_rows", 64)])
+@pytest.mark.parametrize("n", [1, 31, 33, 100, 127, 129, 260, 389])
+@pytest.mark.parametrize("causal", [False, True])
+def test_mask_ring(ops, oracle_lib, mode, d, n, causal):
+    """An additive mask of N(0,1) values with masked-out (-1e30) columns, its rows on 16-byte boundaries (n a multiple
+    of 4) or not; the modes' own bounds against exact attention with that mask."""
+    import torch
+    q, k, v = normal_qkv(n, 1, 2, 1, n, d)
+    mask = np.random.default_rng(n).standard_normal((n, n)).astype(np.float32)
+    mask[:, n - n // 4:] = -1e30
+    if mode == "tf32":
+        dev, exact = [to_dev(x) for x in (q, k, v)], oracle_lib.flash(0, q, k, v, mask, causal)
+    else:
+        bits = _bf16(oracle_lib, (q, k, v))
+        dev, exact = [to_dev_bf16(x) for x in bits], oracle_lib.flash(0, *map(oracle_lib.bf16_to_f32, bits), mask, causal)
+    out = ops.attn_forward(mode, *dev, to_dev(mask), causal)
+    got = out.float().cpu().numpy()
+    # the quantised modes: a row of few visible keys carries the INT8 rounding of single logits
+    bound = {"bf16": 2e-2, "tf32": 5e-3, "sage": 1e-1, "sage_rows": 1e-1}[mode]
+    assert max_abs(got, exact) <= bound and cosine(got, exact) >= 0.999
+    # the same values at an address that is 4-byte but not 16-byte aligned take the other copy width: the same bits
+    shifted = torch.cat([torch.zeros(1), torch.from_numpy(mask).flatten()]).cuda()[1:].view(n, n)
+    assert torch.equal(out, ops.attn_forward(mode, *dev, shifted, causal))
+    assert ops.last_status(None) == 0
