@@ -488,10 +488,8 @@ int ar_attn_train_forward_tc(const float* q, const float* k, const float* v, flo
   if (!device_ok()) return AR_ERR_NO_DEVICE;
   cudaStream_t stream = (cudaStream_t)cu_stream;
   uint8_t* ws = (uint8_t*)workspace;
-  if (cudaMemsetAsync(ws, 0, sizeof(uint32_t), stream) != cudaSuccess) return AR_ERR_CUDA;
-  if (ar::launch_f32_to_bf16(q, ws + L.q16, B * Hq * S * D, stream) != cudaSuccess ||
-      ar::launch_f32_to_bf16(k, ws + L.k16, B * Hkv * S * D, stream) != cudaSuccess ||
-      ar::launch_f32_to_bf16(v, ws + L.v16, B * Hkv * S * D, stream) != cudaSuccess)
+  if (ar::launch_train_convert(q, k, v, ws + L.q16, ws + L.k16, ws + L.v16, B * Hq * S * D, B * Hkv * S * D, (uint32_t*)ws,
+                               stream) != cudaSuccess)
     return AR_ERR_CUDA;
   ar::TcArgs a;
   memset(&a, 0, sizeof(a));
@@ -513,7 +511,7 @@ int ar_attn_train_forward_tc(const float* q, const float* k, const float* v, flo
       !make_map(&a.tm_v, ws + L.v16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D))
     return AR_ERR_CUDA;
   if (ar::launch_attn_tc(a, stream) != cudaSuccess) return AR_ERR_CUDA;
-  g_launches += 4;
+  g_launches += 2;
   return AR_OK;
 }
 
@@ -534,22 +532,20 @@ int ar_attn_train_backward_tc(const float* q, const float* k, const float* v, co
   if (!device_ok()) return AR_ERR_NO_DEVICE;
   cudaStream_t stream = (cudaStream_t)cu_stream;
   uint8_t* ws = (uint8_t*)workspace;
-  if (cudaMemsetAsync(ws, 0, sizeof(uint32_t), stream) != cudaSuccess) return AR_ERR_CUDA;
   int launches = 0;
-  // D_i = O_i . dO_i, and the bf16 copies of the four operands
-  if (ar::launch_train_prep(o, d_o, (float*)(ws + L.delta), B * Hq * S, (int)D, stream) != cudaSuccess) return AR_ERR_CUDA;
-  if (ar::launch_f32_to_bf16(q, ws + L.q16, B * Hq * S * D, stream) != cudaSuccess ||
-      ar::launch_f32_to_bf16(d_o, ws + L.do16, B * Hq * S * D, stream) != cudaSuccess ||
-      ar::launch_f32_to_bf16(k, ws + L.k16, B * Hkv * S * D, stream) != cudaSuccess ||
-      ar::launch_f32_to_bf16(v, ws + L.v16, B * Hkv * S * D, stream) != cudaSuccess)
+  // D_i = O_i . dO_i, the bf16 copies of the four operands, the status word cleared
+  if (ar::launch_train_prep_tc(o, d_o, (float*)(ws + L.delta), ws + L.do16, B * Hq * S, (int)D, stream) != cudaSuccess ||
+      ar::launch_train_convert(q, k, v, ws + L.q16, ws + L.k16, ws + L.v16, B * Hq * S * D, B * Hkv * S * D, (uint32_t*)ws,
+                               stream) != cudaSuccess)
     return AR_ERR_CUDA;
-  launches += 5;
+  launches += 2;
   ar::TrainBwdTcArgs a;
   memset(&a, 0, sizeof(a));
-  if (!make_map(&a.tm_q, ws + L.q16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hq, S, D) ||
-      !make_map(&a.tm_do, ws + L.do16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hq, S, D) ||
-      !make_map(&a.tm_k, ws + L.k16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D) ||
-      !make_map(&a.tm_v, ws + L.v16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D))
+  auto map64 = [&](CUtensorMap* m, const void* p, int64_t H) {  // boxes of 64 rows: the backward streams 64 at a time
+    return ar::make_tile_map(m, p, (int)CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, H, S, D, H * S * D, S * D, D, 64, 64, nullptr);
+  };
+  if (!map64(&a.tm_q, ws + L.q16, Hq) || !map64(&a.tm_do, ws + L.do16, Hq) || !map64(&a.tm_k, ws + L.k16, Hkv) ||
+      !map64(&a.tm_v, ws + L.v16, Hkv))
     return AR_ERR_CUDA;
   a.lse = lse;
   a.delta = (const float*)(ws + L.delta);

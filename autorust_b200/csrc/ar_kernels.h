@@ -102,12 +102,16 @@ struct TrainBwdArgs {
 };
 // Launches prep, dQ and dK/dV; *launches returns the number of kernels.
 cudaError_t launch_attn_train_backward(const TrainBwdArgs& a, cudaStream_t stream, int* launches);
-// delta[row] = O_row . dO_row over `rows` rows of D floats (the first kernel of the backward, on its own).
-cudaError_t launch_train_prep(const float* o, const float* d_o, float* delta, long long rows, int D, cudaStream_t stream);
+// delta[row] = O_row . dO_row over `rows` rows of D floats, and the bf16 copy of dO.
+cudaError_t launch_train_prep_tc(const float* o, const float* d_o, float* delta, void* do16, long long rows, int D,
+                                 cudaStream_t stream);
+// bf16 copies of q (nq elements), k and v (nk each; multiples of 8); clears *status.
+cudaError_t launch_train_convert(const float* q, const float* k, const float* v, void* q16, void* k16, void* v16,
+                                 long long nq, long long nk, uint32_t* status, cudaStream_t stream);
 
 // The same gradients on the tensor cores (attn_train_tc.cu): bf16 operands (copies the caller made), f32 accumulation.
 struct TrainBwdTcArgs {
-  CUtensorMap tm_q, tm_k, tm_v, tm_do;  // bf16 [B, H, S, D], box of 64 columns x 128 rows, 128-byte swizzle
+  CUtensorMap tm_q, tm_k, tm_v, tm_do;  // bf16 [B, H, S, D], box of 64 columns x 64 rows, 128-byte swizzle
   const float *lse, *delta, *mask;
   float *dq, *dk, *dv;
   int B, Hq, Hkv, S, D;

@@ -5,16 +5,26 @@
 // src/runtime/cuda_flash_train.rs:118-309) -- p = exp(s - LSE) rebuilt tile by tile, dS = p (dO.v - D_i),
 // dQ = dS K / sqrt(D), dK = dS^T Q / sqrt(D), dV = P^T dO -- but every product is a tcgen05.mma:
 //
-//   dQ kernel   one CTA per (128 queries, batch x head); per 128-key tile
+//   dQ kernel   one CTA per (128 queries, batch x head); per step of 64 keys
 //                 S = Q K^T, dP = dO V^T           (both operands K-major in shared memory, accumulators in TMEM)
 //                 dS = p (dP - D) -> bf16 in TMEM over S
 //                 dQ += dS K                       (A from TMEM, K consumed MN-major from the tile it was loaded as)
-//   dK/dV kernel one CTA per (128 keys, batch x kv head); per 128-query tile of every query head of the GQA group
+//   dK/dV kernel one CTA per (128 keys, batch x kv head); per step of 64 queries of every query head of the GQA group
 //                 S^T = K Q^T, dP^T = V dO^T       (TMEM lanes are KEYS here, so that P^T and dS^T can be A operands)
 //                 P^T, dS^T -> bf16 in TMEM
 //                 dV += P^T dO, dK += dS^T Q       (dO and Q consumed MN-major from the tiles S^T and dP^T read K-major)
 //
-// 192 threads: warps 0-3 do the element-wise part (thread = TMEM lane), warp 4 loads with TMA, warp 5 issues the MMAs.
+// One CTA per SM.  A step's scores and dP take 128 TMEM columns, and the columns that the accumulators leave hold
+// STAGES = 3 steps (2 for dK/dV at D = 128), each with an element-wise warpgroup of its own (thread = TMEM lane).  The
+// MMA warp keeps STAGES steps of S and dP issued ahead, so that the tensor pipe works on later steps while the
+// warpgroups are on theirs:  ... dQ(n), S/dP(n + STAGES), dQ(n + 1), S/dP(n + 1 + STAGES) ...  MMAs of one thread
+// execute in issue order, which is what lets S(n + STAGES) overwrite the columns dQ(n) has read.
+// Floor of a step per SM at D = 64: S and dP 384 cycles of the tensor pipe (N = 64 with both operands from shared memory
+// reads 6 KB for 32 cycles of math), dK and dV 256, and 512 cycles for 8192 exponentials.  Measured, B=4 H=16 S=2048
+// D=64: dQ 163 -> 157 us (1190 cycles per step and SM), dK/dV 254 -> 213 us (1650) against two CTAs per SM that each
+// ran S/dP -> element-wise -> dQ with nothing issued ahead; the element-wise warps wait on TMEM loads (6.4 and 4.2
+// cycles per issue), with the tensor pipe 31 % and the MUFU unit 34-44 % busy.
+//
 // No atomics: a CTA owns its output tile and walks its reduction in a fixed order, so two launches give the same
 // bits.  Operands are bf16 copies of the f32 tensors (made by the caller of these kernels); P and dS are rounded to
 // bf16 like P in the forward kernels.  On the reference test's inputs (tests/flash_train_cuda.rs:18-22) that keeps
@@ -24,395 +34,246 @@
 // exact path.
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
+#include "cta_order.cuh"
 
 namespace ar {
 namespace {
 using namespace arptx;
 
-constexpr int T = 128;  // tile edge: queries and keys
+constexpr int T = 128;  // rows a CTA owns: queries (dQ) or keys (dK/dV)
+constexpr int NH = 64;  // rows streamed per step: keys (dQ) or queries (dK/dV)
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int BWD_THREADS = 192;
 
-template <int D>
+template <int D, bool DKV>
 struct TcBwd {
   static constexpr int ROW_BYTES = D * 2;
-  static constexpr int BOXES = ROW_BYTES / 128;  // 64-column boxes of a tile
-  static constexpr int TILE_BYTES = T * ROW_BYTES;
-  static constexpr int KSTEPS_D = D / 16;        // k-steps of a product over d
-  static constexpr int KSTEPS_T = T / 16;        // k-steps of a product over 128 queries or keys
-  static constexpr int STAGES = 2;
-  static constexpr int SMEM_BYTES = (2 + 2 * STAGES) * TILE_BYTES + 2 * STAGES * T * 4 + 32 * 8 + 1024;
+  static constexpr int OWN_BYTES = T * ROW_BYTES;     // one tile of the CTA's own rows (two: Q and dO, or K and V)
+  static constexpr int STREAM_BYTES = NH * ROW_BYTES; // one streamed tile (two per step)
+  static constexpr int ACC_COLS = DKV ? 2 * D : D;    // TMEM columns of the gradient accumulators
+  static constexpr int STAGES = (512 - ACC_COLS) / (2 * NH) < 3 ? (512 - ACC_COLS) / (2 * NH) : 3;
+  static constexpr int SLOTS = D == 64 ? 6 : 4;       // streamed steps in shared memory; STAGES + 1 keep the MMAs fed
+  static_assert(SLOTS > STAGES, "a slot beyond the steps in flight");
+  static constexpr int ROWVALS_BYTES = STAGES * 2 * 2 * NH * 4;  // dK/dV: LSE and D_i of a step's queries, double-buffered
+  static constexpr int NUM_BARS = 2 + 2 * SLOTS + 2 * STAGES;
+  static constexpr int SMEM_BYTES = 2 * OWN_BYTES + SLOTS * 2 * STREAM_BYTES + ROWVALS_BYTES + NUM_BARS * 8 + 16 + 1024;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-  // D = 64: a tile of 128 keys (dQ kernel) or 128 queries (dK/dV kernel) is walked in two halves of 64, so that the
-  // scores, dP and the accumulators of a CTA fit 256 TMEM columns and two CTAs share an SM -- one CTA's MMAs and
-  // waits run under the other's element-wise pass.  D = 128: one step per tile, one CTA per SM (shared memory).
-  static constexpr int HALVES = D == 64 ? 2 : 1;
-  static constexpr int NH = T / HALVES;              // score columns per step
-  static constexpr int TMEM_COLS = HALVES == 2 ? 256 : 512;
-  static constexpr int MIN_CTAS = HALVES;
-  static_assert(HALVES == 1 || 2 * SMEM_BYTES <= 226 * 1024, "two CTAs must fit an SM");
-  static constexpr int KSTEPS_NH = NH / 16;          // k-steps of a product over one step's queries or keys
+  static constexpr int KSTEPS_D = D / 16;             // k-steps of a product over d
+  static constexpr int KSTEPS_NH = NH / 16;           // k-steps of a product over one step's rows
   static constexpr uint32_t IDESC_SS = make_idesc(1, 1, 1, 0, 0, T, NH);  // bf16 x bf16 -> f32, both K-major, N = NH
   static constexpr uint32_t IDESC_TS = make_idesc(1, 1, 1, 0, 1, T, D);   // A from TMEM, B MN-major, N = D
+  static constexpr int W_PROD = 4 * STAGES, W_MMA = W_PROD + 1;           // two more warps complete the last warpgroup
+  static constexpr int NUM_THREADS = 128 * STAGES + 128;
+  // registers per thread: launched with LAUNCH_REGS, then moved from the last warpgroup to the element-wise ones
+  static constexpr int LAUNCH_REGS = STAGES == 3 ? 128 : 168;
+  static constexpr int EW_REGS = STAGES == 3 ? 144 : 208;
+  static constexpr int SERVICE_REGS = STAGES == 3 ? 80 : 88;
+  static_assert(128 * STAGES * EW_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
+  static_assert(LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
 };
 
-// D[tmem, 128 x NH] = A[128 x D] B_half[NH x D]^T, both tiles K-major (rows of 128-byte boxes, 128-byte swizzle);
-// `half` selects rows half * NH ... of the B tile
-template <int D>
-__device__ __forceinline__ void mma_abt(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, int half) {
+// D[tmem, 128 x NH] = A[128 x D] B[NH x D]^T, both tiles K-major (rows of 128-byte boxes, 128-byte swizzle)
+template <int D, bool DKV>
+__device__ __forceinline__ void mma_abt(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi) {
   if (!elect_one()) return;
-  const uint32_t b_half = b_lo + (uint32_t)((half * TcBwd<D>::NH * 128) >> 4);
 #pragma unroll
-  for (int s = 0; s < TcBwd<D>::KSTEPS_D; s++) {
-    const uint32_t off = ((s >> 2) * (T * 128) + (s & 3) * 32) >> 4;
-    mma_ss_lohi<KIND_F16>(d_tmem, a_lo + off, hi, b_half + off, hi, TcBwd<D>::IDESC_SS, s > 0);
+  for (int s = 0; s < TcBwd<D, DKV>::KSTEPS_D; s++) {
+    const uint32_t a = a_lo + (((s >> 2) * (T * 128) + (s & 3) * 32) >> 4);
+    const uint32_t b = b_lo + (((s >> 2) * (NH * 128) + (s & 3) * 32) >> 4);
+    mma_ss_lohi<KIND_F16>(d_tmem, a, hi, b, hi, TcBwd<D, DKV>::IDESC_SS, s > 0);
   }
 }
-// D[tmem, 128 x D] (+)= A[tmem, 128 x NH bf16] B_half[NH x D], B consumed MN-major from a row-major tile (rows
-// half * NH ... of it)
-template <int D>
-__device__ __forceinline__ void mma_tb(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, bool acc, int half) {
+// D[tmem, 128 x D] (+)= A[tmem, 128 x NH bf16] B[NH x D], B consumed MN-major from a row-major tile
+template <int D, bool DKV>
+__device__ __forceinline__ void mma_tb(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, bool acc) {
   if (!elect_one()) return;
-  const uint32_t b_half = b_lo + (uint32_t)(half * TcBwd<D>::KSTEPS_NH) * (2048 >> 4);
 #pragma unroll
-  for (int s = 0; s < TcBwd<D>::KSTEPS_NH; s++)
-    mma_ts_lohi<KIND_F16>(d_tmem, a_tmem + s * 8, b_half + s * (2048 >> 4), b_hi, TcBwd<D>::IDESC_TS, (acc || s > 0) ? 1u : 0u);
+  for (int s = 0; s < TcBwd<D, DKV>::KSTEPS_NH; s++)
+    mma_ts_lohi<KIND_F16>(d_tmem, a_tmem + s * 8, b_lo + s * (2048 >> 4), b_hi, TcBwd<D, DKV>::IDESC_TS,
+                          (acc || s > 0) ? 1u : 0u);
 }
 
-// One [128 x D] bf16 tile of a [B, H, S, D] tensor into shared memory (boxes of 64 columns).
+// `rows` (64 or 128) rows of D bf16 from a [B, H, S, D] tensor into a tile of boxes of 64 columns; the maps' boxes are
+// 64 rows high.
 template <int D>
-__device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int row0, int head, int b) {
-  for (int bx = 0; bx < TcBwd<D>::BOXES; bx++) tma_load_4d(dst + bx * (T * 128), m, bar, bx * 64, row0, head, b);
+__device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int rows, int row0, int head,
+                                          int b) {
+  for (int bx = 0; bx < D / 64; bx++)
+    for (int r = 0; r < rows; r += NH) tma_load_4d(dst + (bx * rows + r) * 128, m, bar, bx * 64, row0 + r, head, b);
 }
 
-// ------------------------------------------------------------------------------------------------ dQ
-template <int D>
-__global__ void __launch_bounds__(BWD_THREADS, TcBwd<D>::MIN_CTAS)
-train_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                   const float* __restrict__ LSE, const float* __restrict__ delta, const float* __restrict__ mask,
-                   float* __restrict__ dQ, int N, int Hq, int Hkv, int causal, uint32_t* status, uint32_t* sticky) {
-  using C = TcBwd<D>;
-  constexpr int ST = C::STAGES;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQ = smem;
-  uint8_t* sdO = sQ + C::TILE_BYTES;
-  uint8_t* sK = sdO + C::TILE_BYTES;
-  uint8_t* sV = sK + ST * C::TILE_BYTES;
-  uint64_t* bars = (uint64_t*)(sV + ST * C::TILE_BYTES + 2 * ST * T * 4);
-  uint64_t* qdo_full = bars;            // Q and dO tiles landed
-  uint64_t* kv_full = qdo_full + 1;     // [ST]
-  uint64_t* kv_empty = kv_full + ST;    // [ST]
-  uint64_t* s_full = kv_empty + ST;     // S and dP of a key tile complete
-  uint64_t* ds_full = s_full + 1;       // dS written by the 128 threads
-  uint64_t* acc_full = ds_full + 1;     // every MMA complete
-  uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
-  volatile uint32_t* abort_flag = tmem_slot + 1;
-  const WaitCtx wctx{abort_flag, status, sticky};
-
-  const int tid = threadIdx.x;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int lane = tid & 31;
-  const int bh = blockIdx.y, b = bh / Hq, h = bh - b * Hq, kvh = h / (Hq / Hkv);
-  const int q0 = blockIdx.x * T;
-  const int nkt_all = (N + T - 1) / T;
-  const int nkt = causal ? min(nkt_all, blockIdx.x + 1) : nkt_all;  // key tiles this query tile sees
-
-  if (warp == 4 && lane == 0) {
-    *abort_flag = 0;
-    mbar_init(qdo_full, 1);
-    mbar_init(s_full, 1);
-    mbar_init(ds_full, 128);
-    mbar_init(acc_full, 1);
-    for (int i = 0; i < ST; i++) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-    }
-    fence_mbar_init();
-  }
-  if (warp == 5) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tb = *tmem_slot;
-  constexpr int HV = C::HALVES, NH = C::NH;
-  const uint32_t col_S = 0, col_dP = NH, col_dQ = 2 * NH;
-
-  if (warp == 4) {
-    if (lane == 0) {
-      mbar_arrive_expect_tx(qdo_full, 2 * C::TILE_BYTES);
-      load_rows<D>(sQ, &tm_q, qdo_full, q0, h, b);
-      load_rows<D>(sdO, &tm_do, qdo_full, q0, h, b);
-      int issued = 0;
-      for (int j = 0; j < nkt; j++) {
-        const int s = j % ST;
-        if (j >= ST && !mbar_wait(&kv_empty[s], ((j / ST) - 1) & 1, wctx, 0x50)) break;
-        mbar_arrive_expect_tx(&kv_full[s], 2 * C::TILE_BYTES);
-        load_rows<D>(sK + s * C::TILE_BYTES, &tm_k, &kv_full[s], j * T, kvh, b);
-        load_rows<D>(sV + s * C::TILE_BYTES, &tm_v, &kv_full[s], j * T, kvh, b);
-        issued = j + 1;
-      }
-      if (*abort_flag) {  // let what was started land before the shared memory goes back
-        mbar_wait_quiet(qdo_full, 0);
-        for (int j = max(0, issued - ST); j < issued; j++) mbar_wait_quiet(&kv_full[j % ST], (j / ST) & 1);
-      }
-    }
-  } else if (warp == 5) {
-    const uint64_t k_proto = make_sdesc_sw128(0, 16, 1024);       // K-major
-    const uint64_t mn_proto = make_sdesc_sw128(0, T * 128, 1024);  // MN-major: 64-column boxes T * 128 bytes apart
-    const uint32_t k_hi = (uint32_t)(k_proto >> 32), mn_hi = (uint32_t)(mn_proto >> 32);
-    const uint32_t q_lo = (uint32_t)k_proto | (smem_u32(sQ) >> 4), do_lo = (uint32_t)k_proto | (smem_u32(sdO) >> 4);
-    bool ok = __all_sync(0xffffffffu, mbar_wait(qdo_full, 0, wctx, 0x51));
-    for (int j = 0; j < nkt && ok; j++) {
-      const int s = j % ST;
-      ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[s], (j / ST) & 1, wctx, 0x52));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t kt = smem_u32(sK + s * C::TILE_BYTES) >> 4, vt = smem_u32(sV + s * C::TILE_BYTES) >> 4;
-      for (int hf = 0; hf < HV && ok; hf++) {  // the tile's keys in steps of NH
-        mma_abt<D>(tb + col_S, q_lo, (uint32_t)k_proto | kt, k_hi, hf);    // S = Q K^T
-        mma_abt<D>(tb + col_dP, do_lo, (uint32_t)k_proto | vt, k_hi, hf);  // dP = dO V^T
-        commit_one(s_full);
-        ok = __all_sync(0xffffffffu, mbar_wait(ds_full, (j * HV + hf) & 1, wctx, 0x53));
-        if (!ok) break;
-        tc_fence_after();
-        mma_tb<D>(tb + col_dQ, tb + col_S, (uint32_t)mn_proto | kt, mn_hi, j > 0 || hf > 0, hf);  // dQ += dS K
-      }
-      if (!ok) break;
-      commit_one(&kv_empty[s]);
-    }
-    if (ok) commit_one(acc_full);
-  } else {
-    // element-wise: thread r owns query row q0 + r
-    const int r = tid;
-    const int row = q0 + r;
-    const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
-    const uint32_t tS = tmem_addr(tb, lane_base, col_S), tdP = tmem_addr(tb, lane_base, col_dP);
-    const float scale_log2 = (1.0f / sqrtf((float)D)) * LOG2E;
-    const float lse2 = row < N ? LSE[(size_t)bh * N + row] * LOG2E : 0.f;
-    const float dl = row < N ? delta[(size_t)bh * N + row] : 0.f;
-    const float* mrow = (mask != nullptr && row < N) ? mask + (size_t)row * N : nullptr;
-    bool ok = true;
-    for (int g = 0; g < nkt * HV; g++) {  // steps of NH keys
-      const int j = g / HV, hf = g - j * HV;
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full, g & 1, wctx, 0x54));
-      if (!ok) break;
-      tc_fence_after();
-      // a step whose 128 x NH block lies inside the sequence, below the causal diagonal and under no additive mask
-      // needs none of the per-element tests: two lanes per instruction
-      const int colh = j * T + hf * NH;
-      const bool interior = mask == nullptr && colh + NH <= N && q0 + T <= N && (!causal || colh + NH - 1 <= q0);
-#pragma unroll 1
-      for (int c = 0; c < NH / 32; c++) {
-        uint32_t sv[32], pv[32], pk[16];
-        tmem_ld32(tS + c * 32, sv);
-        tmem_ld32(tdP + c * 32, pv);
-        tmem_wait_ld();
-        if (interior) {
-          const uint64_t sc2 = pack_f32x2(scale_log2, scale_log2), nl2 = pack_f32x2(-lse2, -lse2),
-                         ndl2 = pack_f32x2(-dl, -dl);
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float a, b2;
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sc2, nl2), a, b2);
-            const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(pv[i]), __uint_as_float(pv[i + 1])), ndl2);
-            float d0, d1;
-            unpack_f32x2(mul_f32x2(pack_f32x2(ex2f(a), ex2f(b2)), d2), d0, d1);
-            pk[i >> 1] = pack_bf16x2(d0, d1);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float ds[2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-              const int col = colh + c * 32 + i + e;
-              float x = __uint_as_float(sv[i + e]) * scale_log2;
-              if (mrow != nullptr && col < N) x = fmaf(mrow[col], LOG2E, x);
-              const bool out = col >= N || row >= N || (causal && col > row);
-              const float p = out ? 0.f : ex2f(x - lse2);
-              ds[e] = p * (__uint_as_float(pv[i + e]) - dl);
-            }
-            pk[i >> 1] = pack_bf16x2(ds[0], ds[1]);
-          }
-        }
-        tmem_st16(tS + c * 16, pk);  // dS over the columns of S that have been read
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(ds_full);
-    }
-    if (ok && nkt > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wctx, 0x55));
-    if (ok) {
-      tc_fence_after();
-      const float scale = 1.0f / sqrtf((float)D);
-      const uint32_t tQ = tmem_addr(tb, lane_base, col_dQ);
-#pragma unroll 1
-      for (int c = 0; c < D / 32; c++) {
-        uint32_t ov[32];
-        if (nkt > 0) {
-          tmem_ld32(tQ + c * 32, ov);
-          tmem_wait_ld();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i++) ov[i] = 0u;
-        }
-        if (row < N) {
-          float4* dst = (float4*)(dQ + ((size_t)bh * N + row) * D + c * 32);
-#pragma unroll
-          for (int i = 0; i < 8; i++)
-            dst[i] = make_float4(__uint_as_float(ov[4 * i]) * scale, __uint_as_float(ov[4 * i + 1]) * scale,
-                                 __uint_as_float(ov[4 * i + 2]) * scale, __uint_as_float(ov[4 * i + 3]) * scale);
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 5) tmem_dealloc(tb, C::TMEM_COLS);
-}
-
-// --------------------------------------------------------------------------------------------- dK, dV
-template <int D>
-__global__ void __launch_bounds__(BWD_THREADS, TcBwd<D>::MIN_CTAS)
-train_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+// dQ (DKV = false): own rows are queries (A tiles Q, dO), K and V stream.  dK/dV (DKV = true): own rows are keys (A
+// tiles K, V), Q and dO of the group's query heads stream.
+template <int D, bool DKV>
+__global__ void __launch_bounds__(TcBwd<D, DKV>::NUM_THREADS, 1)
+train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const float* __restrict__ LSE, const float* __restrict__ delta, const float* __restrict__ mask,
-                    float* __restrict__ dK, float* __restrict__ dV, int N, int Hq, int Hkv, int causal, uint32_t* status,
-                    uint32_t* sticky) {
-  using C = TcBwd<D>;
-  constexpr int ST = C::STAGES;
+                    float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int head_group, int causal,
+                    uint32_t* status, uint32_t* sticky) {
+  using C = TcBwd<D, DKV>;
+  constexpr int ST = C::STAGES, SL = C::SLOTS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + C::TILE_BYTES;
-  uint8_t* sQ = sV + C::TILE_BYTES;
-  uint8_t* sdO = sQ + ST * C::TILE_BYTES;
-  float* s_lse = (float*)(sdO + ST * C::TILE_BYTES);  // [2][T]: log-sum-exp (log2 domain) of the item's query rows
-  float* s_dl = s_lse + 2 * T;                        // [2][T]: D_i of the same rows
-  uint64_t* bars = (uint64_t*)(s_dl + 2 * T);
-  uint64_t* kv_full = bars;
-  uint64_t* qd_full = kv_full + 1;     // [ST]
-  uint64_t* qd_empty = qd_full + ST;   // [ST]
-  uint64_t* s_full = qd_empty + ST;    // S^T and dP^T complete
-  uint64_t* p_full = s_full + 1;       // P^T and dS^T written
-  uint64_t* acc_full = p_full + 1;
-  uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+  uint8_t* own0 = smem;                               // Q | K
+  uint8_t* own1 = own0 + C::OWN_BYTES;                // dO | V
+  uint8_t* ring = own1 + C::OWN_BYTES;                // per slot: K, V | Q, dO
+  float* rowvals = (float*)(ring + SL * 2 * C::STREAM_BYTES);
+  uint64_t* bars = (uint64_t*)((uint8_t*)rowvals + C::ROWVALS_BYTES);
+  uint64_t* own_full = bars;
+  uint64_t* acc_full = own_full + 1;                  // every MMA complete
+  uint64_t* slot_full = acc_full + 1;                 // [SL]
+  uint64_t* slot_empty = slot_full + SL;              // [SL]
+  uint64_t* s_full = slot_empty + SL;                 // [ST] S and dP of a step complete
+  uint64_t* p_full = s_full + ST;                     // [ST] dS (and P) written by the stage's 128 threads
+  uint32_t* tmem_slot = (uint32_t*)(p_full + ST);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const WaitCtx wctx{abort_flag, status, sticky};
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int kvbh = blockIdx.y, b = kvbh / Hkv, kvh = kvbh - b * Hkv;
-  const int G = Hq / Hkv;
-  const int k0 = blockIdx.x * T;
-  const int nqt_all = (N + T - 1) / T;
-  const int i_first = causal ? (int)blockIdx.x : 0;  // query tiles before the diagonal see none of these keys
-  const int per_head = nqt_all - i_first;
-  const int items = G * per_head;                    // (query head of the group, query tile), in that order
+  int tile, bh;
+  cta_order(head_group, tile, bh);
+  // dQ under a causal mask: the last query tile sees the most keys; dK/dV: the first key tile sees the most queries
+  if (!DKV && causal) tile = (int)gridDim.x - 1 - tile;
+  const int H = DKV ? Hkv : Hq, G = Hq / Hkv;
+  const int b = bh / H, h = bh - b * H;               // DKV: h is a kv head
+  const int row0 = tile * T;
+  // the steps this tile walks: dQ -- blocks of 64 keys; dK/dV -- blocks of 64 queries, head by head of the group
+  const int first = DKV && causal ? row0 / NH : 0;    // queries before the key tile see none of it
+  const int last = !DKV && causal ? (min(N, row0 + T) + NH - 1) / NH : (N + NH - 1) / NH;
+  const int per_head = last - first;
+  const int steps = DKV ? G * per_head : per_head;
 
-  if (warp == 4 && lane == 0) {
+  if (warp == C::W_PROD && lane == 0) {
     *abort_flag = 0;
-    mbar_init(kv_full, 1);
-    mbar_init(s_full, 1);
-    mbar_init(p_full, 128);
+    mbar_init(own_full, 1);
     mbar_init(acc_full, 1);
+    for (int i = 0; i < SL; i++) {
+      mbar_init(&slot_full[i], 1);
+      mbar_init(&slot_empty[i], 1);
+    }
     for (int i = 0; i < ST; i++) {
-      mbar_init(&qd_full[i], 1);
-      mbar_init(&qd_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 128);
     }
     fence_mbar_init();
   }
-  if (warp == 5) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
+  if (warp == C::W_MMA) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tb = *tmem_slot;
-  constexpr int HV = C::HALVES, NH = C::NH;
-  const uint32_t col_S = 0, col_dP = NH, col_dV = 2 * NH, col_dK = 2 * NH + D;
+  const uint32_t col_acc = ST * 2 * NH;               // accumulators: dQ | dV, dK
 
-  if (warp == 4) {
+  if (warp >= C::W_PROD) setmaxnreg_dec<C::SERVICE_REGS>();
+  if (warp == C::W_PROD) {
     if (lane == 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * C::TILE_BYTES);
-      load_rows<D>(sK, &tm_k, kv_full, k0, kvh, b);
-      load_rows<D>(sV, &tm_v, kv_full, k0, kvh, b);
+      const int own_h = h;
+      mbar_arrive_expect_tx(own_full, 2 * C::OWN_BYTES);
+      load_rows<D>(own0, DKV ? &tm_k : &tm_q, own_full, T, row0, own_h, b);
+      load_rows<D>(own1, DKV ? &tm_v : &tm_do, own_full, T, row0, own_h, b);
       int issued = 0;
-      for (int it = 0; it < items; it++) {
-        const int s = it % ST;
-        const int g = it / per_head, i = i_first + (it - g * per_head);
-        if (it >= ST && !mbar_wait(&qd_empty[s], ((it / ST) - 1) & 1, wctx, 0x58)) break;
-        mbar_arrive_expect_tx(&qd_full[s], 2 * C::TILE_BYTES);
-        load_rows<D>(sQ + s * C::TILE_BYTES, &tm_q, &qd_full[s], i * T, kvh * G + g, b);
-        load_rows<D>(sdO + s * C::TILE_BYTES, &tm_do, &qd_full[s], i * T, kvh * G + g, b);
-        issued = it + 1;
+      for (int n = 0; n < steps; n++) {
+        const int sl = n % SL;
+        const int g = DKV ? n / per_head : 0;
+        const int r = (first + n - g * per_head) * NH;
+        const int sh = DKV ? h * G + g : h / G;       // head of the streamed tensors
+        if (n >= SL && !mbar_wait(&slot_empty[sl], ((n / SL) - 1) & 1, wctx, 0x50)) break;
+        uint8_t* dst = ring + sl * 2 * C::STREAM_BYTES;
+        mbar_arrive_expect_tx(&slot_full[sl], 2 * C::STREAM_BYTES);
+        load_rows<D>(dst, DKV ? &tm_q : &tm_k, &slot_full[sl], NH, r, sh, b);
+        load_rows<D>(dst + C::STREAM_BYTES, DKV ? &tm_do : &tm_v, &slot_full[sl], NH, r, sh, b);
+        issued = n + 1;
       }
-      if (*abort_flag) {
-        mbar_wait_quiet(kv_full, 0);
-        for (int it = max(0, issued - ST); it < issued; it++) mbar_wait_quiet(&qd_full[it % ST], (it / ST) & 1);
+      if (*abort_flag) {  // let what was started land before the shared memory goes back
+        mbar_wait_quiet(own_full, 0);
+        for (int n = max(0, issued - SL); n < issued; n++) mbar_wait_quiet(&slot_full[n % SL], (n / SL) & 1);
       }
     }
-  } else if (warp == 5) {
-    const uint64_t k_proto = make_sdesc_sw128(0, 16, 1024);
-    const uint64_t mn_proto = make_sdesc_sw128(0, T * 128, 1024);
+  } else if (warp == C::W_MMA) {
+    const uint64_t k_proto = make_sdesc_sw128(0, 16, 1024);         // K-major
+    const uint64_t mn_proto = make_sdesc_sw128(0, NH * 128, 1024);  // MN-major: 64-column boxes NH * 128 bytes apart
     const uint32_t k_hi = (uint32_t)(k_proto >> 32), mn_hi = (uint32_t)(mn_proto >> 32);
-    const uint32_t k_lo = (uint32_t)k_proto | (smem_u32(sK) >> 4), v_lo = (uint32_t)k_proto | (smem_u32(sV) >> 4);
-    bool ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, wctx, 0x59));
-    for (int it = 0; it < items && ok; it++) {
-      const int s = it % ST;
-      ok = __all_sync(0xffffffffu, mbar_wait(&qd_full[s], (it / ST) & 1, wctx, 0x5a));
+    const uint32_t a0 = (uint32_t)k_proto | (smem_u32(own0) >> 4), a1 = (uint32_t)k_proto | (smem_u32(own1) >> 4);
+    const uint32_t ring0 = smem_u32(ring) >> 4;
+    bool ok = __all_sync(0xffffffffu, mbar_wait(own_full, 0, wctx, 0x51));
+    auto scores = [&](int n) {  // S and dP of step n into its stage
+      const int st = n % ST;
+      if (!__all_sync(0xffffffffu, mbar_wait(&slot_full[n % SL], (n / SL) & 1, wctx, 0x52))) return false;
+      tc_fence_after();
+      const uint32_t x = ring0 + (n % SL) * (2 * C::STREAM_BYTES >> 4), y = x + (C::STREAM_BYTES >> 4);
+      mma_abt<D, DKV>(tb + st * 2 * NH, a0, (uint32_t)k_proto | x, k_hi);       // S = Q K^T     | S^T = K Q^T
+      mma_abt<D, DKV>(tb + st * 2 * NH + NH, a1, (uint32_t)k_proto | y, k_hi);  // dP = dO V^T   | dP^T = V dO^T
+      commit_one(&s_full[st]);
+      return true;
+    };
+    for (int n = 0; n < min(ST, steps) && ok; n++) ok = scores(n);
+    for (int n = 0; n < steps && ok; n++) {
+      const int st = n % ST;
+      ok = __all_sync(0xffffffffu, mbar_wait(&p_full[st], (n / ST) & 1, wctx, 0x53));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t qt = smem_u32(sQ + s * C::TILE_BYTES) >> 4, dot = smem_u32(sdO + s * C::TILE_BYTES) >> 4;
-      for (int hf = 0; hf < HV && ok; hf++) {  // the tile's queries in steps of NH
-        mma_abt<D>(tb + col_S, k_lo, (uint32_t)k_proto | qt, k_hi, hf);    // S^T = K Q^T
-        mma_abt<D>(tb + col_dP, v_lo, (uint32_t)k_proto | dot, k_hi, hf);  // dP^T = V dO^T
-        commit_one(s_full);
-        ok = __all_sync(0xffffffffu, mbar_wait(p_full, (it * HV + hf) & 1, wctx, 0x5b));
-        if (!ok) break;
-        tc_fence_after();
-        mma_tb<D>(tb + col_dV, tb + col_S, (uint32_t)mn_proto | dot, mn_hi, it > 0 || hf > 0, hf);  // dV += P^T dO
-        mma_tb<D>(tb + col_dK, tb + col_dP, (uint32_t)mn_proto | qt, mn_hi, it > 0 || hf > 0, hf);  // dK += dS^T Q
+      const uint32_t x = ring0 + (n % SL) * (2 * C::STREAM_BYTES >> 4), y = x + (C::STREAM_BYTES >> 4);
+      const uint32_t s_cols = tb + st * 2 * NH, p_cols = s_cols + NH;
+      if constexpr (DKV) {
+        mma_tb<D, DKV>(tb + col_acc, s_cols, (uint32_t)mn_proto | y, mn_hi, n > 0);      // dV += P^T dO
+        mma_tb<D, DKV>(tb + col_acc + D, p_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);  // dK += dS^T Q
+      } else {
+        mma_tb<D, DKV>(tb + col_acc, s_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);      // dQ += dS K
       }
-      if (!ok) break;
-      commit_one(&qd_empty[s]);
+      commit_one(&slot_empty[n % SL]);
+      if (n + ST < steps) ok = scores(n + ST);
     }
     if (ok) commit_one(acc_full);
-  } else {
-    // element-wise: thread r owns key k0 + r
-    const int r = tid;
-    const int key = k0 + r;
+  } else if (warp < C::W_PROD) {
+    // element-wise: warpgroup wg takes steps wg, wg + STAGES, ...; thread r owns the CTA's row row0 + r
+    setmaxnreg_inc<C::EW_REGS>();
+    const int wg = warp >> 2;
+    const int r = tid & 127;
+    const int row = row0 + r;
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
-    const uint32_t tS = tmem_addr(tb, lane_base, col_S), tdP = tmem_addr(tb, lane_base, col_dP);
+    const uint32_t tS = tmem_addr(tb, lane_base, wg * 2 * NH), tdP = tS + NH;
     const float scale_log2 = (1.0f / sqrtf((float)D)) * LOG2E;
+    const uint64_t sc2 = pack_f32x2(scale_log2, scale_log2);
+    // dQ: this query's -LSE (log2 domain) and -D_i
+    float nlse = 0.f, ndl = 0.f;
+    if (!DKV && row < N) {
+      nlse = -LSE[(size_t)bh * N + row] * LOG2E;
+      ndl = -delta[(size_t)bh * N + row];
+    }
+    // dK/dV: the same of the step's 64 queries, through shared memory; threads 0-63 bring LSE, 64-127 D_i, one step of
+    // this warpgroup ahead
+    float* vals = rowvals + wg * (2 * 2 * NH);
+    auto fetch = [&](int n) {
+      const int g = n / per_head, qrow = (first + n - g * per_head) * NH + (r & (NH - 1));
+      if (n >= steps || qrow >= N) return 0.f;
+      const size_t at = (size_t)(b * Hq + h * G + g) * N + qrow;
+      return r < NH ? -LSE[at] * LOG2E : -delta[at];
+    };
+    float next_val = 0.f;
+    if constexpr (DKV) next_val = fetch(wg);
     bool ok = true;
-    for (int it = 0; it < items; it++) {
-      const int g = it / per_head, i = i_first + (it - g * per_head);
-      const int bhq = b * Hq + kvh * G + g;
-      // the item's per-query values: every thread brings one, all 128 read them
-      {
-        const int qrow = i * T + r;
-        s_lse[(it & 1) * T + r] = qrow < N ? -LSE[(size_t)bhq * N + qrow] * LOG2E : 0.f;  // (negated: added below)
-        s_dl[(it & 1) * T + r] = qrow < N ? -delta[(size_t)bhq * N + qrow] : 0.f;
+    int it = 0;
+    for (int n = wg; n < steps; n += ST, it++) {
+      const float* lv = vals + (it & 1) * (2 * NH);  // [NH] -LSE, [NH] -D_i
+      if constexpr (DKV) {
+        vals[(it & 1) * (2 * NH) + r] = next_val;
+        next_val = fetch(n + ST);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float* nlse2 = s_lse + (it & 1) * T;
-      const float* ndl = s_dl + (it & 1) * T;
-      for (int hf = 0; hf < HV && ok; hf++) {
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full, (it * HV + hf) & 1, wctx, 0x5c));
+      const int g = DKV ? n / per_head : 0;
+      const int c0 = (first + n - g * per_head) * NH;  // first streamed row: key (dQ) or query (dK/dV)
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[wg], it & 1, wctx, 0x54));
       if (!ok) break;
       tc_fence_after();
-      // a step whose 128 keys x NH queries lie inside the sequence, on the visible side of the causal diagonal and
-      // under no additive mask needs none of the per-element tests: two lanes per instruction
-      const int qh = i * T + hf * NH;
-      const bool interior = mask == nullptr && k0 + T <= N && qh + NH <= N && (!causal || k0 + T - 1 <= qh);
+      // a step whose 128 x 64 block lies inside the sequence, on the visible side of the causal diagonal and under no
+      // additive mask needs none of the per-element tests: two lanes per instruction
+      const bool interior = mask == nullptr && row0 + T <= N && c0 + NH <= N &&
+                            (!causal || (DKV ? row0 + T - 1 <= c0 : c0 + NH - 1 <= row0));
 #pragma unroll 1
       for (int c = 0; c < NH / 32; c++) {
         uint32_t sv[32], pv[32], pk[16], dk[16];
@@ -420,117 +281,172 @@ train_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_ld32(tdP + c * 32, pv);
         tmem_wait_ld();
         if (interior) {
-          const uint64_t sc2 = pack_f32x2(scale_log2, scale_log2);
-          const float2* nl = reinterpret_cast<const float2*>(nlse2 + hf * NH + c * 32);
-          const float2* nd = reinterpret_cast<const float2*>(ndl + hf * NH + c * 32);
 #pragma unroll
-          for (int e2 = 0; e2 < 32; e2 += 2) {
-            const float2 l = nl[e2 >> 1], dd = nd[e2 >> 1];
-            float a, b2;
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[e2]), __uint_as_float(sv[e2 + 1])), sc2,
-                                   pack_f32x2(l.x, l.y)), a, b2);
-            const float p0 = ex2f(a), p1 = ex2f(b2);
-            const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(pv[e2]), __uint_as_float(pv[e2 + 1])),
-                                          pack_f32x2(dd.x, dd.y));
-            float d0, d1;
-            unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), d2), d0, d1);
-            pk[e2 >> 1] = pack_bf16x2(p0, p1);
-            dk[e2 >> 1] = pack_bf16x2(d0, d1);
+          for (int i = 0; i < 32; i += 4) {
+            float4 l = make_float4(nlse, nlse, nlse, nlse), d = make_float4(ndl, ndl, ndl, ndl);
+            if constexpr (DKV) {
+              l = *(const float4*)(lv + c * 32 + i);
+              d = *(const float4*)(lv + NH + c * 32 + i);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              float x0, x1, d0, d1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i + e]), __uint_as_float(sv[i + e + 1])), sc2,
+                                     e ? pack_f32x2(l.z, l.w) : pack_f32x2(l.x, l.y)), x0, x1);
+              const float p0 = ex2f(x0), p1 = ex2f(x1);
+              const uint64_t t2 = add_f32x2(pack_f32x2(__uint_as_float(pv[i + e]), __uint_as_float(pv[i + e + 1])),
+                                            e ? pack_f32x2(d.z, d.w) : pack_f32x2(d.x, d.y));
+              unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), t2), d0, d1);
+              if constexpr (DKV) pk[(i + e) >> 1] = pack_bf16x2(p0, p1);
+              dk[(i + e) >> 1] = pack_bf16x2(d0, d1);
+            }
           }
         } else {
 #pragma unroll
-        for (int e2 = 0; e2 < 32; e2 += 2) {
-          float p[2], ds[2];
+          for (int i = 0; i < 32; i += 2) {
+            float p[2], ds[2];
 #pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int cc = hf * NH + c * 32 + e2 + e;
-            const int qrow = i * T + cc;
-            float x = __uint_as_float(sv[e2 + e]) * scale_log2;
-            if (mask != nullptr && qrow < N && key < N) x = fmaf(mask[(size_t)qrow * N + key], LOG2E, x);
-            const bool out = key >= N || qrow >= N || (causal && key > qrow);
-            p[e] = out ? 0.f : ex2f(x + nlse2[cc]);
-            ds[e] = p[e] * (__uint_as_float(pv[e2 + e]) + ndl[cc]);
+            for (int e = 0; e < 2; e++) {
+              const int cc = c * 32 + i + e;
+              const int key = DKV ? row : c0 + cc, qrow = DKV ? c0 + cc : row;
+              const float l = DKV ? lv[cc] : nlse, d = DKV ? lv[NH + cc] : ndl;
+              float x = __uint_as_float(sv[i + e]) * scale_log2;
+              if (mask != nullptr && qrow < N && key < N) x = fmaf(mask[(size_t)qrow * N + key], LOG2E, x);
+              const bool out = key >= N || qrow >= N || (causal && key > qrow);
+              p[e] = out ? 0.f : ex2f(x + l);
+              ds[e] = p[e] * (__uint_as_float(pv[i + e]) + d);
+            }
+            if constexpr (DKV) pk[i >> 1] = pack_bf16x2(p[0], p[1]);
+            dk[i >> 1] = pack_bf16x2(ds[0], ds[1]);
           }
-          pk[e2 >> 1] = pack_bf16x2(p[0], p[1]);
-          dk[e2 >> 1] = pack_bf16x2(ds[0], ds[1]);
         }
+        // over the columns that have been read: dS | P^T over S^T, dS^T over dP^T
+        if constexpr (DKV) {
+          tmem_st16(tS + c * 16, pk);
+          tmem_st16(tdP + c * 16, dk);
+        } else {
+          tmem_st16(tS + c * 16, dk);
         }
-        tmem_st16(tS + c * 16, pk);   // P^T over the columns of S^T that have been read
-        tmem_st16(tdP + c * 16, dk);  // dS^T likewise over dP^T
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(p_full);
-      }
-      if (!ok) break;
+      mbar_arrive(&p_full[wg]);
     }
-    if (ok && items > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wctx, 0x5d));
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wctx, 0x55));
     if (ok) {
       tc_fence_after();
       const float scale = 1.0f / sqrtf((float)D);
+      // the accumulators' 32-column chunks, shared out over the warpgroups
 #pragma unroll 1
-      for (int which = 0; which < 2; which++) {
-        const uint32_t tA = tmem_addr(tb, lane_base, which ? col_dK : col_dV);
-        float* base = (which ? dK : dV) + ((size_t)kvbh * N + key) * D;
-        const float f = which ? scale : 1.0f;
-#pragma unroll 1
-        for (int c = 0; c < D / 32; c++) {
-          uint32_t ov[32];
-          if (items > 0) {
-            tmem_ld32(tA + c * 32, ov);
-            tmem_wait_ld();
-          } else {
+      for (int c = wg; c < C::ACC_COLS / 32; c += ST) {
+        const bool second = DKV && c >= D / 32;  // dV first, then dK
+        const int cd = second ? c - D / 32 : c;
+        const float f = DKV && !second ? 1.0f : scale;
+        uint32_t ov[32];
+        tmem_ld32(tmem_addr(tb, lane_base, col_acc + c * 32), ov);
+        tmem_wait_ld();
+        if (row < N) {
+          float4* dst = (float4*)((second ? out1 : out0) + ((size_t)bh * N + row) * D + cd * 32);
 #pragma unroll
-            for (int i = 0; i < 32; i++) ov[i] = 0u;
-          }
-          if (key < N) {
-            float4* dst = (float4*)(base + c * 32);
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-              dst[i] = make_float4(__uint_as_float(ov[4 * i]) * f, __uint_as_float(ov[4 * i + 1]) * f,
-                                   __uint_as_float(ov[4 * i + 2]) * f, __uint_as_float(ov[4 * i + 3]) * f);
-          }
+          for (int i = 0; i < 8; i++)
+            dst[i] = make_float4(__uint_as_float(ov[4 * i]) * f, __uint_as_float(ov[4 * i + 1]) * f,
+                                 __uint_as_float(ov[4 * i + 2]) * f, __uint_as_float(ov[4 * i + 3]) * f);
         }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) tmem_dealloc(tb, C::TMEM_COLS);
+  if (warp == C::W_MMA) tmem_dealloc(tb, 512);
 }
 
+// delta[row] = O_row . dO_row and the bf16 copy of dO in one pass over both: D / 4 lanes per row.
 template <int D>
-cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream, int* launches) {
-  using C = TcBwd<D>;
-  auto dq_kern = train_dq_tc_kernel<D>;
-  auto dkv_kern = train_dkv_tc_kernel<D>;
+__global__ void __launch_bounds__(256) train_prep_tc_kernel(const float* __restrict__ O, const float* __restrict__ dO,
+                                                            float* __restrict__ delta, uint2* __restrict__ dO16,
+                                                            long long rows) {
+  constexpr int LPR = D / 4;
+  const long long at = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long row = at / LPR;
+  float acc = 0.f;
+  if (row < rows) {
+    const float4 a = ((const float4*)O)[at], g = ((const float4*)dO)[at];
+    acc = fmaf(a.w, g.w, fmaf(a.z, g.z, fmaf(a.y, g.y, a.x * g.x)));
+    dO16[at] = make_uint2(pack_bf16x2(g.x, g.y), pack_bf16x2(g.z, g.w));
+  }
+#pragma unroll
+  for (int sh = LPR / 2; sh > 0; sh >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sh);
+  if (row < rows && threadIdx.x % LPR == 0) delta[row] = acc;
+}
+
+// bf16 copies of q, k and v in one launch, and the launch's status word cleared on the way (the attention kernels that
+// follow on the stream want it zero).
+__global__ void __launch_bounds__(256) train_convert_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                            const float* __restrict__ v, uint4* __restrict__ q16,
+                                                            uint4* __restrict__ k16, uint4* __restrict__ v16,
+                                                            long long nq8, long long nk8, uint32_t* status) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0u;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < nq8 + 2 * nk8; i += (long long)gridDim.x * 256) {
+    const float* src = i < nq8 ? q : i < nq8 + nk8 ? k : v;
+    uint4* dst = i < nq8 ? q16 : i < nq8 + nk8 ? k16 : v16;
+    const long long at = i < nq8 ? i : i < nq8 + nk8 ? i - nq8 : i - nq8 - nk8;
+    const float4 a = *(const float4*)(src + at * 8), c = *(const float4*)(src + at * 8 + 4);
+    dst[at] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(c.x, c.y), pack_bf16x2(c.z, c.w));
+  }
+}
+
+template <int D, bool DKV>
+cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
+  using C = TcBwd<D, DKV>;
+  auto kern = train_bwd_tc_kernel<D, DKV>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(dq_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(dkv_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int tiles = (a.S + T - 1) / T;
-  dq_kern<<<dim3(tiles, a.B * a.Hq, 1), BWD_THREADS, C::SMEM_BYTES, stream>>>(
-      a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv, a.causal, a.status, a.sticky);
-  (*launches)++;
-  dkv_kern<<<dim3(tiles, a.B * a.Hkv, 1), BWD_THREADS, C::SMEM_BYTES, stream>>>(
-      a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv, a.causal, a.status, a.sticky);
-  (*launches)++;
+  const int heads = a.B * (DKV ? a.Hkv : a.Hq), group = a.Hq / a.Hkv;
+  // bf16 bytes that stream past a tile: Q and dO of the group's heads, or the shared K and V
+  const size_t head_bytes = (size_t)a.S * D * 4 * (DKV ? group : 1) / (DKV ? 1 : group);
+  kern<<<dim3((a.S + T - 1) / T, heads, 1), C::NUM_THREADS, C::SMEM_BYTES, stream>>>(
+      a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask, DKV ? a.dv : a.dq, DKV ? a.dk : nullptr, a.S, a.Hq, a.Hkv,
+      head_group_for(head_bytes, heads, (long long)((a.S + T - 1) / T) * heads), a.causal, a.status, a.sticky);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_attn_train_backward_tc(const TrainBwdTcArgs& a, cudaStream_t stream, int* launches) {
-  if (a.D == 64) return launch_bwd_tc<64>(a, stream, launches);
-  if (a.D == 128) return launch_bwd_tc<128>(a, stream, launches);
-  return cudaErrorInvalidValue;
+  if (a.D != 64 && a.D != 128) return cudaErrorInvalidValue;
+  cudaError_t e = a.D == 64 ? launch_bwd_tc<64, false>(a, stream) : launch_bwd_tc<128, false>(a, stream);
+  if (e != cudaSuccess) return e;
+  (*launches)++;
+  e = a.D == 64 ? launch_bwd_tc<64, true>(a, stream) : launch_bwd_tc<128, true>(a, stream);
+  if (e != cudaSuccess) return e;
+  (*launches)++;
+  return cudaSuccess;
+}
+
+cudaError_t launch_train_prep_tc(const float* o, const float* d_o, float* delta, void* do16, long long rows, int D,
+                                 cudaStream_t stream) {
+  const unsigned blocks = (unsigned)((rows * (D / 4) + 255) / 256);
+  if (D == 64)
+    train_prep_tc_kernel<64><<<blocks, 256, 0, stream>>>(o, d_o, delta, (uint2*)do16, rows);
+  else
+    train_prep_tc_kernel<128><<<blocks, 256, 0, stream>>>(o, d_o, delta, (uint2*)do16, rows);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_train_convert(const float* q, const float* k, const float* v, void* q16, void* k16, void* v16,
+                                 long long nq, long long nk, uint32_t* status, cudaStream_t stream) {
+  const long long n8 = nq / 8 + 2 * (nk / 8);
+  const long long blocks = (n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16;
+  train_convert_kernel<<<(unsigned)blocks, 256, 0, stream>>>(q, k, v, (uint4*)q16, (uint4*)k16, (uint4*)v16, nq / 8, nk / 8,
+                                                             status);
+  return cudaGetLastError();
 }
 
 }  // namespace ar

@@ -49,3 +49,31 @@ def test_mask_ring(ops, oracle_lib, mode, d, n, causal):
     shifted = torch.cat([torch.zeros(1), torch.from_numpy(mask).flatten()]).cuda()[1:].view(n, n)
     assert torch.equal(out, ops.attn_forward(mode, *dev, shifted, causal))
     assert ops.last_status(None) == 0
+
+
+@pytest.mark.parametrize("tc", [False, True])
+@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321),
+                                        (5, 30, 30, 130)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_training_steps(ops, oracle_lib, tc, b, hq, hkv, n, d, causal):
+    """Fewer steps than stages, ragged tiles, several query heads per K/V head, and enough rows for the 128-row exact
+    kernels.  Exact: 2e-5 of the largest entry, as the training tests hold it; bf16 operands: 1e-2 of it."""
+    import torch
+    rng = np.random.default_rng(n)
+    q, k, v = normal_qkv(n, b, hq, hkv, n, d)
+    d_o = rng.standard_normal(q.shape, dtype=np.float32)
+    mask = sawtooth_mask(n) if n == 129 else None
+    want = dict(zip(("o", "lse", "dq", "dk", "dv"), oracle_lib.attn_train(q, k, v, d_o, mask, causal)))
+    tq, tk, tv, tdo = map(to_dev, (q, k, v, d_o))
+    tm = None if mask is None else to_dev(mask)
+    o, lse = ops.train_forward(tq, tk, tv, tm, causal, tensor_cores=tc)
+    grads = ops.train_backward(tq, tk, tv, o, tdo, lse, tm, causal, tensor_cores=tc)
+    again = ops.train_backward(tq, tk, tv, o, tdo, lse, tm, causal, tensor_cores=tc)
+    for name, got in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, *grads)):
+        w = want[name]
+        bound = (2e-2 if tc else 2e-5) * max(1.0, float(np.abs(w).max()))
+        assert max_abs(got.cpu().numpy(), w) <= bound, (name, max_abs(got.cpu().numpy(), w), bound)
+    for x, y in zip(grads, again):  # no atomics: two launches give the same bits
+        assert torch.equal(x, y)
+    assert ops.last_status(None) == 0
