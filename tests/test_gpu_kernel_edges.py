@@ -51,6 +51,20 @@ def test_mask_ring(ops, oracle_lib, mode, d, n, causal):
     assert ops.last_status(None) == 0
 
 
+@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 12, 12, 197), (1, 2, 2, 64), (1, 2, 2, 65), (2, 74, 74, 130),
+                                        (1, 148, 74, 257), (1, 2, 2, 1100)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_exact_tiles(ops, oracle_lib, b, hq, hkv, n, d, causal):
+    """Calls on both sides of the tile rule (16-row tiles for few rows, 128- or 64-row ones for many), the key groups
+    with more groups than tiles; 1e-5 of the largest value as for the exact mode elsewhere."""
+    q, k, v = normal_qkv(n, b, hq, hkv, n, d)
+    mask = sawtooth_mask(n) if n == 65 else None
+    got = ops.attn_forward("exact", *map(to_dev, (q, k, v)), None if mask is None else to_dev(mask), causal).cpu().numpy()
+    want = oracle_lib.flash(0, q, k, v, mask, causal)
+    assert np.all(np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1.0))
+
+
 @pytest.mark.parametrize("tc", [False, True])
 @pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321),
                                         (5, 30, 30, 130)])
