@@ -10,7 +10,12 @@
 // matrix, every thread a 4 x 4 block of it (rows ty*4+i, keys tx+16*jj, as in the forward) for the two products that
 // rebuild p and dS, and a 4 x D/16 block of the gradient tile for the product that accumulates it.  f32 on the FFMA
 // pipe throughout: this is the path held to the graph's autograd, not a tensor-core path.
+// At D = 64, where the tiles of 128 rows fit, calls with enough rows take the kernels with 8 x 8 blocks per thread (the
+// _wide ones): four d of a 4 x 4 block read 8 x 16 bytes of shared memory per thread (32 cycles per warp and SM) for 16
+// cycles of FFMA, an 8 x 8 block 64 for 64.
 #include "ar_kernels.h"
+#include "ar_ptx.cuh"
+#include "cta_order.cuh"
 
 namespace ar {
 namespace {
@@ -111,7 +116,7 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
                                                        const float* __restrict__ V, const float* __restrict__ dO,
                                                        const float* __restrict__ LSE, const float* __restrict__ delta,
                                                        const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq,
-                                                       int Hkv, int causal) {
+                                                       int Hkv, int head_group, int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
   float* sQ = smem_t;
@@ -122,10 +127,12 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int bh = blockIdx.y;
+  int tile, bh;
+  cta_order(head_group, tile, bh);
+  if (causal) tile = (int)gridDim.x - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
-  const int q0 = blockIdx.x * BT;
+  const int q0 = tile * BT;
   const float scale = 1.0f / sqrtf((float)D);
   constexpr int OD = D / 64;
   load_tile<D>(sQ, Q + (size_t)bh * N * D, q0, N, tid);
@@ -199,7 +206,8 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
                                                         const float* __restrict__ V, const float* __restrict__ dO,
                                                         const float* __restrict__ LSE, const float* __restrict__ delta,
                                                         const float* __restrict__ M, float* __restrict__ dK,
-                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int causal) {
+                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int head_group,
+                                                        int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
   float* sK = smem_t;
@@ -211,10 +219,11 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int kvbh = blockIdx.y;
+  int tile, kvbh;
+  cta_order(head_group, tile, kvbh);  // (under a causal mask the first key tile sees the most queries)
   const int b = kvbh / Hkv, hk = kvbh - b * Hkv;
   const int group = Hq / Hkv;
-  const int k0 = blockIdx.x * BT;
+  const int k0 = tile * BT;
   const float scale = 1.0f / sqrtf((float)D);
   constexpr int OD = D / 64;
   load_tile<D>(sK, K + (size_t)kvbh * N * D, k0, N, tid);
@@ -290,6 +299,302 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
   }
 }
 
+// ---------------------------------------------------------------- D = 64, 8 x 8 blocks
+namespace wide {
+using namespace arptx;
+constexpr int D = 64, LD = D + 4;  // padded row (floats): 16-byte aligned, conflict-free float4 reads
+constexpr int OWN = 128;           // rows a CTA owns
+constexpr int STREAM = 64;         // rows of a streamed tile
+constexpr int LDS_DQ = STREAM + 8;    // dS row of the dQ kernel: a warp's 4 rows x 8 keys fall into different banks
+constexpr int LDS_DKV = OWN + 16;     // P and dS rows of the dK/dV kernel: 2 rows x 16 keys
+constexpr int DQ_GROUP = 2 * STREAM * LD + OWN * LDS_DQ;  // floats: K, V, dS of one group
+constexpr int DQ_SMEM = (2 * OWN * LD + 2 * DQ_GROUP) * 4;
+constexpr int DKV_STAGE = 2 * STREAM * LD + 2 * STREAM;   // Q, dO, LSE, D_i of one query tile
+constexpr int DKV_SMEM = (2 * OWN * LD + 2 * DKV_STAGE + 2 * STREAM * LDS_DKV) * 4;
+static_assert(DQ_SMEM <= 227 * 1024 && DKV_SMEM <= 227 * 1024, "shared memory budget");
+static_assert(128 * 64 <= DQ_GROUP, "a group's dQ passes through its own tiles");
+
+// `rows` rows of a [.., N, D] tensor into a padded tile by `threads` threads; rows past the end become zeros
+__device__ __forceinline__ void load_async(float* dst, const float* src, int rows, int row0, int N, int t, int threads) {
+#pragma unroll 4
+  for (int i = t; i < rows * (D / 4); i += threads) {
+    const int r = i / (D / 4), c = i % (D / 4);
+    const bool in = row0 + r < N;
+    cp_async16(smem_u32(dst + r * LD + c * 4), in ? src + (size_t)(row0 + r) * D + c * 4 : src, in);
+  }
+}
+
+// s[i][jj] = A[(ra + RA * i)] . B[(rb + RB * jj)] over d
+template <int RA, int RB>
+__device__ __forceinline__ void product(const float* sA, const float* sB, int ra, int rb, float (&s)[8][8]) {
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int jj = 0; jj < 8; jj++) s[i][jj] = 0.f;
+#pragma unroll 1
+  for (int d4 = 0; d4 < D / 4; d4++) {
+    float4 bv[8];
+#pragma unroll
+    for (int jj = 0; jj < 8; jj++) bv[jj] = *(const float4*)(sB + (rb + RB * jj) * LD + d4 * 4);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float4 av = *(const float4*)(sA + (ra + RA * i) * LD + d4 * 4);
+#pragma unroll
+      for (int jj = 0; jj < 8; jj++) {
+        s[i][jj] = fmaf(av.x, bv[jj].x, s[i][jj]);
+        s[i][jj] = fmaf(av.y, bv[jj].y, s[i][jj]);
+        s[i][jj] = fmaf(av.z, bv[jj].z, s[i][jj]);
+        s[i][jj] = fmaf(av.w, bv[jj].w, s[i][jj]);
+      }
+    }
+  }
+}
+
+// p of one element from its raw product
+__device__ __forceinline__ float prob(float s, float scale, const float* __restrict__ M, int row, int key, int N, int causal,
+                                      float lse) {
+  float x = s * scale;
+  if (M != nullptr && row < N && key < N) x += M[(size_t)row * N + key];
+  return key >= N || row >= N || (causal && key > row) ? 0.f : expf(x - lse);
+}
+
+// dQ: one CTA per (128 queries, batch x head); two groups of 128 threads take the key tiles of 64 in turn, each with a
+// dQ of its own (8 rows x 8 columns per thread); group 0 adds the two.
+__global__ void __launch_bounds__(256, 1)
+    train_dq_wide_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
+                         const float* __restrict__ dO, const float* __restrict__ LSE, const float* __restrict__ delta,
+                         const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq, int Hkv, int head_group,
+                         int causal) {
+  extern __shared__ __align__(16) float smem_t[];
+  const int tid = threadIdx.x, grp = tid >> 7, gt = tid & 127;
+  const int tx = gt & 7, ty = gt >> 3;  // rows ty + 16 * i, keys tx + 8 * jj, columns (tx + 8 * dd) * 4 ..
+  float* sQ = smem_t;
+  float* sdO = sQ + OWN * LD;
+  float* sK = sdO + OWN * LD + grp * DQ_GROUP;
+  float* sV = sK + STREAM * LD;
+  float* sDS = sV + STREAM * LD;
+  int tile, bh;
+  cta_order(head_group, tile, bh);
+  if (causal) tile = (int)gridDim.x - 1 - tile;  // the last query tile sees the most keys
+  const int b = bh / Hq, h = bh - b * Hq;
+  const size_t kv = (size_t)(b * Hkv + h / (Hq / Hkv)) * N * D;
+  const int q0 = tile * OWN;
+  const float scale = 1.0f / sqrtf((float)D);
+  const int tiles = ((causal ? min(N, q0 + OWN) : N) + STREAM - 1) / STREAM;
+  load_async(sQ, Q + (size_t)bh * N * D, OWN, q0, N, tid, 256);
+  load_async(sdO, dO + (size_t)bh * N * D, OWN, q0, N, tid, 256);
+  load_async(sK, K + kv, STREAM, grp * STREAM, N, gt, 128);
+  load_async(sV, V + kv, STREAM, grp * STREAM, N, gt, 128);
+  cp_async_commit();
+  float lse[8], dl[8], acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int row = q0 + ty + 16 * i;
+    lse[i] = row < N ? LSE[(size_t)bh * N + row] : 0.f;
+    dl[i] = row < N ? delta[(size_t)bh * N + row] : 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[i][c] = 0.f;
+  }
+  auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int kt = grp; kt < tiles; kt += 2) {
+    const int k0 = kt * STREAM;
+    cp_async_wait<0>();
+    group_sync();
+    float p[8][8], t[8][8];
+    product<16, 8>(sQ, sK, ty, tx, p);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int jj = 0; jj < 8; jj++)
+        p[i][jj] = prob(p[i][jj], scale, M, q0 + ty + 16 * i, k0 + tx + 8 * jj, N, causal, lse[i]);
+    product<16, 8>(sdO, sV, ty, tx, t);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int jj = 0; jj < 8; jj++) sDS[(ty + 16 * i) * LDS_DQ + tx + 8 * jj] = p[i][jj] * (t[i][jj] - dl[i]);
+    group_sync();  // dS is complete and V consumed
+    load_async(sV, V + kv, STREAM, min(k0 + 2 * STREAM, N), N, gt, 128);
+    cp_async_commit();
+    // dQ += dS . K
+#pragma unroll 2
+    for (int k4 = 0; k4 < STREAM / 4; k4++) {
+      float4 kr[4][2];
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++)
+#pragma unroll
+        for (int dd = 0; dd < 2; dd++) kr[kk][dd] = *(const float4*)(sK + (k4 * 4 + kk) * LD + (tx + 8 * dd) * 4);
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const float4 ds = *(const float4*)(sDS + (ty + 16 * i) * LDS_DQ + k4 * 4);
+#pragma unroll
+        for (int kk = 0; kk < 4; kk++) {
+          const float w = kk == 0 ? ds.x : kk == 1 ? ds.y : kk == 2 ? ds.z : ds.w;
+#pragma unroll
+          for (int dd = 0; dd < 2; dd++) {
+            acc[i][dd * 4 + 0] = fmaf(w, kr[kk][dd].x, acc[i][dd * 4 + 0]);
+            acc[i][dd * 4 + 1] = fmaf(w, kr[kk][dd].y, acc[i][dd * 4 + 1]);
+            acc[i][dd * 4 + 2] = fmaf(w, kr[kk][dd].z, acc[i][dd * 4 + 2]);
+            acc[i][dd * 4 + 3] = fmaf(w, kr[kk][dd].w, acc[i][dd * 4 + 3]);
+          }
+        }
+      }
+    }
+    group_sync();  // K and dS are consumed
+    load_async(sK, K + kv, STREAM, min(k0 + 2 * STREAM, N), N, gt, 128);
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  float* mine = sK + gt;
+  if (grp == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int c = 0; c < 8; c++) mine[(i * 8 + c) * 128] = acc[i][c];
+  }
+  __syncthreads();
+  if (grp == 1) return;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int row = q0 + ty + 16 * i;
+    if (row >= N) continue;
+    const float* other = mine + DQ_GROUP + i * 8 * 128;
+#pragma unroll
+    for (int dd = 0; dd < 2; dd++)
+      *(float4*)(dQ + ((size_t)bh * N + row) * D + (tx + 8 * dd) * 4) =
+          make_float4((acc[i][dd * 4 + 0] + other[(dd * 4 + 0) * 128]) * scale, (acc[i][dd * 4 + 1] + other[(dd * 4 + 1) * 128]) * scale,
+                      (acc[i][dd * 4 + 2] + other[(dd * 4 + 2) * 128]) * scale, (acc[i][dd * 4 + 3] + other[(dd * 4 + 3) * 128]) * scale);
+  }
+}
+
+// dK, dV: one CTA per (128 keys, batch x kv head), walking the query tiles of 64 of every query head of the group in a
+// fixed order.  Threads 0-127 rebuild p and accumulate dV = P^T dO, threads 128-255 form dS from their dO.V and that p
+// and accumulate dK = dS^T Q, so that each holds one 8 x 8 block of scores and one of gradients.  The next query tile
+// arrives under this one's products.
+__global__ void __launch_bounds__(256, 1)
+    train_dkv_wide_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
+                          const float* __restrict__ dO, const float* __restrict__ LSE, const float* __restrict__ delta,
+                          const float* __restrict__ M, float* __restrict__ dK, float* __restrict__ dV, int N, int Hq, int Hkv,
+                          int head_group, int causal) {
+  extern __shared__ __align__(16) float smem_t[];
+  const int tid = threadIdx.x, half = tid >> 7, ht = tid & 127;
+  const int tx = ht & 15, ty = ht >> 4;  // scores: queries ty + 8 * i, keys tx + 16 * jj
+  const int cx = ht & 7, ky = ht >> 3;   // gradients: keys ky * 8 + i, columns (cx + 8 * dd) * 4 ..
+  float* sK = smem_t;
+  float* sV = sK + OWN * LD;
+  float* stages = sV + OWN * LD;
+  float* sP = stages + 2 * DKV_STAGE;
+  float* sDS = sP + STREAM * LDS_DKV;
+  int tile, kvbh;
+  cta_order(head_group, tile, kvbh);  // (under a causal mask the first key tile sees the most queries)
+  const int b = kvbh / Hkv, hk = kvbh - b * Hkv, group = Hq / Hkv;
+  const int k0 = tile * OWN;
+  const float scale = 1.0f / sqrtf((float)D);
+  const int first = causal ? k0 / STREAM : 0;  // queries before the key tile see none of it
+  const int per_head = (N + STREAM - 1) / STREAM - first;
+  const int steps = group * per_head;
+  auto load_step = [&](int n) {
+    if (n < steps) {
+      const int g = n / per_head, r0 = (first + n - g * per_head) * STREAM;
+      const size_t bh = (size_t)(b * Hq + hk * group + g);
+      float* st = stages + (n & 1) * DKV_STAGE;
+      load_async(st, Q + bh * N * D, STREAM, r0, N, tid, 256);
+      load_async(st + STREAM * LD, dO + bh * N * D, STREAM, r0, N, tid, 256);
+      if (tid < 2 * STREAM) {
+        const int r = r0 + (tid & (STREAM - 1));
+        const float* src = tid < STREAM ? LSE : delta;
+        cp_async4(smem_u32(st + 2 * STREAM * LD + tid), r < N ? src + bh * N + r : src, r < N);
+      }
+    }
+    cp_async_commit();
+  };
+  load_async(sK, K + (size_t)kvbh * N * D, OWN, k0, N, tid, 256);
+  load_async(sV, V + (size_t)kvbh * N * D, OWN, k0, N, tid, 256);
+  load_step(0);
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[i][c] = 0.f;
+  for (int n = 0; n < steps; n++) {
+    load_step(n + 1);
+    cp_async_wait<1>();
+    __syncthreads();  // this step's tiles (and K, V) are in place
+    const int g = n / per_head, q0 = (first + n - g * per_head) * STREAM;
+    const float* sQ = stages + (n & 1) * DKV_STAGE;
+    const float* sdO = sQ + STREAM * LD;
+    const float* sL = sdO + STREAM * LD;
+    float s[8][8];
+    product<8, 16>(half ? sdO : sQ, half ? sV : sK, ty, tx, s);
+    if (half == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int jj = 0; jj < 8; jj++)
+          sP[(ty + 8 * i) * LDS_DKV + tx + 16 * jj] =
+              prob(s[i][jj], scale, M, q0 + ty + 8 * i, k0 + tx + 16 * jj, N, causal, sL[ty + 8 * i]);
+    }
+    __syncthreads();  // P is in place
+    if (half == 1) {
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int jj = 0; jj < 8; jj++) {
+          const int at = (ty + 8 * i) * LDS_DKV + tx + 16 * jj;
+          sDS[at] = sP[at] * (s[i][jj] - sL[STREAM + ty + 8 * i]);
+        }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
+    const float* sW = half ? sDS : sP;
+    const float* sX = half ? sQ : sdO;
+#pragma unroll 4
+    for (int q = 0; q < STREAM; q++) {
+      const float4 w0 = *(const float4*)(sW + q * LDS_DKV + ky * 8), w1 = *(const float4*)(sW + q * LDS_DKV + ky * 8 + 4);
+      const float4 x0 = *(const float4*)(sX + q * LD + cx * 4), x1 = *(const float4*)(sX + q * LD + (cx + 8) * 4);
+      const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+      const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) acc[i][c] = fmaf(w[i], x[c], acc[i][c]);
+    }
+    __syncthreads();  // this step's tiles, P and dS are consumed
+  }
+  cp_async_wait<0>();
+  float* out = half ? dK : dV;
+  const float f = half ? scale : 1.0f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int key = k0 + ky * 8 + i;
+    if (key >= N) continue;
+#pragma unroll
+    for (int dd = 0; dd < 2; dd++)
+      *(float4*)(out + ((size_t)kvbh * N + key) * D + (cx + 8 * dd) * 4) =
+          make_float4(acc[i][dd * 4] * f, acc[i][dd * 4 + 1] * f, acc[i][dd * 4 + 2] * f, acc[i][dd * 4 + 3] * f);
+  }
+}
+
+cudaError_t configure() {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev < 64 && configured[dev])) return e;
+  e = cudaFuncSetAttribute(train_dq_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(train_dkv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM);
+  if (e == cudaSuccess && dev < 64) configured[dev] = true;
+  return e;
+}
+
+// The 128-row tiles take one CTA per SM, the 64-row ones work at about 0.6 of their rate: the form that ends first.
+bool worth_it(int S, int heads) {
+  const long long w = (long long)((S + 127) / 128) * heads, n = (long long)((S + 63) / 64) * heads;
+  return ((w + 147) / 148) * 128 * 6 <= ((n + 147) / 148) * 64 * 10;
+}
+}  // namespace wide
+
 template <int D>
 cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches) {
   using C = BwdCfg<D>;
@@ -311,11 +616,28 @@ cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches
   train_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(a.o, a.d_o, a.delta, rows, D);
   (*launches)++;
   const int tiles = (a.S + BT - 1) / BT;
-  dq_kern<<<dim3(tiles, a.B * a.Hq, 1), 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
-                                                                  a.Hq, a.Hkv, a.causal);
+  const bool wide_dq = D == 64 && wide::worth_it(a.S, a.B * a.Hq), wide_dkv = D == 64 && wide::worth_it(a.S, a.B * a.Hkv);
+  if (wide_dq || wide_dkv) {
+    e = wide::configure();
+    if (e != cudaSuccess) return e;
+  }
+  const int wide_tiles = (a.S + wide::OWN - 1) / wide::OWN, group = a.Hq / a.Hkv;
+  // f32 bytes that stream past a tile: the shared K and V, or Q and dO of the group's heads
+  const int dq_heads = head_group_for((size_t)a.S * D * 8 / (size_t)group, a.B * a.Hq, (long long)tiles * a.B * a.Hq);
+  const int dkv_heads = head_group_for((size_t)a.S * D * 8 * (size_t)group, a.B * a.Hkv, (long long)tiles * a.B * a.Hkv);
+  if (wide_dq)
+    wide::train_dq_wide_kernel<<<dim3(wide_tiles, a.B * a.Hq, 1), 256, wide::DQ_SMEM, stream>>>(
+        a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv, dq_heads, a.causal);
+  else
+    dq_kern<<<dim3(tiles, a.B * a.Hq, 1), 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
+                                                                    a.Hq, a.Hkv, dq_heads, a.causal);
   (*launches)++;
-  dkv_kern<<<dim3(tiles, a.B * a.Hkv, 1), 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
-                                                                     a.dv, a.S, a.Hq, a.Hkv, a.causal);
+  if (wide_dkv)
+    wide::train_dkv_wide_kernel<<<dim3(wide_tiles, a.B * a.Hkv, 1), 256, wide::DKV_SMEM, stream>>>(
+        a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv, dkv_heads, a.causal);
+  else
+    dkv_kern<<<dim3(tiles, a.B * a.Hkv, 1), 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
+                                                                       a.dv, a.S, a.Hq, a.Hkv, dkv_heads, a.causal);
   (*launches)++;
   return cudaGetLastError();
 }
