@@ -54,6 +54,9 @@ struct TcArgs {
   uint32_t* sticky;     // the library's accumulator of the same bits (nullable)
 };
 cudaError_t launch_attn_tc(const TcArgs& a, cudaStream_t stream);
+// The short-sequence bf16 form (attn_fwd_short.cu) and the calls launch_attn_tc hands to it.
+bool attn_short_takes(const TcArgs& a);
+cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream);
 // y = LayerNorm(x + r) * gamma + beta over rows of `cols` bf16 elements (cols a multiple of 8, at most 4096); r and
 // sum_out may be null (sum_out receives bf16(x + r) and may be x itself).
 cudaError_t launch_add_layernorm(const void* x, const void* r, const void* gamma, const void* beta, void* sum_out,

@@ -38,6 +38,7 @@
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
 #include "cta_order.cuh"
+#include "softmax_math.cuh"
 
 #include <type_traits>
 
@@ -49,10 +50,6 @@ using namespace arptx;
 __device__ int g_test_skip_k_tile = -1;
 #endif
 
-// Up to this length a CTA of the D = 64 bf16 kernel takes one query tile instead of two (measured: S=100 22.9 against
-// 33.8 us, S=197 46.5 against 48.7 us for 768 heads; from S=512 on the two-tile form is ahead, 37.2 against 37.8 us).
-constexpr int SHORT_SEQUENCE = 256;
-
 constexpr int BM = 128;  // query rows per tile
 constexpr int BN = 128;  // keys per step
 constexpr int NPART = 2;  // P of a step is handed to the MMA warp in two halves of 64 keys
@@ -62,23 +59,16 @@ constexpr float LOG2E = 1.4426950408889634f;
 // masked row, as in the reference).
 constexpr float NEG = -1e30f * LOG2E;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
-// Shape of a CTA.  TILES = 2: two query tiles, 384 threads -- softmax warpgroup 0, softmax warpgroup 1,
-// {TMA producer, MMA issuer, 2 idle warps}; one CTA per SM (all 512 TMEM columns).  TILES = 1: one query tile,
-// 256 threads, 256 TMEM columns and at most half of the shared memory and registers, so that two CTAs share an SM:
-// the form for short sequences, where a CTA is a chain of latencies (loads, two or three key steps, epilogue) with
-// nothing of its own to overlap them with.
-// setmaxnreg moves registers inside the pool the CTA was launched with (168 per thread for 384 threads, 128 per
-// thread for 256 threads at two CTAs per SM); an increase that the pool cannot cover waits forever.
-template <int TILES>
-struct Shape {
-  static constexpr int NUM_THREADS = 128 * TILES + 128;
-  static constexpr int MIN_CTAS = TILES == 1 ? 2 : 1;
-  static constexpr int LAUNCH_REGS = TILES == 1 ? 128 : 168;
-  static constexpr int SOFTMAX_REGS = TILES == 1 ? 208 : 216;  // softmax warps after setmaxnreg
-  static constexpr int SERVICE_REGS = TILES == 1 ? 48 : 72;    // the last warpgroup
-  static_assert(TILES * 4 * 32 * SOFTMAX_REGS + 4 * 32 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
-  static_assert(LAUNCH_REGS * NUM_THREADS * MIN_CTAS <= 65536, "register file of the SM");
-};
+// Two query tiles, 384 threads: softmax warpgroup 0, softmax warpgroup 1, {TMA producer, MMA issuer, 2 idle warps}; one CTA
+// per SM (all 512 TMEM columns).  setmaxnreg moves registers inside the pool the CTA was launched with (168 per thread);
+// an increase that the pool cannot cover waits forever.
+constexpr int TILES = 2;
+constexpr int NUM_THREADS = 128 * TILES + 128;
+constexpr int LAUNCH_REGS = 168;
+constexpr int SOFTMAX_REGS = 216;  // softmax warps after setmaxnreg
+constexpr int SERVICE_REGS = 72;   // the last warpgroup
+static_assert(TILES * 128 * SOFTMAX_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
+static_assert(LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
 
 // Largest scale c of an INT8 step that may fold its conversion: (12582912 + 127 * 127 * 128) * c < 2^14.
 constexpr float FOLD_MAX_C = 1.0e-3f;
@@ -86,34 +76,6 @@ constexpr float FOLD_MAX_C = 1.0e-3f;
 // Which of the 16 column pairs of each 32-column group take their exponential on the FMA pipe (bit i = pair i):
 // the MUFU unit delivers 16 ex2 per clock and SM, which alone would bound a step of two tiles at 2048 cycles.
 constexpr uint32_t POLY_MASK = 0x8888u;  // one pair in four
-
-// 2^x for two lanes on the MUFU unit.
-__device__ __forceinline__ void exp2_mufu_x2(uint64_t x2, float& p0, float& p1) {
-  float a, b;
-  unpack_f32x2(x2, a, b);
-  p0 = ex2f(a);
-  p1 = ex2f(b);
-}
-// 2^x for two lanes without the MUFU unit: x = n + f with n the nearest integer (read from the low mantissa bits of
-// x + 1.5 * 2^23) and f in [-0.5, 0.5], 2^f by a cubic whose relative error stays below 1.1e-4 (P is rounded to
-// bf16, 2^-9, afterwards), n added to the exponent field.  x is clamped at -126 so that the exponent cannot wrap;
-// 2^0 is exactly 1.
-__device__ __forceinline__ void exp2_poly_x2(uint64_t x2, float& p0, float& p1) {
-  float a, b;
-  unpack_f32x2(x2, a, b);
-  const uint64_t xc = pack_f32x2(fmaxf(a, -126.0f), fmaxf(b, -126.0f));
-  const uint64_t t2 = add_f32x2(xc, pack_f32x2(12582912.0f, 12582912.0f));
-  const uint64_t n2 = add_f32x2(t2, pack_f32x2(-12582912.0f, -12582912.0f));
-  const uint64_t f2 = fma_f32x2(n2, pack_f32x2(-1.0f, -1.0f), xc);
-  uint64_t y2 = fma_f32x2(pack_f32x2(0.055008914f, 0.055008914f), f2, pack_f32x2(0.242211f, 0.242211f));
-  y2 = fma_f32x2(y2, f2, pack_f32x2(0.69328296f, 0.69328296f));
-  y2 = fma_f32x2(y2, f2, pack_f32x2(1.0f, 1.0f));
-  float ya, yb, ta, tb;
-  unpack_f32x2(y2, ya, yb);
-  unpack_f32x2(t2, ta, tb);
-  p0 = __uint_as_float(__float_as_uint(ya) + (__float_as_uint(ta) << 23));
-  p1 = __uint_as_float(__float_as_uint(yb) + (__float_as_uint(tb) << 23));
-}
 
 // The additive mask of a warp's 32 query rows, staged through shared memory in chunks of 32 keys.  A thread owns a row,
 // so reading the mask from memory in place would touch 32 lines per load instruction; here a warp copies a chunk row by
@@ -339,7 +301,7 @@ __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float
   l += lsum + lsum_hi;
 }
 
-template <int MODE, int D, int TILES = 2, bool MASKED = false>
+template <int MODE, int D, bool MASKED = false>
 struct Cfg {
   static constexpr bool QUANT = MODE == TC_SAGE || MODE == TC_SAGE_FP8;  // 8-bit Q and K with per-block scales
   static constexpr int QK_ESIZE = QUANT ? 1 : MODE == TC_TF32 ? 4 : 2;
@@ -363,7 +325,7 @@ struct Cfg {
   static constexpr int V_TILE_BYTES = BN * D * V_ESIZE;
   static constexpr int PV_KSTEPS = MODE == TC_TF32 ? BN / 8 : BN / 16;
   static constexpr int STAGES =
-      TILES == 1 || MASKED ? 2 : ((2 * Q_TILE_STRIDE + 3 * (QK_TILE_BYTES + V_TILE_BYTES) <= 200 * 1024) ? 3 : 2);
+      MASKED ? 2 : ((2 * Q_TILE_STRIDE + 3 * (QK_TILE_BYTES + V_TILE_BYTES) <= 200 * 1024) ? 3 : 2);
   static constexpr int SMEM_TILES = TILES * Q_TILE_STRIDE + STAGES * (QK_TILE_BYTES + V_TILE_BYTES);
   // chunks of the additive mask in flight per softmax warp (4 KB each): as many of a step's four as fit
   static constexpr int MASK_RING = !MASKED ? 0 : (224 * 1024 - SMEM_TILES) / (TILES * 4 * 4096) >= 4 ? 4
@@ -373,7 +335,6 @@ struct Cfg {
   static constexpr int NUM_BARS = 2 + 4 * STAGES + 4 + 2 * NPART;
   static constexpr int SMEM_BYTES = SMEM_TILES + MASK_BYTES + NUM_BARS * 8 + 16 + 1024;  // + alignment slack
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-  static_assert(TILES == 2 || SMEM_BYTES <= 113 * 1024, "two one-tile CTAs must fit an SM");
   static constexpr int QK_KIND = MODE == TC_SAGE ? KIND_I8 : MODE == TC_SAGE_FP8 ? KIND_F8 : MODE == TC_TF32 ? KIND_TF32 : KIND_F16;
   static constexpr uint32_t IDESC_QK = MODE == TC_SAGE       ? make_idesc(2, 1, 1, 0, 0, BM, BN)  // s8 x s8 -> s32
                                        : MODE == TC_SAGE_FP8 ? make_idesc(1, 0, 0, 0, 0, BM, BN)  // e4m3 x e4m3 -> f32
@@ -385,15 +346,15 @@ struct Cfg {
 // ROWS: Sage with one scale per query row and per key row; MASKED: an additive mask (instantiations of their own, so
 // that the plain kernel carries none of either).
 // head_group: cta_order.cuh; the heaviest query block is the last one of a causal call, else the partial one comes last.
-template <int MODE, int D, int TILES, bool ROWS, bool MASKED>
-__global__ void __launch_bounds__(Shape<TILES>::NUM_THREADS, Shape<TILES>::MIN_CTAS)
+template <int MODE, int D, bool ROWS, bool MASKED>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ out, const float* __restrict__ mask,
                    const float* __restrict__ q_scale, const float* __restrict__ k_scale, int N, int Hq, int Hkv,
                    int head_group, int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
                    const OutReplicas reps, const OutProgress progress, float* __restrict__ lse_out, uint32_t* status,
                    uint32_t* sticky) {
-  using C = Cfg<MODE, D, TILES, MASKED>;
+  using C = Cfg<MODE, D, MASKED>;
   constexpr int ST = C::STAGES;
   constexpr int W_PROD = 4 * TILES;     // warp that loads
   constexpr int W_MMA = 4 * TILES + 1;  // warp that issues the MMAs
@@ -517,7 +478,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after();
   const uint32_t tb = *tmem_slot;
 
-  if (warp >= W_PROD) setmaxnreg_dec<Shape<TILES>::SERVICE_REGS>();
+  if (warp >= W_PROD) setmaxnreg_dec<SERVICE_REGS>();
   if (warp == W_PROD) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -636,7 +597,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     }
   } else if (warp < W_PROD) {
     // ------------------------------------------------------------ softmax warps
-    setmaxnreg_inc<Shape<TILES>::SOFTMAX_REGS>();
+    setmaxnreg_inc<SOFTMAX_REGS>();
     const int t = warp >> 2;
     const int r = tid & 127;
     const int row = q0 + t * BM + r;
@@ -802,13 +763,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int MODE, int D, int TILES, bool ROWS = false, bool MASKED = false>
+template <int MODE, int D, bool ROWS = false, bool MASKED = false>
 cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
   if constexpr (!MASKED) {
-    if (a.mask != nullptr) return launch_one<MODE, D, 2, ROWS, true>(a, stream);  // (no one-tile form with a mask)
+    if (a.mask != nullptr) return launch_one<MODE, D, ROWS, true>(a, stream);
   }
-  using C = Cfg<MODE, D, TILES, MASKED>;
-  auto kern = attn_fwd_tc_kernel<MODE, D, TILES, ROWS, MASKED>;
+  using C = Cfg<MODE, D, MASKED>;
+  auto kern = attn_fwd_tc_kernel<MODE, D, ROWS, MASKED>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -822,7 +783,7 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
   // Heads whose K and V stay in L2 together are walked as one group; completion reports want pairs to finish one by one.
   const size_t head_bytes = (size_t)a.S * D * (C::QK_ESIZE + C::V_ESIZE) / (size_t)(a.Hq / a.Hkv);
   const int head_group = a.progress.count != nullptr ? 1 : head_group_for(head_bytes, (int)grid.y, (long long)grid.x * grid.y);
-  kern<<<grid, Shape<TILES>::NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale,
+  kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale,
                                                                    a.k_scale, a.S, a.Hq, a.Hkv, head_group, a.causal, a.out_f32,
                                                                    a.token_major, a.o_sb, a.o_sh, a.o_ss, a.replicas,
                                                                    a.progress, a.lse_out, a.status, a.sticky);
@@ -872,18 +833,17 @@ bool attn_tc_has(int mode, int D) {
 }
 
 cudaError_t launch_attn_tc(const TcArgs& a, cudaStream_t stream) {
-  // short sequences at D = 64: one query tile per CTA, two CTAs per SM
-  if (a.mode == TC_BF16 && a.D == 64 && a.S <= SHORT_SEQUENCE) return launch_one<TC_BF16, 64, 1>(a, stream);
-  if (a.mode == TC_BF16 && a.D == 128) return launch_one<TC_BF16, 128, 2>(a, stream);
-  if (a.mode == TC_BF16 && a.D == 64) return launch_one<TC_BF16, 64, 2>(a, stream);
-  if (a.mode == TC_SAGE && a.scale_rows && a.D == 128) return launch_one<TC_SAGE, 128, 2, true>(a, stream);
-  if (a.mode == TC_SAGE && a.scale_rows && a.D == 64) return launch_one<TC_SAGE, 64, 2, true>(a, stream);
+  if (attn_short_takes(a)) return launch_attn_short(a, stream);
+  if (a.mode == TC_BF16 && a.D == 128) return launch_one<TC_BF16, 128>(a, stream);
+  if (a.mode == TC_BF16 && a.D == 64) return launch_one<TC_BF16, 64>(a, stream);
+  if (a.mode == TC_SAGE && a.scale_rows && a.D == 128) return launch_one<TC_SAGE, 128, true>(a, stream);
+  if (a.mode == TC_SAGE && a.scale_rows && a.D == 64) return launch_one<TC_SAGE, 64, true>(a, stream);
   if (a.scale_rows) return cudaErrorInvalidValue;
-  if (a.mode == TC_SAGE && a.D == 128) return launch_one<TC_SAGE, 128, 2>(a, stream);
-  if (a.mode == TC_SAGE && a.D == 64) return launch_one<TC_SAGE, 64, 2>(a, stream);
-  if (a.mode == TC_SAGE_FP8 && a.D == 128) return launch_one<TC_SAGE_FP8, 128, 2>(a, stream);
-  if (a.mode == TC_SAGE_FP8 && a.D == 64) return launch_one<TC_SAGE_FP8, 64, 2>(a, stream);
-  if (a.mode == TC_TF32 && a.D == 64) return launch_one<TC_TF32, 64, 2>(a, stream);
+  if (a.mode == TC_SAGE && a.D == 128) return launch_one<TC_SAGE, 128>(a, stream);
+  if (a.mode == TC_SAGE && a.D == 64) return launch_one<TC_SAGE, 64>(a, stream);
+  if (a.mode == TC_SAGE_FP8 && a.D == 128) return launch_one<TC_SAGE_FP8, 128>(a, stream);
+  if (a.mode == TC_SAGE_FP8 && a.D == 64) return launch_one<TC_SAGE_FP8, 64>(a, stream);
+  if (a.mode == TC_TF32 && a.D == 64) return launch_one<TC_TF32, 64>(a, stream);
   return cudaErrorInvalidValue;
 }
 

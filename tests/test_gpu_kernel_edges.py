@@ -25,6 +25,34 @@ def _bf16(oracle_lib, arrays):
     return [oracle_lib.f32_to_bf16(x) for x in arrays]
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 33, 96, 127, 128, 129, 144, 160, 197, 255, 256, 257])
+@pytest.mark.parametrize("causal", [False, True])
+def test_bf16_short_sequences(ops, oracle_lib, n, causal):
+    """bf16 P (2^-9) and a quarter of the exponentials within 1.1e-4: the bf16 forward's 2e-2 against exact, 5e-3
+    against the oracle's model of the same rounding points (which keeps N(0,1) outputs below about 4)."""
+    qb, kb, vb = _bf16(oracle_lib, normal_qkv(n, 2, 4, 2, n, 64))
+    got = oracle_lib.bf16_to_f32(from_dev_bf16(ops.attn_forward("bf16", *map(to_dev_bf16, (qb, kb, vb)), None, causal)))
+    exact = oracle_lib.flash(0, *map(oracle_lib.bf16_to_f32, (qb, kb, vb)), None, causal)
+    assert max_abs(got, exact) <= 2e-2 and cosine(got, exact) >= 0.999
+    assert ops.last_status(None) == 0
+
+
+def test_bf16_short_sequences_many_items_per_cta(ops, oracle_lib):
+    """More (head, tile) items than resident CTAs: every CTA walks several, and its buffers change hands."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1)
+    B, H, S, D = 40, 12, 197, 64
+    qkv = torch.randn(B, S, 3, H, D, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
+    out = ops.attn_forward_views(q, k, v)
+    want = torch.nn.functional.scaled_dot_product_attention(q.double(), k.double(), v.double())
+    assert (out.double() - want).abs().max().item() <= 2e-2
+    assert torch.equal(out, ops.attn_forward_views(q, k, v))
+    # the last item alone gives the bits it had among the others
+    one = ops.attn_forward_views(q[-1:], k[-1:], v[-1:])
+    assert torch.equal(out[-1:], one)
+
+
 @pytest.mark.parametrize("mode,d", [("bf16", 64), ("bf16", 128), ("tf32", 64), ("sage", 128), ("sage_rows", 64)])
 @pytest.mark.parametrize("n", [1, 31, 33, 100, 127, 129, 260, 389])
 @pytest.mark.parametrize("causal", [False, True])
