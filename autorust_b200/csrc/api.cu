@@ -14,9 +14,10 @@ namespace {
 std::atomic<uint64_t> g_selected[6];
 std::atomic<uint64_t> g_launches;
 
-// The library's status block on each device.  Word 0: launch status of calls that bring no workspace (cleared before
-// every such launch).  Word 1: every expiry of a bounded wait in any kernel of the library is OR-ed in here as well,
-// and only ar_attn_last_status(NULL, ..) clears it -- a launch cannot erase what an earlier one reported.
+// The library's status block on each device.  Word 0: launch status of calls that bring no workspace (cleared before the
+// launch, or marked with the launch's ticket when a wait runs out: prepare_status).  Word 1: every expiry of a bounded
+// wait in any kernel of the library is OR-ed in here as well, and only ar_attn_last_status(NULL, ..) clears it -- a
+// launch cannot erase what an earlier one reported.
 __device__ __align__(256) uint32_t g_status_word[64];
 
 // 1 when the current device is compute capability 10.x.
@@ -83,6 +84,21 @@ uint32_t* library_words() {
 uint32_t* status_ptr(void* workspace) {
   if (workspace) return (uint32_t*)workspace;
   return library_words();
+}
+// The status word of a launch that no earlier kernel of the call clears.  The caller's word is cleared on the stream.
+// The library's word is not: the launch gets a ticket instead, which saves the stream a memset of its own in front of a
+// kernel of 20 microseconds.  A captured call would replay its ticket, so that one clears the word as well.
+bool prepare_status(ar::TcArgs& a, bool callers_word, cudaStream_t stream) {
+  if (!callers_word) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return false;
+    if (capture == cudaStreamCaptureStatusNone) {
+      static std::atomic<uint32_t> next{0};
+      a.ticket = (next.fetch_add(1) & 0x3fffffffu) + 1u;  // 1 .. 2^30: never 0, never the bit an OR-ed status carries
+      return true;
+    }
+  }
+  return cudaMemsetAsync(a.status, 0, sizeof(uint32_t), stream) == cudaSuccess;
 }
 uint32_t* sticky_ptr() {
   uint32_t* p = library_words();
@@ -258,7 +274,8 @@ int forward_impl(int mode, int dtype, const void* q, const void* k, const void* 
   } else if (mode == AR_MODE_TF32) {
     const int64_t S_pad = (S + 3) / 4 * 4;
     float* vt = (float*)((uint8_t*)workspace + STATUS_BYTES);
-    if (ar::launch_transpose_v((const float*)v, vt, (int)(B * Hkv), (int)S, (int)S_pad, (int)D, stream) != cudaSuccess)
+    if (ar::launch_transpose_v((const float*)v, vt, (int)(B * Hkv), (int)S, (int)S_pad, (int)D, status, stream) !=
+        cudaSuccess)
       return AR_ERR_CUDA;
     g_launches++;
     a.mode = ar::TC_TF32;
@@ -306,9 +323,7 @@ int forward_impl(int mode, int dtype, const void* q, const void* k, const void* 
         !make_map(&a.tm_v, v16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D))
       return AR_ERR_CUDA;
   }
-  if (mode != AR_MODE_SAGE_INT8 && mode != AR_MODE_SAGE_FP8 && mode != AR_MODE_SAGE_INT8_ROWS &&
-      cudaMemsetAsync(status, 0, sizeof(uint32_t), stream) != cudaSuccess)
-    return AR_ERR_CUDA;
+  if (mode == AR_MODE_BF16 && !prepare_status(a, workspace != nullptr, stream)) return AR_ERR_CUDA;
   cudaError_t e = ar::launch_attn_tc(a, stream);
   if (e != cudaSuccess) return AR_ERR_CUDA;
   g_launches++;
@@ -401,7 +416,7 @@ int ar_attn_forward_strided(int mode, int dtype, const void* q, const void* k, c
       !ar::make_tile_map(&a.tm_v, v, bf16, 2, B, Hkv, S, D, v_strides[0], v_strides[1], v_strides[2], 64, 128, &tv))
     return AR_ERR_ALIGNMENT;  // strides that are not 16-byte multiples, or that the copy engine cannot express
   a.token_major = tq | (tk << 1) | (tv << 2);
-  if (cudaMemsetAsync(status, 0, sizeof(uint32_t), stream) != cudaSuccess) return AR_ERR_CUDA;
+  if (!prepare_status(a, workspace != nullptr, stream)) return AR_ERR_CUDA;
   if (ar::launch_attn_tc(a, stream) != cudaSuccess) return AR_ERR_CUDA;
   g_launches++;
   g_selected[mode]++;
@@ -602,7 +617,7 @@ int sage_prequantized_any(int mode, const void* q8, const void* k8, const float*
       !make_map(&a.tm_k, k8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B, Hkv, S, D) ||
       !make_map(&a.tm_v, v_bf16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D))
     return AR_ERR_CUDA;
-  if (cudaMemsetAsync(status, 0, sizeof(uint32_t), stream) != cudaSuccess) return AR_ERR_CUDA;
+  if (!prepare_status(a, status_word != nullptr, stream)) return AR_ERR_CUDA;
   if (ar::launch_attn_tc(a, stream) != cudaSuccess) return AR_ERR_CUDA;
   g_launches++;
   g_selected[mode]++;

@@ -52,6 +52,7 @@ struct TcArgs {
   float* lse_out;       // [B*Hq, S] natural-log sum of exponentials per row (the training forward), or null
   uint32_t* status;     // the launch's device status word: zero at launch, set when a bounded wait ran out
   uint32_t* sticky;     // the library's accumulator of the same bits (nullable)
+  uint32_t ticket;      // nonzero: `status` is shared and not cleared, an expiry leaves this value there
 };
 cudaError_t launch_attn_tc(const TcArgs& a, cudaStream_t stream);
 // The short-sequence bf16 form (attn_fwd_short.cu) and the calls launch_attn_tc hands to it.
@@ -141,8 +142,9 @@ struct PrologueArgs {
 // Returns the number of kernels launched through *launches.
 cudaError_t launch_sage_prologue(const PrologueArgs& a, cudaStream_t stream, int* launches);
 // [BH, S, D] f32 -> [BH, D, S_pad] f32 (S_pad = S rounded up to 4; the padding is zeroed): the K-major V
-// operand of the TF32 kernel.
-cudaError_t launch_transpose_v(const float* v, float* vt, int BH, int S, int S_pad, int D, cudaStream_t stream);
+// operand of the TF32 kernel.  Clears *status, the word of the launch that follows.
+cudaError_t launch_transpose_v(const float* v, float* vt, int BH, int S, int S_pad, int D, uint32_t* status,
+                               cudaStream_t stream);
 // f32 -> bf16 copy of V for Sage with f32 tensors.
 cudaError_t launch_f32_to_bf16(const float* src, void* dst, int64_t n, cudaStream_t stream);
 

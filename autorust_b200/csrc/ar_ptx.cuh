@@ -55,12 +55,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Where a wait that ran out is recorded.  `abort_flag` is a CTA-shared word: once any wait in the CTA has run out,
 // every later wait returns false at once.  `status` is the launch's device word (cleared by the host before the
 // launch; a CTA that finds it set on entry leaves without working), `sticky` the library's accumulator, which only
-// the host clears when it reads it.  Either may be null.
+// the host clears when it reads it.  Either may be null.  `ticket` nonzero: `status` is a word that launches share
+// without clearing it; an expiry leaves the launch's own ticket there, and only CTAs with that ticket leave.
 struct WaitCtx {
   volatile uint32_t* abort_flag;
   uint32_t* status;
   uint32_t* sticky;
+  uint32_t ticket = 0;
 };
+// True when a wait of this launch has already run out in another CTA.
+__device__ __forceinline__ bool launch_lost(const uint32_t* status, uint32_t ticket) {
+  if (status == nullptr) return false;
+  const uint32_t w = *(const volatile uint32_t*)status;
+  return ticket ? w == ticket : (w & 0x80000000u) != 0;
+}
 
 // Bounded wait on `bar` for phase `parity`.  On expiry the site id is OR-ed into the status words.
 // mbarrier.try_wait suspends the thread in hardware for a bounded time, so the loop is not a hot spin.
@@ -75,7 +83,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
       if (*w.abort_flag) return false;
       if (clock64() - t0 > AR_WAIT_BUDGET_CYCLES) {
         *w.abort_flag = 1u;
-        if (w.status) atomicOr(w.status, 0x80000000u | site);
+        if (w.status) {
+          if (w.ticket)
+            atomicExch(w.status, w.ticket);
+          else
+            atomicOr(w.status, 0x80000000u | site);
+        }
         if (w.sticky) atomicOr(w.sticky, 0x80000000u | site);
         return false;
       }

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, void* __restrict__ out, int N, int Hq, int Hkv, int items,
                           int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
-                          float* __restrict__ lse_out, uint32_t* status, uint32_t* sticky) {
+                          float* __restrict__ lse_out, uint32_t* status, uint32_t* sticky, uint32_t ticket) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   uint64_t* o_empty = bars + 7;    // O read: the columns may take the next S
   uint32_t* tmem_slot = (uint32_t*)(bars + NUM_BARS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const WaitCtx wctx{abort_flag, status, sticky};
+  const WaitCtx wctx{abort_flag, status, sticky, ticket};
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   bool lost = false;  // (meaningful in the producer thread only)
   if (warp == W_PROD && lane == 0) {
     // a launch whose status word is already set is lost: this CTA only allocates and frees its TMEM
-    lost = status != nullptr && (*(volatile uint32_t*)status & 0x80000000u) != 0;
+    lost = launch_lost(status, ticket);
     *abort_flag = lost ? 1u : 0u;
     for (int i = 0; i < NUM_BARS; i++) mbar_init(&bars[i], &bars[i] == p_full || &bars[i] == o_empty ? 128 : 1);
     fence_mbar_init();
@@ -340,7 +340,7 @@ cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream) {
   const int resident = 2 * (dev < 64 ? sm_count[dev] : 148);
   attn_fwd_short_kernel<<<items < resident ? items : resident, NUM_THREADS, SMEM_BYTES, stream>>>(
       a.tm_q, a.tm_k, a.tm_v, a.out, a.S, a.Hq, a.Hkv, items, a.causal, a.out_f32, a.token_major, a.o_sb, a.o_sh, a.o_ss,
-      a.lse_out, a.status, a.sticky);
+      a.lse_out, a.status, a.sticky, a.ticket);
   return cudaGetLastError();
 }
 

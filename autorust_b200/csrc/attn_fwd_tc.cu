@@ -353,7 +353,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                    const float* __restrict__ q_scale, const float* __restrict__ k_scale, int N, int Hq, int Hkv,
                    int head_group, int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
                    const OutReplicas reps, const OutProgress progress, float* __restrict__ lse_out, uint32_t* status,
-                   uint32_t* sticky) {
+                   uint32_t* sticky, uint32_t ticket) {
   using C = Cfg<MODE, D, MASKED>;
   constexpr int ST = C::STAGES;
   constexpr int W_PROD = 4 * TILES;     // warp that loads
@@ -375,7 +375,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* o_full = p_part + 2 * NPART;  // [2]
   uint32_t* tmem_slot = (uint32_t*)(o_full + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const WaitCtx wctx{abort_flag, status, sticky};
+  const WaitCtx wctx{abort_flag, status, sticky, ticket};
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler as well
@@ -443,7 +443,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp == W_PROD && lane == 0) {
     // A launch whose status word is already set (a wait ran out in an earlier CTA) is lost: this CTA only allocates
     // and frees its TMEM, so that the rest of the grid drains in microseconds instead of one wait budget per wave.
-    lost = status != nullptr && (*(volatile uint32_t*)status & 0x80000000u) != 0;
+    lost = launch_lost(status, ticket);
     *abort_flag = lost ? 1u : 0u;
     for (int i = 0; i < 2; i++) {
       mbar_init(&q_full[i], 1);
@@ -786,7 +786,7 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
   kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale,
                                                                    a.k_scale, a.S, a.Hq, a.Hkv, head_group, a.causal, a.out_f32,
                                                                    a.token_major, a.o_sb, a.o_sh, a.o_ss, a.replicas,
-                                                                   a.progress, a.lse_out, a.status, a.sticky);
+                                                                   a.progress, a.lse_out, a.status, a.sticky, a.ticket);
   return cudaGetLastError();
 }
 

@@ -389,7 +389,8 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restric
 // vt[bh][d][s] = v[bh][s][d] through a 32x33 shared tile; columns S..S_pad-1 are written as zero so that
 // a masked key (p = 0) can never meet a NaN left in the scratch.
 __global__ void __launch_bounds__(256) transpose_v_kernel(const float* __restrict__ v, float* __restrict__ vt, int S,
-                                                          int S_pad, int D) {
+                                                          int S_pad, int D, uint32_t* status) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0u;
   __shared__ float tile[32][33];
   const int bh = blockIdx.z;
   const int s0 = blockIdx.x * 32, d0 = blockIdx.y * 32;
@@ -492,9 +493,10 @@ cudaError_t launch_sage_prologue(const PrologueArgs& a, cudaStream_t stream, int
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_transpose_v(const float* v, float* vt, int BH, int S, int S_pad, int D, cudaStream_t stream) {
+cudaError_t launch_transpose_v(const float* v, float* vt, int BH, int S, int S_pad, int D, uint32_t* status,
+                               cudaStream_t stream) {
   dim3 grid((S_pad + 31) / 32, D / 32, BH);
-  transpose_v_kernel<<<grid, 256, 0, stream>>>(v, vt, S, S_pad, D);
+  transpose_v_kernel<<<grid, 256, 0, stream>>>(v, vt, S, S_pad, D, status);
   return cudaGetLastError();
 }
 
