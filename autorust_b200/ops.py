@@ -157,6 +157,58 @@ def attn_forward_views(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: 
     return out
 
 
+def views_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, stream: torch.cuda.Stream):
+    """attn_forward_views (bf16, no mask, not causal) for a caller that makes the same call on many tensors of one layout,
+    as the layers of an encoder do: checks and strides are worked out once, the function returned takes the device
+    addresses of four tensors that differ from these in their memory only (same shapes, strides, dtype and device -- the
+    caller's word).  To be used with q's device current, while the caller keeps the tensors alive."""
+    L = _abi.load()
+    for t in (q, k, v, out):
+        if t.dim() != 4 or not t.is_cuda or t.stride(3) != 1 or t.dtype != torch.bfloat16 or t.device != q.device:
+            raise ValueError("q, k, v, out must be 4-D bfloat16 CUDA tensors [B, H, S, D] with a contiguous last dimension")
+    if k.shape != v.shape or q.shape != out.shape or q.shape[0] != k.shape[0] or q.shape[2:] != k.shape[2:]:
+        raise ValueError("shape mismatch between q, k, v, out")
+    B, Hq, S, D = q.shape
+    arr = ctypes.c_int64 * 3
+    strides = tuple(arr(*t.stride()[:3]) for t in (q, k, v, out))
+    tail = (None, B, Hq, k.shape[1], S, D, 0, *strides, None, 0, stream.cuda_stream)
+    fn = L.ar_attn_forward_strided
+
+    def call(q, k, v, out):
+        rc = fn(_abi.MODE_BF16, _abi.DTYPE_BF16, q, k, v, out, *tail)
+        if rc != _abi.AR_OK:
+            _abi.check(rc, "ar_attn_forward_strided")
+
+    return call
+
+
+def layernorm_call(x: torch.Tensor, stream: torch.cuda.Stream, eps: float = 1e-5):
+    """add_layernorm for a caller that makes the same call many times: the function returned does x += residual (when
+    there is one) and y = LayerNorm(x) * gamma + beta; y has x's layout, the other tensors are checked.  The same
+    terms as views_call."""
+    L = _abi.load()
+    _check_dense("x", x, x.shape, torch.bfloat16, x.device)
+    cols = x.shape[-1]
+    numel, device, vector = x.numel(), x.device, torch.Size((cols,))
+    tail = (numel // cols, cols, float(eps), _abi.DTYPE_BF16, stream.cuda_stream)
+    fn = L.ar_add_layernorm
+
+    def call(x, residual, gamma, beta, y):
+        for t in (gamma, beta):
+            if t.dtype != torch.bfloat16 or t.shape != vector or t.device != device or not t.is_contiguous():
+                raise ValueError("gamma and beta must be contiguous bfloat16 vectors on the tensors' device")
+        if residual is not None and (residual.dtype != torch.bfloat16 or residual.numel() != numel
+                                     or residual.device != device or not residual.is_contiguous()):
+            raise ValueError("the residual must be a contiguous bfloat16 tensor of x's size")
+        xp = x.data_ptr()
+        rc = fn(xp, None if residual is None else residual.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+                None if residual is None else xp, y.data_ptr(), *tail)
+        if rc != _abi.AR_OK:
+            _abi.check(rc, "ar_add_layernorm")
+
+    return call
+
+
 def train_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torch.Tensor | None = None,
                   causal: bool = False, stream=None, tensor_cores: bool = False):
     """Forward that also returns the rows' log-sum-exp: (o [B,Hq,S,D], lse [B,Hq,S]), float32 tensors.  Exact f32
