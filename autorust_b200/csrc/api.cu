@@ -617,7 +617,8 @@ int sage_prequantized_any(int mode, const void* q8, const void* k8, const float*
       !make_map(&a.tm_k, k8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B, Hkv, S, D) ||
       !make_map(&a.tm_v, v_bf16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, Hkv, S, D))
     return AR_ERR_CUDA;
-  if (!prepare_status(a, status_word != nullptr, stream)) return AR_ERR_CUDA;
+  // (the INT8 kernel takes no ticket)
+  if (!prepare_status(a, status_word != nullptr || mode == AR_MODE_SAGE_INT8, stream)) return AR_ERR_CUDA;
   if (ar::launch_attn_tc(a, stream) != cudaSuccess) return AR_ERR_CUDA;
   g_launches++;
   g_selected[mode]++;

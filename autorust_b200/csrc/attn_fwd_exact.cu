@@ -43,7 +43,7 @@ template <int D, int RQ, int TX, int TY, int GROUPS>
 __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     attn_fwd_exact_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                           float* __restrict__ O, const float* __restrict__ M, float* __restrict__ LSE, int N, int Hq,
-                          int Hkv, int head_group, int causal) {
+                          int Hkv, int grouped, int causal) {
   using C = ExactCfg<D, RQ, TX, TY, GROUPS>;
   constexpr int JK = C::JK, OD = C::OD, D4 = D / 4;
   extern __shared__ __align__(16) float smem_f[];
@@ -53,9 +53,9 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
   float* sK = sQ + C::BQ * C::LDQ + grp * C::GROUP_FLOATS;
   float* sV = sK + BK * C::LDQ;
   float* sP = sV + BK * D;
-  int tile, bh;
-  cta_order(head_group, tile, bh);
-  if (causal) tile = (int)gridDim.x - 1 - tile;  // the last query tile sees the most keys
+  const int bh = cta_head(grouped);
+  int tile = cta_tile(grouped);
+  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * C::BQ;
@@ -260,10 +260,9 @@ cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const dim3 grid((a.S + C::BQ - 1) / C::BQ, a.B * a.Hq, 1);
-  const int head_group = head_group_for((size_t)a.S * D * 8 / (size_t)(a.Hq / a.Hkv), a.B * a.Hq, (long long)grid.x * grid.y);
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, head_group,
-                                                   a.causal);
+  const CtaGrid g = cta_grid((size_t)a.S * D * 8 / (size_t)(a.Hq / a.Hkv), a.B * a.Hq, (a.S + C::BQ - 1) / C::BQ);
+  kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped,
+                                                     a.causal);
   return cudaGetLastError();
 }
 

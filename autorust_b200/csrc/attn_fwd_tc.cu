@@ -53,6 +53,7 @@ __device__ int g_test_skip_k_tile = -1;
 constexpr int BM = 128;  // query rows per tile
 constexpr int BN = 128;  // keys per step
 constexpr int NPART = 2;  // P of a step is handed to the MMA warp in two halves of 64 keys
+enum { ORDER_PLAIN, ORDER_GROUPED, ORDER_ARG };
 constexpr float LOG2E = 1.4426950408889634f;
 // The reference's finite sentinel (-1e30), expressed in the log2 domain the softmax works in, so that
 // a logit masked by an additive -1e30 still ties with the initial running max (p = 1 for a fully
@@ -83,7 +84,9 @@ constexpr uint32_t POLY_MASK = 0x8888u;  // one pair in four
 // pieces.  Piece p of row r lies at p ^ (r & 7), which keeps both sides free of bank conflicts.  RING chunks are in
 // flight, so the next step's first chunks land under this step's exponentials.  Rows and keys past the sequence end
 // are filled with zeros (the caller excludes those keys).
-// Measured, B=4 H=16 S=789 D=64 with a mask (this and the order of cta_order.cuh): 133 -> 85 us.
+// Measured, B=4 H=16 S=789 D=64 with a mask (this and the order of cta_order.cuh): 133 -> 78 us.  Copies by the two warps
+// of the last warpgroup that have nothing else to do took 144 us, 16-byte copies from the boundary before each row with
+// a shift on reading 90 us.
 template <int RING>
 struct MaskRing {
   const float* mask;
@@ -106,11 +109,22 @@ struct MaskRing {
         const int col = n * 32 + lane;
         const float* src = mask + (size_t)row0 * N + col;
         const uint32_t d = dst + ((lane & 3) << 2);
-#pragma unroll 8
-        for (int r = 0; r < 32; r++) {
-          const bool in = row0 + r < N && col < N;
-          cp_async4(d + r * 128 + (((lane >> 2) ^ (r & 7)) << 4), in ? src : mask, in);
-          src += N;
+        if (row0 + 32 <= N) {  // every row is inside: a lane's column decides for all of them
+          const bool in = col < N;
+          const size_t step = in ? (size_t)N : 0;
+          src = in ? src : mask;
+#pragma unroll
+          for (int r = 0; r < 32; r++) {
+            cp_async4(d + r * 128 + (((lane >> 2) ^ (r & 7)) << 4), src, in);
+            src += step;
+          }
+        } else {
+#pragma unroll 4
+          for (int r = 0; r < 32; r++) {
+            const bool in = row0 + r < N && col < N;
+            cp_async4(d + r * 128 + (((lane >> 2) ^ (r & 7)) << 4), in ? src : mask, in);
+            src += N;
+          }
         }
       }
     }
@@ -134,11 +148,13 @@ struct NoMask {};
 
 // One softmax step of one row: scores of 128 keys (sv, raw accumulator bits) -> P in TMEM, running
 // max m and running sum l updated, O rescaled in place when the max grows by more than the threshold.
-// EDGE = 1 selects the element-wise path of launches with an additive mask (MASK is a MaskRing) or one scale per key.
+// EDGE = 1: the element-wise path of launches with an additive mask (MASK is a MaskRing).  EDGE = 3: the same for INT8
+// scores, with the mask read in place (see the kernel) and one scale per key where kcol is given.
 template <int MODE, int D, int EDGE, class MASK = NoMask>
 __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float& l, float c, int j, int col0, int row,
                                              int N, int causal, uint32_t tS, uint32_t tO, uint64_t* p_parts,
-                                             const float* __restrict__ kcol = nullptr, MASK* ring = nullptr) {
+                                             MASK* ring = nullptr, const float* __restrict__ kcol = nullptr,
+                                             const float* __restrict__ mask = nullptr) {
   float mc;  // row maximum of this step in the scaled (log2) domain
   // INT8 scores stay integers through the maximum on interior steps only; a bounds-only boundary step converts
   // them first (the same exact bit trick as below), so that the excluded columns can be marked with -inf
@@ -164,32 +180,55 @@ __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float
     for (int i = 0; i < BN; i++)
       if (i >= first_out) sv[i] = 0xff800000u;
   }
-  if constexpr (EDGE == 1) {
+  if constexpr (EDGE == 3) {
     // leaves scaled logits in sv and c = 1
+    const float* mrow = (mask != nullptr && row < N) ? mask + (size_t)row * N : nullptr;
+    float mx = NEG;
+#pragma unroll
+    for (int i = 0; i < BN; i++) {
+      const int col = col0 + i;
+      // kcol: one scale per key
+      const float ci = kcol != nullptr ? c * (col < N ? kcol[i] : 0.f) : c;
+      float x = MODE == TC_SAGE ? (float)(int)sv[i] * ci : __uint_as_float(sv[i]) * ci;
+      if (mrow != nullptr && col < N) x = fmaf(mrow[col], LOG2E, x);
+      if (col >= N || (causal && col > row)) x = NEG;
+      sv[i] = __float_as_uint(x);
+      mx = fmaxf(mx, x);
+    }
+    c = 1.0f;
+    mc = mx;
+  } else if constexpr (EDGE == 1) {
+    // leaves scaled logits in sv and c = 1
+    // (uniform) a step inside the sequence and below the diagonal excludes nothing: its columns take no comparison
+    const bool bounds = col0 + BN > N || (causal && __any_sync(0xffffffffu, col0 + BN - 1 > row));
     const int first_out = min(causal ? row - col0 + 1 : BN, N - col0);
+    const uint64_t c2 = pack_f32x2(c, c), log2e2 = pack_f32x2(LOG2E, LOG2E);
     float mx = NEG;
 #pragma unroll
     for (int q = 0; q < BN / 32; q++) {
-      const float* mrow = nullptr;
-      if constexpr (!std::is_same_v<MASK, NoMask>) mrow = ring->acquire(j * (BN / 32) + q);
+      const float* mrow = ring->acquire(j * (BN / 32) + q);
 #pragma unroll
       for (int p4 = 0; p4 < 8; p4++) {
-        float4 mv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr (!std::is_same_v<MASK, NoMask>) mv = *(const float4*)(mrow + ((p4 ^ (row & 7)) << 2));
-        const float mvv[4] = {mv.x, mv.y, mv.z, mv.w};
+        const float4 mv = *(const float4*)(mrow + ((p4 ^ (row & 7)) << 2));
+        const uint64_t mv2[2] = {pack_f32x2(mv.x, mv.y), pack_f32x2(mv.z, mv.w)};
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
+        for (int e = 0; e < 4; e += 2) {
           const int i = q * 32 + p4 * 4 + e;
-          // kcol: one scale per key
-          const float ci = kcol != nullptr ? c * (col0 + i < N ? kcol[i] : 0.f) : c;
-          float x = MODE == TC_SAGE ? (float)(int)sv[i] * ci : __uint_as_float(sv[i]) * ci;
-          if constexpr (!std::is_same_v<MASK, NoMask>) x = fmaf(mvv[e], LOG2E, x);
-          if (i >= first_out) x = NEG;
-          sv[i] = __float_as_uint(x);
-          mx = fmaxf(mx, x);
+          float x0, x1;
+          unpack_f32x2(fma_f32x2(mv2[e >> 1], log2e2,
+                                 mul_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), c2)), x0, x1);
+          sv[i] = __float_as_uint(x0);
+          sv[i + 1] = __float_as_uint(x1);
         }
       }
-      if constexpr (!std::is_same_v<MASK, NoMask>) ring->release(j * (BN / 32) + q);
+      if (bounds) {
+#pragma unroll
+        for (int i = q * 32; i < q * 32 + 32; i++)
+          if (i >= first_out) sv[i] = __float_as_uint(NEG);
+      }
+#pragma unroll
+      for (int i = q * 32; i < q * 32 + 32; i += 2) mx = fmax3(mx, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+      ring->release(j * (BN / 32) + q);
     }
     c = 1.0f;
     mc = mx;
@@ -345,17 +384,18 @@ struct Cfg {
 
 // ROWS: Sage with one scale per query row and per key row; MASKED: an additive mask (instantiations of their own, so
 // that the plain kernel carries none of either).
-// head_group: cta_order.cuh; the heaviest query block is the last one of a causal call, else the partial one comes last.
-template <int MODE, int D, bool ROWS, bool MASKED>
+// ORDER: the grid of cta_order.cuh, known when the plain kernel is compiled for the same reason; the heaviest query block is the last one of a causal call, else the partial one comes last.
+template <int MODE, int D, bool ROWS, bool MASKED, int ORDER>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ out, const float* __restrict__ mask,
                    const float* __restrict__ q_scale, const float* __restrict__ k_scale, int N, int Hq, int Hkv,
-                   int head_group, int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
+                   int grouped_arg, int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
                    const OutReplicas reps, const OutProgress progress, float* __restrict__ lse_out, uint32_t* status,
                    uint32_t* sticky, uint32_t ticket) {
   using C = Cfg<MODE, D, MASKED>;
   constexpr int ST = C::STAGES;
+  const bool grouped = ORDER == ORDER_ARG ? grouped_arg != 0 : ORDER == ORDER_GROUPED;
   constexpr int W_PROD = 4 * TILES;     // warp that loads
   constexpr int W_MMA = 4 * TILES + 1;  // warp that issues the MMAs
   extern __shared__ uint8_t smem_raw[];
@@ -375,13 +415,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* o_full = p_part + 2 * NPART;  // [2]
   uint32_t* tmem_slot = (uint32_t*)(o_full + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const WaitCtx wctx{abort_flag, status, sticky, ticket};
+  const WaitCtx wctx{abort_flag, status, sticky, MODE == TC_SAGE ? 0u : ticket};  // (see the softmax step's branches)
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler as well
   const int lane = tid & 31;
-  int xblk, bh;
-  cta_order(head_group, xblk, bh);
+  const int bh = cta_head(grouped);
   const int b = bh / Hq;
   const int h = bh - b * Hq;
   const int kvh = h / (Hq / Hkv);
@@ -393,7 +432,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     else
       tma_load_4d(dst, m, bar, x, tok, head, b);
   };
-  const int qblock = causal ? (int)gridDim.x - 1 - xblk : xblk;
+  const int qblock = causal ? cta_tiles(grouped) - 1 - cta_tile(grouped) : cta_tile(grouped);
   const int q0 = qblock * (TILES * BM);
   const int nkv_all = (N + BN - 1) / BN;
   int nkv[2] = {0, 0};
@@ -443,7 +482,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp == W_PROD && lane == 0) {
     // A launch whose status word is already set (a wait ran out in an earlier CTA) is lost: this CTA only allocates
     // and frees its TMEM, so that the rest of the grid drains in microseconds instead of one wait budget per wave.
-    lost = launch_lost(status, ticket);
+    lost = launch_lost(status, wctx.ticket);
     *abort_flag = lost ? 1u : 0u;
     for (int i = 0; i < 2; i++) {
       mbar_init(&q_full[i], 1);
@@ -639,11 +678,21 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       // masks by -inf and runs the interior code (INT8 scores are converted first); an additive mask, whose -1e30
       // must tie with the initial running max, takes the element-wise path.
       if constexpr (MASKED) {
-        softmax_step<MODE, D, 1>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t], kcol, &ring);
-      } else if constexpr (ROWS) {
-        softmax_step<MODE, D, 1>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t], kcol);
+        softmax_step<MODE, D, 1>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t], &ring);
+      } else if constexpr (MODE == TC_SAGE) {
+        // INT8 keeps its mask in this kernel, read in place: the interior step of this instantiation loses 2 % with the
+        // branch taken out, and as much with the launch ticket (S=8192: 3.07 -> 3.13 ms each; 3.19 ms without both)
+        const bool edge = (col0 + BN > N) || (causal && col0 + BN - 1 > q0 + t * BM) || (mask != nullptr) ||
+                          (MODE == TC_SAGE && c >= FOLD_MAX_C) || ROWS;
+        if (!edge)
+          softmax_step<MODE, D, 0>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t]);
+        else if (mask == nullptr && !ROWS)
+          softmax_step<MODE, D, 2>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t]);
+        else  // an additive mask, or one scale per key: element by element
+          softmax_step<MODE, D, 3>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t], (NoMask*)nullptr, kcol,
+                                   mask);
       } else {
-        const bool edge = (col0 + BN > N) || (causal && col0 + BN - 1 > q0 + t * BM) || (MODE == TC_SAGE && c >= FOLD_MAX_C);
+        const bool edge = (col0 + BN > N) || (causal && col0 + BN - 1 > q0 + t * BM);
         if (!edge)
           softmax_step<MODE, D, 0>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t]);
         else
@@ -763,13 +812,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int MODE, int D, bool ROWS = false, bool MASKED = false>
-cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
-  if constexpr (!MASKED) {
-    if (a.mask != nullptr) return launch_one<MODE, D, ROWS, true>(a, stream);
-  }
+template <int MODE, int D, bool ROWS, bool MASKED, int ORDER>
+cudaError_t launch_grid(const TcArgs& a, const CtaGrid& g, cudaStream_t stream) {
   using C = Cfg<MODE, D, MASKED>;
-  auto kern = attn_fwd_tc_kernel<MODE, D, ROWS, MASKED>;
+  auto kern = attn_fwd_tc_kernel<MODE, D, ROWS, MASKED, ORDER>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -779,15 +825,28 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  dim3 grid((a.S + TILES * BM - 1) / (TILES * BM), a.B * a.Hq, 1);
-  // Heads whose K and V stay in L2 together are walked as one group; completion reports want pairs to finish one by one.
-  const size_t head_bytes = (size_t)a.S * D * (C::QK_ESIZE + C::V_ESIZE) / (size_t)(a.Hq / a.Hkv);
-  const int head_group = a.progress.count != nullptr ? 1 : head_group_for(head_bytes, (int)grid.y, (long long)grid.x * grid.y);
-  kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale,
-                                                                   a.k_scale, a.S, a.Hq, a.Hkv, head_group, a.causal, a.out_f32,
-                                                                   a.token_major, a.o_sb, a.o_sh, a.o_ss, a.replicas,
-                                                                   a.progress, a.lse_out, a.status, a.sticky, a.ticket);
+  kern<<<g.grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale, a.k_scale, a.S, a.Hq,
+                                                       a.Hkv, g.grouped, a.causal, a.out_f32, a.token_major, a.o_sb, a.o_sh,
+                                                       a.o_ss, a.replicas, a.progress, a.lse_out, a.status, a.sticky,
+                                                       a.ticket);
   return cudaGetLastError();
+}
+
+template <int MODE, int D, bool ROWS = false>
+cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
+  using C = Cfg<MODE, D>;
+  // completion reports want pairs to finish one by one
+  const size_t head_bytes = a.progress.count != nullptr ? ~(size_t)0
+                                                        : (size_t)a.S * D * (C::QK_ESIZE + C::V_ESIZE) / (size_t)(a.Hq / a.Hkv);
+  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + TILES * BM - 1) / (TILES * BM));
+  if constexpr (MODE != TC_SAGE) {
+    if (a.mask != nullptr) return launch_grid<MODE, D, ROWS, true, ORDER_ARG>(a, g, stream);
+  }
+  if constexpr (ROWS)
+    return launch_grid<MODE, D, true, false, ORDER_ARG>(a, g, stream);
+  else
+    return g.grouped ? launch_grid<MODE, D, false, false, ORDER_GROUPED>(a, g, stream)
+                     : launch_grid<MODE, D, false, false, ORDER_PLAIN>(a, g, stream);
 }
 
 }  // namespace

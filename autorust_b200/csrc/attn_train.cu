@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
                                                        const float* __restrict__ V, const float* __restrict__ dO,
                                                        const float* __restrict__ LSE, const float* __restrict__ delta,
                                                        const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq,
-                                                       int Hkv, int head_group, int causal) {
+                                                       int Hkv, int grouped, int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
   float* sQ = smem_t;
@@ -127,9 +127,9 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int tile, bh;
-  cta_order(head_group, tile, bh);
-  if (causal) tile = (int)gridDim.x - 1 - tile;  // the last query tile sees the most keys
+  const int bh = cta_head(grouped);
+  int tile = cta_tile(grouped);
+  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * BT;
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
                                                         const float* __restrict__ V, const float* __restrict__ dO,
                                                         const float* __restrict__ LSE, const float* __restrict__ delta,
                                                         const float* __restrict__ M, float* __restrict__ dK,
-                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int head_group,
+                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int grouped,
                                                         int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int tile, kvbh;
-  cta_order(head_group, tile, kvbh);  // (under a causal mask the first key tile sees the most queries)
+  const int kvbh = cta_head(grouped);
+  const int tile = cta_tile(grouped);  // (under a causal mask the first key tile sees the most queries)
   const int b = kvbh / Hkv, hk = kvbh - b * Hkv;
   const int group = Hq / Hkv;
   const int k0 = tile * BT;
@@ -363,7 +363,7 @@ __device__ __forceinline__ float prob(float s, float scale, const float* __restr
 __global__ void __launch_bounds__(256, 1)
     train_dq_wide_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                          const float* __restrict__ dO, const float* __restrict__ LSE, const float* __restrict__ delta,
-                         const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq, int Hkv, int head_group,
+                         const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq, int Hkv, int grouped,
                          int causal) {
   extern __shared__ __align__(16) float smem_t[];
   const int tid = threadIdx.x, grp = tid >> 7, gt = tid & 127;
@@ -373,9 +373,9 @@ __global__ void __launch_bounds__(256, 1)
   float* sK = sdO + OWN * LD + grp * DQ_GROUP;
   float* sV = sK + STREAM * LD;
   float* sDS = sV + STREAM * LD;
-  int tile, bh;
-  cta_order(head_group, tile, bh);
-  if (causal) tile = (int)gridDim.x - 1 - tile;  // the last query tile sees the most keys
+  const int bh = cta_head(grouped);
+  int tile = cta_tile(grouped);
+  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const size_t kv = (size_t)(b * Hkv + h / (Hq / Hkv)) * N * D;
   const int q0 = tile * OWN;
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(256, 1)
     train_dkv_wide_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                           const float* __restrict__ dO, const float* __restrict__ LSE, const float* __restrict__ delta,
                           const float* __restrict__ M, float* __restrict__ dK, float* __restrict__ dV, int N, int Hq, int Hkv,
-                          int head_group, int causal) {
+                          int grouped, int causal) {
   extern __shared__ __align__(16) float smem_t[];
   const int tid = threadIdx.x, half = tid >> 7, ht = tid & 127;
   const int tx = ht & 15, ty = ht >> 4;  // scores: queries ty + 8 * i, keys tx + 16 * jj
@@ -487,8 +487,8 @@ __global__ void __launch_bounds__(256, 1)
   float* stages = sV + OWN * LD;
   float* sP = stages + 2 * DKV_STAGE;
   float* sDS = sP + STREAM * LDS_DKV;
-  int tile, kvbh;
-  cta_order(head_group, tile, kvbh);  // (under a causal mask the first key tile sees the most queries)
+  const int kvbh = cta_head(grouped);
+  const int tile = cta_tile(grouped);  // (under a causal mask the first key tile sees the most queries)
   const int b = kvbh / Hkv, hk = kvbh - b * Hkv, group = Hq / Hkv;
   const int k0 = tile * OWN;
   const float scale = 1.0f / sqrtf((float)D);
@@ -623,21 +623,22 @@ cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches
   }
   const int wide_tiles = (a.S + wide::OWN - 1) / wide::OWN, group = a.Hq / a.Hkv;
   // f32 bytes that stream past a tile: the shared K and V, or Q and dO of the group's heads
-  const int dq_heads = head_group_for((size_t)a.S * D * 8 / (size_t)group, a.B * a.Hq, (long long)tiles * a.B * a.Hq);
-  const int dkv_heads = head_group_for((size_t)a.S * D * 8 * (size_t)group, a.B * a.Hkv, (long long)tiles * a.B * a.Hkv);
+  const size_t dq_bytes = (size_t)a.S * D * 8 / (size_t)group, dkv_bytes = (size_t)a.S * D * 8 * (size_t)group;
+  const CtaGrid gq = cta_grid(dq_bytes, a.B * a.Hq, wide_dq ? wide_tiles : tiles);
+  const CtaGrid gk = cta_grid(dkv_bytes, a.B * a.Hkv, wide_dkv ? wide_tiles : tiles);
   if (wide_dq)
-    wide::train_dq_wide_kernel<<<dim3(wide_tiles, a.B * a.Hq, 1), 256, wide::DQ_SMEM, stream>>>(
-        a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv, dq_heads, a.causal);
+    wide::train_dq_wide_kernel<<<gq.grid, 256, wide::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
+                                                                       a.Hq, a.Hkv, gq.grouped, a.causal);
   else
-    dq_kern<<<dim3(tiles, a.B * a.Hq, 1), 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
-                                                                    a.Hq, a.Hkv, dq_heads, a.causal);
+    dq_kern<<<gq.grid, 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv,
+                                                  gq.grouped, a.causal);
   (*launches)++;
   if (wide_dkv)
-    wide::train_dkv_wide_kernel<<<dim3(wide_tiles, a.B * a.Hkv, 1), 256, wide::DKV_SMEM, stream>>>(
-        a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv, dkv_heads, a.causal);
+    wide::train_dkv_wide_kernel<<<gk.grid, 256, wide::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
+                                                                         a.dv, a.S, a.Hq, a.Hkv, gk.grouped, a.causal);
   else
-    dkv_kern<<<dim3(tiles, a.B * a.Hkv, 1), 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
-                                                                       a.dv, a.S, a.Hq, a.Hkv, dkv_heads, a.causal);
+    dkv_kern<<<gk.grid, 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv,
+                                                   gk.grouped, a.causal);
   (*launches)++;
   return cudaGetLastError();
 }

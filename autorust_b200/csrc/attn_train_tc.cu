@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(TcBwd<D, DKV>::NUM_THREADS, 1)
 train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const float* __restrict__ LSE, const float* __restrict__ delta, const float* __restrict__ mask,
-                    float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int head_group, int causal,
+                    float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int grouped, int causal,
                     uint32_t* status, uint32_t* sticky) {
   using C = TcBwd<D, DKV>;
   constexpr int ST = C::STAGES, SL = C::SLOTS;
@@ -132,10 +132,10 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  int tile, bh;
-  cta_order(head_group, tile, bh);
+  const int bh = cta_head(grouped);
+  int tile = cta_tile(grouped);
   // dQ under a causal mask: the last query tile sees the most keys; dK/dV: the first key tile sees the most queries
-  if (!DKV && causal) tile = (int)gridDim.x - 1 - tile;
+  if (!DKV && causal) tile = cta_tiles(grouped) - 1 - tile;
   const int H = DKV ? Hkv : Hq, G = Hq / Hkv;
   const int b = bh / H, h = bh - b * H;               // DKV: h is a kv head
   const int row0 = tile * T;
@@ -411,9 +411,10 @@ cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
   const int heads = a.B * (DKV ? a.Hkv : a.Hq), group = a.Hq / a.Hkv;
   // bf16 bytes that stream past a tile: Q and dO of the group's heads, or the shared K and V
   const size_t head_bytes = (size_t)a.S * D * 4 * (DKV ? group : 1) / (DKV ? 1 : group);
-  kern<<<dim3((a.S + T - 1) / T, heads, 1), C::NUM_THREADS, C::SMEM_BYTES, stream>>>(
-      a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask, DKV ? a.dv : a.dq, DKV ? a.dk : nullptr, a.S, a.Hq, a.Hkv,
-      head_group_for(head_bytes, heads, (long long)((a.S + T - 1) / T) * heads), a.causal, a.status, a.sticky);
+  const CtaGrid g = cta_grid(head_bytes, heads, (a.S + T - 1) / T);
+  kern<<<g.grid, C::NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask,
+                                                          DKV ? a.dv : a.dq, DKV ? a.dk : nullptr, a.S, a.Hq, a.Hkv, g.grouped,
+                                                          a.causal, a.status, a.sticky);
   return cudaGetLastError();
 }
 

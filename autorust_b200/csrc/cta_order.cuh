@@ -1,10 +1,15 @@
-// The order in which the CTAs of a (tiles, batch x head) grid take their work, shared by the attention kernels.
+// The order in which the CTAs of a (tiles, batch x head) problem take their work, shared by the attention kernels.
 //
 // The hardware starts CTAs in the order of their linear index.  With the tiles of one head behind one another, the
-// last CTAs to start are those of the last heads, heavy and light ones alike, and a launch of one to a few waves ends
-// on whatever heavy CTA started last.  Here the heads are walked in groups whose streamed operands fit the L2
+// last CTAs to start are those of the last heads, heavy and light ones alike, and a launch of one to a few rounds ends
+// on whatever heavy CTA started last.  A grouped grid walks the heads in groups whose streamed operands fit the L2
 // together; inside a group the tile index is outermost, and each kernel counts its tiles from the heaviest (the far
 // end of a causal triangle, a full tile before a partial one), so that a group ends on its lightest CTAs.
+//   plain:    grid (tiles, heads)
+//   grouped:  grid (heads of a group, tiles, groups)
+// The order is in the shape of the grid, so that a kernel reads tile and head from its block index wherever it needs
+// them: with one computed from a linear index they stay in registers, which cost the D = 128 forward kernels 12 bytes
+// of spills and 3 % (B=4 H=32 S=8192 INT8 3.11 -> 3.25 ms).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -16,26 +21,33 @@ namespace ar {
 // a copy.  Heads beyond that would stream from memory once per tile instead of once per group.
 constexpr size_t HEAD_GROUP_BYTES = (size_t)32 << 20;
 
-// Heads per group when every head streams `bytes_per_head` (K/V heads shared by a GQA group count once).  Launches of
-// more than eight rounds keep the heads one by one: their end weighs little, and a head whose CTAs run side by side
-// reads its operands from nearby rows of L2 at about the same time (B=4 H=32 S=8192 D=128 INT8, 4096 CTAs: 3.11 ms head by
-// head, 3.25 ms in groups of ten).
-inline int head_group_for(size_t bytes_per_head, int heads, long long ctas) {
-  if (ctas > 8 * 148) return 1;
-  const size_t fit = HEAD_GROUP_BYTES / (bytes_per_head ? bytes_per_head : 1);
-  return fit < 1 ? 1 : fit < (size_t)heads ? (int)fit : heads;
+struct CtaGrid {
+  dim3 grid;
+  int grouped;
+};
+// `bytes_per_head`: what every head streams past its tiles (K/V heads shared by a GQA group count once); `split`
+// neighbouring CTAs share a tile.  Launches of more than eight rounds of CTAs stay plain: their end weighs little.
+inline CtaGrid cta_grid(size_t bytes_per_head, int heads, int tiles, int split = 1) {
+  int group = 1;
+  if ((long long)tiles * heads <= 8 * 148 && tiles <= 65535) {
+    const size_t fit = HEAD_GROUP_BYTES / (bytes_per_head ? bytes_per_head : 1);
+    for (int d = 2; d <= heads && (size_t)d <= fit; d++)
+      if (heads % d == 0) group = d;
+  }
+  if (group == 1) return {dim3((unsigned)(tiles * split), (unsigned)heads, 1), 0};
+  return {dim3((unsigned)(group * split), (unsigned)tiles, (unsigned)(heads / group)), 1};
 }
 
 #ifdef __CUDACC__
-// This CTA's tile (0 = first to run) and head in a grid of (tiles, heads).
-__device__ __forceinline__ void cta_order(int head_group, int& tile, int& head) {
-  const uint32_t lin = blockIdx.y * gridDim.x + blockIdx.x;
-  const uint32_t per = (uint32_t)head_group * gridDim.x;
-  const uint32_t grp = lin / per, in_grp = lin - grp * per;
-  const uint32_t heads = min((uint32_t)head_group, gridDim.y - grp * (uint32_t)head_group);
-  const uint32_t t = in_grp / heads;
-  tile = (int)t;
-  head = (int)(grp * (uint32_t)head_group + in_grp - t * heads);
+__device__ __forceinline__ int cta_tiles(int grouped, int split = 1) {
+  return (int)(grouped ? gridDim.y : gridDim.x / (uint32_t)split);
+}
+// This CTA's tile (0 = first to run).
+__device__ __forceinline__ int cta_tile(int grouped, int split = 1) {
+  return (int)(grouped ? blockIdx.y : blockIdx.x / (uint32_t)split);
+}
+__device__ __forceinline__ int cta_head(int grouped, int split = 1) {
+  return (int)(grouped ? blockIdx.z * (gridDim.x / (uint32_t)split) + blockIdx.x / (uint32_t)split : blockIdx.y);
 }
 #endif
 
