@@ -21,9 +21,10 @@
 // execute in issue order, which is what lets S(n + STAGES) overwrite the columns dQ(n) has read.
 // Floor of a step per SM at D = 64: S and dP 384 cycles of the tensor pipe (N = 64 with both operands from shared memory
 // reads 6 KB for 32 cycles of math), dK and dV 256, and 512 cycles for 8192 exponentials.  Measured, B=4 H=16 S=2048
-// D=64: dQ 163 -> 157 us (1190 cycles per step and SM), dK/dV 254 -> 213 us (1650) against two CTAs per SM that each
-// ran S/dP -> element-wise -> dQ with nothing issued ahead; the element-wise warps wait on TMEM loads (6.4 and 4.2
-// cycles per issue), with the tensor pipe 31 % and the MUFU unit 34-44 % busy.
+// D=64: dQ 163 -> 158 us (1030 cycles per step), dK/dV 254 -> 205 us (1250) against two CTAs per SM that each ran S/dP ->
+// element-wise -> dQ with nothing issued ahead.  What bounds it now is the MMA warp: of a step's 1030 cycles it spends
+// 760 issuing into a full tensor queue and 270 on its waits, its instructions queueing behind the element-wise warps';
+// the element-wise part takes a warpgroup 1050 of the 3060 cycles it has (2000 of 3750 in dK/dV).
 //
 // No atomics: a CTA owns its output tile and walks its reduction in a fixed order, so two launches give the same
 // bits.  Operands are bf16 copies of the f32 tensors (made by the caller of these kernels); P and dS are rounded to
@@ -35,6 +36,8 @@
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
 #include "cta_order.cuh"
+
+#include <cooperative_groups.h>
 
 namespace ar {
 namespace {
@@ -57,16 +60,17 @@ struct TcBwd {
   static constexpr int NUM_BARS = 2 + 2 * SLOTS + 2 * STAGES;
   static constexpr int SMEM_BYTES = 2 * OWN_BYTES + SLOTS * 2 * STREAM_BYTES + ROWVALS_BYTES + NUM_BARS * 8 + 16 + 1024;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+  static_assert(ACC_COLS * T * 4 <= 2 * OWN_BYTES + SLOTS * 2 * STREAM_BYTES, "accumulators pass through the tiles");
   static constexpr int KSTEPS_D = D / 16;             // k-steps of a product over d
   static constexpr int KSTEPS_NH = NH / 16;           // k-steps of a product over one step's rows
   static constexpr uint32_t IDESC_SS = make_idesc(1, 1, 1, 0, 0, T, NH);  // bf16 x bf16 -> f32, both K-major, N = NH
   static constexpr uint32_t IDESC_TS = make_idesc(1, 1, 1, 0, 1, T, D);   // A from TMEM, B MN-major, N = D
   static constexpr int W_PROD = 4 * STAGES, W_MMA = W_PROD + 1;           // two more warps complete the last warpgroup
   static constexpr int NUM_THREADS = 128 * STAGES + 128;
-  // registers per thread: launched with LAUNCH_REGS, then moved from the last warpgroup to the element-wise ones
+  // registers per thread: launched with LAUNCH_REGS, then (two stages) moved from the last warpgroup to the others
   static constexpr int LAUNCH_REGS = STAGES == 3 ? 128 : 168;
-  static constexpr int EW_REGS = STAGES == 3 ? 144 : 208;
-  static constexpr int SERVICE_REGS = STAGES == 3 ? 80 : 88;
+  static constexpr int EW_REGS = STAGES == 3 ? 128 : 192;
+  static constexpr int SERVICE_REGS = STAGES == 3 ? 128 : 120;
   static_assert(128 * STAGES * EW_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
   static_assert(LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
 };
@@ -103,13 +107,15 @@ __device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* m, ui
 
 // dQ (DKV = false): own rows are queries (A tiles Q, dO), K and V stream.  dK/dV (DKV = true): own rows are keys (A
 // tiles K, V), Q and dO of the group's query heads stream.
+// dK/dV with split > 1: a cluster of `split` CTAs shares a key tile, each walks its part of the group's query heads, and
+// the CTAs add their accumulators through distributed shared memory, column by column in rank order.
 template <int D, bool DKV>
 __global__ void __launch_bounds__(TcBwd<D, DKV>::NUM_THREADS, 1)
 train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const float* __restrict__ LSE, const float* __restrict__ delta, const float* __restrict__ mask,
-                    float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int grouped, int causal,
-                    uint32_t* status, uint32_t* sticky) {
+                    float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int grouped, int split,
+                    int causal, uint32_t* status, uint32_t* sticky) {
   using C = TcBwd<D, DKV>;
   constexpr int ST = C::STAGES, SL = C::SLOTS;
   extern __shared__ uint8_t smem_raw[];
@@ -132,18 +138,22 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int bh = cta_head(grouped);
-  int tile = cta_tile(grouped);
+  if (!DKV) split = 1;
+  const int bh = cta_head(grouped, split);
+  int tile = cta_tile(grouped, split);
+  const int rank = DKV && split > 1 ? (int)(blockIdx.x % (uint32_t)split) : 0;
   // dQ under a causal mask: the last query tile sees the most keys; dK/dV: the first key tile sees the most queries
   if (!DKV && causal) tile = cta_tiles(grouped) - 1 - tile;
   const int H = DKV ? Hkv : Hq, G = Hq / Hkv;
+  const int heads = DKV ? G / split : 1;              // query heads this CTA walks, from g0 on
+  const int g0 = rank * heads;
   const int b = bh / H, h = bh - b * H;               // DKV: h is a kv head
   const int row0 = tile * T;
   // the steps this tile walks: dQ -- blocks of 64 keys; dK/dV -- blocks of 64 queries, head by head of the group
   const int first = DKV && causal ? row0 / NH : 0;    // queries before the key tile see none of it
   const int last = !DKV && causal ? (min(N, row0 + T) + NH - 1) / NH : (N + NH - 1) / NH;
   const int per_head = last - first;
-  const int steps = DKV ? G * per_head : per_head;
+  const int steps = heads * per_head;
 
   if (warp == C::W_PROD && lane == 0) {
     *abort_flag = 0;
@@ -169,7 +179,24 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t tb = *tmem_slot;
   const uint32_t col_acc = ST * 2 * NH;               // accumulators: dQ | dV, dK
 
-  if (warp >= C::W_PROD) setmaxnreg_dec<C::SERVICE_REGS>();
+  bool finished = false;  // (element-wise warps)
+  // 32 accumulator columns of one of the CTA's rows to the output they belong to
+  auto store_chunk = [&](const uint32_t(&ov)[32], int c, int row) {
+    const bool second = DKV && c >= D / 32;  // dV first, then dK
+    const int cd = second ? c - D / 32 : c;
+    const float f = DKV && !second ? 1.0f : 1.0f / sqrtf((float)D);
+    if (row < N) {
+      float4* dst = (float4*)((second ? out1 : out0) + ((size_t)bh * N + row) * D + cd * 32);
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        dst[i] = make_float4(__uint_as_float(ov[4 * i]) * f, __uint_as_float(ov[4 * i + 1]) * f,
+                             __uint_as_float(ov[4 * i + 2]) * f, __uint_as_float(ov[4 * i + 3]) * f);
+    }
+  };
+
+  if constexpr (C::EW_REGS > C::LAUNCH_REGS) {
+    if (warp >= C::W_PROD) setmaxnreg_dec<C::SERVICE_REGS>();
+  }
   if (warp == C::W_PROD) {
     if (lane == 0) {
       const int own_h = h;
@@ -181,7 +208,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int sl = n % SL;
         const int g = DKV ? n / per_head : 0;
         const int r = (first + n - g * per_head) * NH;
-        const int sh = DKV ? h * G + g : h / G;       // head of the streamed tensors
+        const int sh = DKV ? h * G + g0 + g : h / G;       // head of the streamed tensors
         if (n >= SL && !mbar_wait(&slot_empty[sl], ((n / SL) - 1) & 1, wctx, 0x50)) break;
         uint8_t* dst = ring + sl * 2 * C::STREAM_BYTES;
         mbar_arrive_expect_tx(&slot_full[sl], 2 * C::STREAM_BYTES);
@@ -198,8 +225,10 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint64_t k_proto = make_sdesc_sw128(0, 16, 1024);         // K-major
     const uint64_t mn_proto = make_sdesc_sw128(0, NH * 128, 1024);  // MN-major: 64-column boxes NH * 128 bytes apart
     const uint32_t k_hi = (uint32_t)(k_proto >> 32), mn_hi = (uint32_t)(mn_proto >> 32);
-    const uint32_t a0 = (uint32_t)k_proto | (smem_u32(own0) >> 4), a1 = (uint32_t)k_proto | (smem_u32(own1) >> 4);
-    const uint32_t ring0 = smem_u32(ring) >> 4;
+    // a descriptor holds 18 bits of an address; in a cluster the rank lies above them, which would fall into the offsets
+    auto desc_addr = [](const void* p) { return (smem_u32(p) & 0x3ffffu) >> 4; };
+    const uint32_t a0 = (uint32_t)k_proto | desc_addr(own0), a1 = (uint32_t)k_proto | desc_addr(own1);
+    const uint32_t ring0 = desc_addr(ring);
     bool ok = __all_sync(0xffffffffu, mbar_wait(own_full, 0, wctx, 0x51));
     auto scores = [&](int n) {  // S and dP of step n into its stage
       const int st = n % ST;
@@ -231,7 +260,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (ok) commit_one(acc_full);
   } else if (warp < C::W_PROD) {
     // element-wise: warpgroup wg takes steps wg, wg + STAGES, ...; thread r owns the CTA's row row0 + r
-    setmaxnreg_inc<C::EW_REGS>();
+    if constexpr (C::EW_REGS > C::LAUNCH_REGS) setmaxnreg_inc<C::EW_REGS>();
     const int wg = warp >> 2;
     const int r = tid & 127;
     const int row = row0 + r;
@@ -251,7 +280,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     auto fetch = [&](int n) {
       const int g = n / per_head, qrow = (first + n - g * per_head) * NH + (r & (NH - 1));
       if (n >= steps || qrow >= N) return 0.f;
-      const size_t at = (size_t)(b * Hq + h * G + g) * N + qrow;
+      const size_t at = (size_t)(b * Hq + h * G + g0 + g) * N + qrow;
       return r < NH ? -LSE[at] * LOG2E : -delta[at];
     };
     float next_val = 0.f;
@@ -263,30 +292,42 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if constexpr (DKV) {
         vals[(it & 1) * (2 * NH) + r] = next_val;
         next_val = fetch(n + ST);
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
+        ok = bar_all(1 + wg, 128, ok);  // (a warp whose wait ran out takes the others with it)
+        if (!ok) break;
       }
       const int g = DKV ? n / per_head : 0;
       const int c0 = (first + n - g * per_head) * NH;  // first streamed row: key (dQ) or query (dK/dV)
       ok = __all_sync(0xffffffffu, mbar_wait(&s_full[wg], it & 1, wctx, 0x54));
-      if (!ok) break;
+      if (!ok) {
+        if constexpr (DKV) continue;
+        break;
+      }
       tc_fence_after();
       // a step whose 128 x 64 block lies inside the sequence, on the visible side of the causal diagonal and under no
       // additive mask needs none of the per-element tests: two lanes per instruction
       const bool interior = mask == nullptr && row0 + T <= N && c0 + NH <= N &&
                             (!causal || (DKV ? row0 + T - 1 <= c0 : c0 + NH - 1 <= row0));
-#pragma unroll 1
-      for (int c = 0; c < NH / 32; c++) {
-        uint32_t sv[32], pv[32], pk[16], dk[16];
-        tmem_ld32(tS + c * 32, sv);
-        tmem_ld32(tdP + c * 32, pv);
-        tmem_wait_ld();
+      // 16 columns at a time, the next 16 on their way meanwhile: [0, 16) of a buffer are scores, [16, 32) dP
+      uint32_t buf[2][32];
+      tmem_ld16(tS, buf[0]);
+      tmem_ld16(tdP, buf[0] + 16);
+#pragma unroll 2
+      for (int c = 0; c < NH / 16; c++) {
+        uint32_t* sv = buf[c & 1];
+        uint32_t* pv = sv + 16;
+        tmem_wait_ld32(sv);
+        if (c + 1 < NH / 16) {
+          tmem_ld16(tS + (c + 1) * 16, buf[(c + 1) & 1]);
+          tmem_ld16(tdP + (c + 1) * 16, buf[(c + 1) & 1] + 16);
+        }
+        uint32_t pk[8], dk[8];
         if (interior) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
+          for (int i = 0; i < 16; i += 4) {
             float4 l = make_float4(nlse, nlse, nlse, nlse), d = make_float4(ndl, ndl, ndl, ndl);
             if constexpr (DKV) {
-              l = *(const float4*)(lv + c * 32 + i);
-              d = *(const float4*)(lv + NH + c * 32 + i);
+              l = *(const float4*)(lv + c * 16 + i);
+              d = *(const float4*)(lv + NH + c * 16 + i);
             }
 #pragma unroll
             for (int e = 0; e < 4; e += 2) {
@@ -303,11 +344,11 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
+          for (int i = 0; i < 16; i += 2) {
             float p[2], ds[2];
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-              const int cc = c * 32 + i + e;
+              const int cc = c * 16 + i + e;
               const int key = DKV ? row : c0 + cc, qrow = DKV ? c0 + cc : row;
               const float l = DKV ? lv[cc] : nlse, d = DKV ? lv[NH + cc] : ndl;
               float x = __uint_as_float(sv[i + e]) * scale_log2;
@@ -322,10 +363,10 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         // over the columns that have been read: dS | P^T over S^T, dS^T over dP^T
         if constexpr (DKV) {
-          tmem_st16(tS + c * 16, pk);
-          tmem_st16(tdP + c * 16, dk);
+          tmem_st8(tS + c * 8, pk);
+          tmem_st8(tdP + c * 8, dk);
         } else {
-          tmem_st16(tS + c * 16, dk);
+          tmem_st8(tS + c * 8, dk);
         }
       }
       tmem_wait_st();
@@ -335,24 +376,48 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wctx, 0x55));
     if (ok) {
       tc_fence_after();
-      const float scale = 1.0f / sqrtf((float)D);
       // the accumulators' 32-column chunks, shared out over the warpgroups
 #pragma unroll 1
       for (int c = wg; c < C::ACC_COLS / 32; c += ST) {
-        const bool second = DKV && c >= D / 32;  // dV first, then dK
-        const int cd = second ? c - D / 32 : c;
-        const float f = DKV && !second ? 1.0f : scale;
         uint32_t ov[32];
         tmem_ld32(tmem_addr(tb, lane_base, col_acc + c * 32), ov);
         tmem_wait_ld();
-        if (row < N) {
-          float4* dst = (float4*)((second ? out1 : out0) + ((size_t)bh * N + row) * D + cd * 32);
+        if (DKV && split > 1) {  // every MMA and copy is done: the tiles' memory takes the accumulators, [column][row]
+          float* buf = (float*)smem + (c * 32) * T + r;
 #pragma unroll
-          for (int i = 0; i < 8; i++)
-            dst[i] = make_float4(__uint_as_float(ov[4 * i]) * f, __uint_as_float(ov[4 * i + 1]) * f,
-                                 __uint_as_float(ov[4 * i + 2]) * f, __uint_as_float(ov[4 * i + 3]) * f);
+          for (int i = 0; i < 32; i++) buf[i * T] = __uint_as_float(ov[i]);
+        } else {
+          store_chunk(ov, c, row);
         }
       }
+    }
+    finished = ok;
+  }
+  if constexpr (DKV) {
+    if (split > 1) {  // (every thread of the cluster comes by here, whatever its waits returned)
+      namespace cg = cooperative_groups;
+      cg::cluster_group cluster = cg::this_cluster();
+      __syncwarp();  // the cluster barrier counts whole warps: the producer's lanes meet again first
+      cluster.sync();
+      if (finished && warp < C::W_PROD) {
+        const int r = tid & 127;
+        const int chunks = C::ACC_COLS / 32, mine = (rank * chunks) / split, end = ((rank + 1) * chunks) / split;
+#pragma unroll 1
+        for (int c = mine + (warp >> 2); c < end; c += ST) {
+          uint32_t ov[32];
+#pragma unroll
+          for (int i = 0; i < 32; i++) ov[i] = 0u;
+#pragma unroll 1
+          for (int k = 0; k < split; k++) {
+            const float* buf = cluster.map_shared_rank((float*)smem, k) + (c * 32) * T + r;
+#pragma unroll
+            for (int i = 0; i < 32; i++) ov[i] = __float_as_uint(__uint_as_float(ov[i]) + buf[i * T]);
+          }
+          store_chunk(ov, c, row0 + r);
+        }
+      }
+      __syncwarp();
+      cluster.sync();  // nobody's shared memory goes away while another CTA reads it
     }
   }
   tc_fence_before();
@@ -408,14 +473,33 @@ cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int heads = a.B * (DKV ? a.Hkv : a.Hq), group = a.Hq / a.Hkv;
+  const int heads = a.B * (DKV ? a.Hkv : a.Hq), group = a.Hq / a.Hkv, tiles = (a.S + T - 1) / T;
   // bf16 bytes that stream past a tile: Q and dO of the group's heads, or the shared K and V
   const size_t head_bytes = (size_t)a.S * D * 4 * (DKV ? group : 1) / (DKV ? 1 : group);
-  const CtaGrid g = cta_grid(head_bytes, heads, (a.S + T - 1) / T);
-  kern<<<g.grid, C::NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask,
-                                                          DKV ? a.dv : a.dq, DKV ? a.dk : nullptr, a.S, a.Hq, a.Hkv, g.grouped,
-                                                          a.causal, a.status, a.sticky);
-  return cudaGetLastError();
+  // dK/dV of a GQA group: few CTAs with `group` times a head's steps each.  Below four of them per SM the query heads of
+  // the group are dealt out over a cluster (its largest divisor up to 8), so that the last CTA to end -- under a causal
+  // mask the one of the first keys -- has a `split`-th of the work.
+  // Measured, B=2 Hq=16 Hkv=4 S=1531 D=128 causal: 168 us for dK/dV before the steps in flight and the split, 93 with both.
+  int split = 1;
+  if (DKV && (long long)tiles * heads < 4 * 148)
+    for (int d = 2; d <= 8; d++)
+      if (group % d == 0) split = d;
+  cudaLaunchConfig_t cfg = {};
+  const CtaGrid g = cta_grid(head_bytes, heads, tiles, split);
+  cfg.gridDim = g.grid;
+  cfg.blockDim = dim3(C::NUM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = C::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, a.tm_q, a.tm_k, a.tm_v, a.tm_do, a.lse, a.delta, a.mask, DKV ? a.dv : a.dq,
+                            DKV ? a.dk : (float*)nullptr, a.S, a.Hq, a.Hkv, g.grouped, split, a.causal,
+                            a.status, a.sticky);
 }
 
 }  // namespace
