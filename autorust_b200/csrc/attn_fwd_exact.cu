@@ -266,26 +266,39 @@ cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// Rounds of one CTA per SM that a launch takes with tiles of `bq` rows, times the rows of a tile: proportional to the
-// time if every tile size worked at the same rate.
-long long rounds_x_rows(const ExactArgs& a, int bq) {
-  const long long ctas = (long long)((a.S + bq - 1) / bq) * a.B * a.Hq;
-  return (ctas + 147) / 148 * bq;
+// What a launch with tiles of `rows` rows costs: rounds of one CTA per SM, each as long as its rows plus the part of a
+// CTA that does not depend on them (loads, softmax, combination: about as much as 8 rows).
+long long rounds_cost(const ExactArgs& a, int rows) {
+  const long long ctas = (long long)((a.S + rows - 1) / rows) * a.B * a.Hq;
+  return (ctas + 147) / 148 * (rows + 8);
 }
 
 }  // namespace
 
 cudaError_t launch_attn_exact(const ExactArgs& a, cudaStream_t stream) {
-  // The 8 x 8 blocks work at about 1.6 times the rate of the 4 x 4 ones, whose tiles of 16 rows spread a small call over
-  // the chip.  The tile that ends first is taken.
-  if (a.D == 64) {
-    if (5 * rounds_x_rows(a, 128) <= 8 * rounds_x_rows(a, 16)) return launch_exact<64, 8, 8, 16, 2>(a, stream);
-    return launch_exact<64, 4, 16, 4, 4>(a, stream);
+  // Few rows: 4 columns of threads per key group and 8 to 32 rows per tile spread the call over the chip; among them the
+  // height whose rounds cost least (a 16-row tile leaves B=1 H=12 S=197 156 CTAs, two rounds, 18.7 us; 20 rows 120 CTAs,
+  // 11.4 us).  Many rows: the 8 x 8 blocks, which work at about 1.6 times the rate of the others.
+  const int wide = a.D == 64 ? 128 : 64;
+  int rows = 16;
+  for (int r : {8, 12, 20, 24, 32})
+    if (rounds_cost(a, r) < rounds_cost(a, rows)) rows = r;
+  if (5 * rounds_cost(a, wide) <= 8 * rounds_cost(a, rows)) rows = wide;
+#define AR_EXACT(D_, G_)                                                     \
+  if (a.D == D_) {                                                           \
+    switch (rows) {                                                          \
+      case 8: return launch_exact<D_, 2, 16, 4, G_>(a, stream);              \
+      case 12: return launch_exact<D_, 3, 16, 4, G_>(a, stream);             \
+      case 16: return launch_exact<D_, 4, 16, 4, G_>(a, stream);             \
+      case 20: return launch_exact<D_, 5, 16, 4, G_>(a, stream);             \
+      case 24: return launch_exact<D_, 6, 16, 4, G_>(a, stream);             \
+      case 32: return launch_exact<D_, 8, 16, 4, G_>(a, stream);             \
+      default: return launch_exact<D_, D_ == 64 ? 8 : 4, 8, 16, 2>(a, stream); \
+    }                                                                        \
   }
-  if (a.D == 128) {
-    if (5 * rounds_x_rows(a, 64) <= 8 * rounds_x_rows(a, 16)) return launch_exact<128, 4, 8, 16, 2>(a, stream);
-    return launch_exact<128, 4, 16, 4, 2>(a, stream);
-  }
+  AR_EXACT(64, 4)
+  AR_EXACT(128, 2)
+#undef AR_EXACT
   return cudaErrorInvalidValue;
 }
 
