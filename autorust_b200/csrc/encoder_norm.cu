@@ -49,6 +49,20 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const uint4* __restr
   if (row >= rows) return;
   const uint4* xr = x + row * chunks;
   const uint4* rr = r ? r + row * chunks : nullptr;
+  // everything a row needs is requested before the first reduction: gamma and beta, needed last, would otherwise start
+  // a second round of latency behind it (wide rows keep them out of the registers)
+  constexpr bool EARLY = NCH <= 4;
+  uint4 gw[EARLY ? NCH : 1], bw[EARLY ? NCH : 1];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int c = 0; c < NCH; c++) {
+      const int idx = lane + 32 * c;
+      if (idx < chunks) {
+        gw[c] = gamma[idx];
+        bw[c] = beta[idx];
+      }
+    }
+  }
   float v[NCH][8];
   float total = 0.f;
 #pragma unroll
@@ -89,8 +103,8 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const uint4* __restr
     const int idx = lane + 32 * c;
     if (idx < chunks) {
       float g[8], b[8], o[8];
-      unpack8(gamma[idx], g);
-      unpack8(beta[idx], b);
+      unpack8(EARLY ? gw[EARLY ? c : 0] : gamma[idx], g);
+      unpack8(EARLY ? bw[EARLY ? c : 0] : beta[idx], b);
 #pragma unroll
       for (int i = 0; i < 8; i++) o[i] = (v[c][i] - mean) * inv * g[i] + b[i];
       y[row * chunks + idx] = pack8(o);
