@@ -12,8 +12,10 @@
 //   TMEM (256 columns): S [0, 256); P (bf16, two per column) overwrites [0, 128) as S is read; O takes [128, 192) once
 //   all of S has been read.
 //
-// Bound: the MUFU unit (128 x S exponentials per item, a quarter of them evaluated on the FMA pipe) while the other CTA
-// of the SM is in its MMAs, waits and stores.
+// Bound: latency.  Measured, B=64 H=12 S=197 on strided views: 45.8 us in the form with two key steps that this replaces, 29.5 us
+// here against 11.8 us for its 77 MB; the MUFU unit and the issue slots are about a third busy.  An item's chain is 7700
+// cycles: maximum 1070, exponentials 2800 (a quarter of them on the FMA pipe), P V with its hand-overs 1350, from O
+// read to the next scores 2300, and two CTAs per SM are what TMEM holds.
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
 #include "softmax_math.cuh"
@@ -66,11 +68,15 @@ __device__ __forceinline__ void exclude(uint32_t* sv, int first_out) {
     if (i >= first_out) sv[i] = 0xff800000u;
 }
 
+// EXTRA: further output buffers or completion reports, an instantiation of its own (with both in the plain one: 29.5 ->
+// 37.9 us for the shape above).
+template <bool EXTRA>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
     attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, void* __restrict__ out, int N, int Hq, int Hkv, int items,
                           int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
-                          float* __restrict__ lse_out, uint32_t* status, uint32_t* sticky, uint32_t ticket) {
+                          const OutReplicas reps, const OutProgress progress, float* __restrict__ lse_out, uint32_t* status,
+                          uint32_t* sticky, uint32_t ticket) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
@@ -213,6 +219,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       // (uniform) no lane of the CTA excludes a column before this chunk
       const int whole = causal ? it.q0 >> 5 : N >> 5;
       float m = NEG, l = 0.f;
+      do {  // (left early by a warp whose wait ran out or whose rows lie past the sequence end)
       ok = __all_sync(0xffffffffu, mbar_wait(s_full, n & 1, wctx, 0x66));
       if (!ok) break;
       tc_fence_after();
@@ -276,7 +283,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       tmem_wait_ld();
       tc_fence_before();
       mbar_arrive(o_empty);  // the next item's Q K^T may start under this item's stores
-      if (!rows_in) continue;
+      if (!rows_in) break;
       const float inv = l > 0.f ? 1.0f / l : 0.f;
       const long long base = (long long)it.b * o_sb + (long long)it.h * o_sh;
       if (lse_out != nullptr && row < N)
@@ -306,9 +313,32 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
         for (int x = 0; x < 8; x++) {
           const int rr = warp * 32 + 4 * x + (lane >> 3), ch = lane & 7;
           const uint4 w = *(const uint4*)(stage + rr * 128 + ((ch ^ (rr & 7)) * 16));
-          if (it.q0 + rr < N) *(uint4*)((uint16_t*)out + base + (long long)(it.q0 + rr) * o_ss + ch * 8) = w;
+          if (it.q0 + rr < N) {
+            const size_t off = (size_t)(base + (long long)(it.q0 + rr) * o_ss + ch * 8) * 2;
+            if (EXTRA && reps.multicast) {
+              multimem_st16((uint8_t*)reps.p[0] + off, w);  // one store, delivered to every GPU by the switch
+            } else {
+              *(uint4*)((uint8_t*)out + off) = w;
+              if constexpr (EXTRA) {
+                for (int e = 0; e < reps.n; e++) *(uint4*)((uint8_t*)reps.p[e] + off) = w;
+              }
+            }
+          }
         }
         __syncwarp();
+      }
+      } while (false);
+      if (EXTRA && progress.count != nullptr) {
+        // Completion report, as in the long kernel: the barrier orders the item's rows before this thread, the count
+        // releases them device-wide, and the pair's last item releases the flag to the host.
+        ok = bar_all(1, 128, ok);
+        if (ok && tid == 0) {
+          const int pair = it.b * Hq + it.h;
+          uint32_t before;
+          asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(progress.count + pair) : "memory");
+          if (before + 1u == (uint32_t)qtiles)
+            asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(progress.flag + pair), "r"(progress.epoch) : "memory");
+        }
       }
     }
   }
@@ -320,17 +350,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
 }  // namespace
 
 bool attn_short_takes(const TcArgs& a) {
-  return a.mode == TC_BF16 && a.D == D && a.S <= KEYS && a.mask == nullptr && a.replicas.n == 0 && a.progress.count == nullptr;
+  return a.mode == TC_BF16 && a.D == D && a.S <= KEYS && a.mask == nullptr;
 }
 
-cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream) {
+template <bool EXTRA>
+cudaError_t launch_short(const TcArgs& a, cudaStream_t stream) {
+  auto kern = attn_fwd_short_kernel<EXTRA>;
   static bool configured[64] = {};
   static int sm_count[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(attn_fwd_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
@@ -338,10 +370,14 @@ cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream) {
   }
   const int items = ((a.S + BM - 1) / BM) * a.B * a.Hq;
   const int resident = 2 * (dev < 64 ? sm_count[dev] : 148);
-  attn_fwd_short_kernel<<<items < resident ? items : resident, NUM_THREADS, SMEM_BYTES, stream>>>(
+  kern<<<items < resident ? items : resident, NUM_THREADS, SMEM_BYTES, stream>>>(
       a.tm_q, a.tm_k, a.tm_v, a.out, a.S, a.Hq, a.Hkv, items, a.causal, a.out_f32, a.token_major, a.o_sb, a.o_sh, a.o_ss,
-      a.lse_out, a.status, a.sticky, a.ticket);
+      a.replicas, a.progress, a.lse_out, a.status, a.sticky, a.ticket);
   return cudaGetLastError();
+}
+
+cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream) {
+  return a.replicas.n > 0 || a.progress.count != nullptr ? launch_short<true>(a, stream) : launch_short<false>(a, stream);
 }
 
 }  // namespace ar

@@ -122,40 +122,8 @@ __global__ void __launch_bounds__(MEAN_SLOTS * D) k_mean_kernel(const void* __re
   if (tid < D) k_mean[(size_t)blockIdx.x * D + tid] = total * (1.0f / (float)S);
 }
 
-// The same mean of longer sequences in two launches: one CTA per span of 128 tokens leaves the span's sums in scratch,
-// then one CTA per (batch, kv head) adds them in span order -- the order, and therefore every bit, of the single-CTA
-// kernel.  Bound: HBM, K read once with every SM's loads in flight from the start.  Measured, 16 pairs of S=3001
-// D=128: 25 us for a cluster of eight CTAs per pair, 12.6 us for the two launches; 128 pairs of S=8192: 61 us for the
-// single-CTA kernel, 132 us.
-// grid = (spans, B * Hkv); thread (g, c) as above.
-template <int DTYPE, int D>
-__global__ void __launch_bounds__(D) k_span_kernel(const void* __restrict__ K, float* __restrict__ span_sums, int S) {
-  constexpr int CH = D / 8;
-  __shared__ float run_sums[8][D];
-  const int tid = threadIdx.x, g = tid / CH, c = tid % CH;
-  const size_t base = (size_t)blockIdx.y * S * D;
-  const int t0 = blockIdx.x * 128 + g * 16;
-  float x[16][8];
-#pragma unroll
-  for (int t = 0; t < 16; t++)
-    if (t0 + t < S) load8<DTYPE>(K, base + (size_t)(t0 + t) * D + c * 8, x[t]);
-  float acc[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) acc[i] = 0.f;
-#pragma unroll
-  for (int t = 0; t < 16; t++)
-    if (t0 + t < S) {
-#pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += x[t][i];
-    }
-#pragma unroll
-  for (int i = 0; i < 8; i++) run_sums[g][c * 8 + i] = acc[i];
-  __syncthreads();
-  float s = 0.f;  // thread d: the 8 run sums, left to right
-#pragma unroll
-  for (int gg = 0; gg < 8; gg++) s += run_sums[gg][tid];
-  span_sums[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * D + tid] = s;
-}
+// The mean of longer sequences from the span sums that the quantiser's first launch leaves (see below): one CTA per
+// (batch, kv head) adds them in span order -- the order, and therefore every bit, of the kernel above.
 template <int D>
 __global__ void __launch_bounds__(D) k_mean_of_spans_kernel(const float* __restrict__ span_sums, float* __restrict__ k_mean,
                                                             int S, int nspan) {
@@ -205,6 +173,12 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const void* __restri
 // shared-memory ring with a bulk copy while the CTA reduces and stores block i, so that each SM keeps
 // tens of KB of reads in flight the whole time instead of one load-reduce-store round per CTA.
 // Needs 16-byte aligned Q and K.
+// With smoothing, K can only be quantised when its mean is known, but Q can be before: sequences of more than
+// MEAN_SLOTS spans take two launches of this kernel, Q blocks quantised and K blocks summed (PART_Q_AND_SUMS), and after
+// k_mean_of_spans_kernel the K blocks quantised (PART_K).  The sum pass over K then streams beside Q's instead of
+// in a launch of its own.  Measured, mean and quantisation: 16 K heads of S=3001 with 64 of Q 48
+// us (cluster mean) -> 31, B=4 H=32 S=8192 214 -> 208.
+enum { PART_ALL, PART_Q_AND_SUMS, PART_K };
 template <int DTYPE, int D>
 struct QuantPipe {
   static constexpr int ES = DTYPE == 1 ? 2 : 4;
@@ -232,12 +206,27 @@ __device__ __forceinline__ void load8_shared(const uint8_t* p, float* x) {
   }
 }
 
+template <int DTYPE>
+__device__ __forceinline__ void load4_shared(const uint8_t* p, float* x) {
+  if constexpr (DTYPE == 1) {
+    const uint2 w = *(const uint2*)p;
+    x[0] = __uint_as_float(w.x << 16);
+    x[1] = __uint_as_float(w.x & 0xffff0000u);
+    x[2] = __uint_as_float(w.y << 16);
+    x[3] = __uint_as_float(w.y & 0xffff0000u);
+  } else {
+    const float4 a = *(const float4*)p;
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+  }
+}
+
 template <int DTYPE, int D>
 __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restrict__ Q, const void* __restrict__ K,
                                                             const float* __restrict__ k_mean, int8_t* __restrict__ q8,
                                                             int8_t* __restrict__ k8, float* __restrict__ q_scale,
                                                             float* __restrict__ k_scale, int S, int BHq, int BHk,
-                                                            int smooth, int fp8, uint32_t* status, uint32_t* sticky) {
+                                                            int smooth, int fp8, int part, float* __restrict__ span_sums,
+                                                            uint32_t* status, uint32_t* sticky) {
   using P = QuantPipe<DTYPE, D>;
   constexpr int CH = D / 8;
   constexpr int NCHUNK = 128 * CH / 256;
@@ -246,10 +235,12 @@ __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restri
   uint8_t* ring = (uint8_t*)(((uintptr_t)qp_smem_raw + 127) & ~(uintptr_t)127);
   __shared__ uint64_t full[ST];
   __shared__ float warp_max[2][8];
+  __shared__ float run_sums[8][D];
   __shared__ uint32_t abort_flag;
   const int tid = threadIdx.x;
   const int nblk = (S + 127) / 128;
   const int q_items = BHq * nblk, items = (BHq + BHk) * nblk;
+  const int first = (part == PART_K ? q_items : 0) + blockIdx.x;
   if (tid == 0) {
     abort_flag = 0;
     for (int i = 0; i < ST; i++) arptx::mbar_init(&full[i], 1);
@@ -269,13 +260,13 @@ __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restri
   };
   if (tid == 0) {
     for (int i = 0; i < ST - 1; i++) {
-      const int w = blockIdx.x + i * gridDim.x;
+      const int w = first + i * gridDim.x;
       if (w < items) issue(w, i);
     }
   }
   const int c = tid % CH;
   int it = 0;
-  for (int w = blockIdx.x; w < items; w += gridDim.x, it++) {
+  for (int w = first; w < items; w += gridDim.x, it++) {
     const int stage = it % ST;
     // the stage that block it + ST - 1 goes to was read in iteration it - 1; every thread is past that
     // read (the barrier at the end of the previous iteration), and the fence orders those generic-proxy
@@ -294,13 +285,38 @@ __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restri
     float mu[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) mu[i] = 0.f;
-    if (is_k && smooth) {
+    if (is_k && smooth && part != PART_Q_AND_SUMS) {
 #pragma unroll
       for (int i = 0; i < 8; i++) mu[i] = k_mean[(size_t)bh * D + c * 8 + i];
     }
     const bool ok = arptx::mbar_wait(&full[stage], (uint32_t)(it / ST) & 1u, arptx::WaitCtx{&abort_flag, status, sticky}, 0x40);
     if (!__syncthreads_and(ok)) break;  // a copy that never lands: the status word says so, the CTA leaves together
     const uint8_t* blockp = ring + stage * P::BLOCK_BYTES;
+    if (is_k && part == PART_Q_AND_SUMS) {
+      // thread (run of 16 tokens, 4 channels): the run left to right; then thread d: the 8 runs left to right
+      const int g = tid / (D / 4), c4 = tid % (D / 4);
+      if (g < 8) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int t = 0; t < 16; t++)
+          if (t0 + g * 16 + t < S) {
+            float v[4];
+            load4_shared<DTYPE>(blockp + (size_t)((g * 16 + t) * D + c4 * 4) * P::ES, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i] += v[i];
+          }
+#pragma unroll
+        for (int i = 0; i < 4; i++) run_sums[g][c4 * 4 + i] = acc[i];
+      }
+      __syncthreads();  // the runs are visible; every thread has finished reading this stage
+      if (tid < D) {
+        float sum = 0.f;
+#pragma unroll
+        for (int gg = 0; gg < 8; gg++) sum += run_sums[gg][tid];
+        span_sums[((size_t)bh * nblk + blk) * D + tid] = sum;
+      }
+      continue;
+    }
     float x[NCHUNK][8];
     float amax = 0.f;
 #pragma unroll
@@ -378,19 +394,12 @@ cudaError_t launch_prologue_t(const PrologueArgs& a, cudaStream_t stream, int* l
   const int nblk = (a.S + 127) / 128;
   const int bhq = a.B * a.Hq, bhk = a.B * a.Hkv;
   *launches = 0;
+  const bool two_part = a.smooth && a.block != 1 && nblk > MEAN_SLOTS;
   if (a.smooth) {
-    // one round of MEAN_SLOTS spans, or pairs enough to keep the memory busy (from about 32 on): one CTA per pair does it
-    // all.  Else the two launches, with the INT8 / FP8 copy of Q,
-    // which the quantiser writes only after them, as scratch (S * D bytes per head against 4 * D per span of 128)
-    if (nblk <= MEAN_SLOTS || bhk > 32) {
+    if (!two_part) {
       k_mean_kernel<DTYPE, D><<<bhk, MEAN_SLOTS * D, 0, stream>>>(a.k, a.k_mean, a.S);
-    } else {
-      float* span_sums = (float*)a.q8;
-      k_span_kernel<DTYPE, D><<<dim3(nblk, bhk, 1), D, 0, stream>>>(a.k, span_sums, a.S);
-      k_mean_of_spans_kernel<D><<<bhk, D, 0, stream>>>(span_sums, a.k_mean, a.S, nblk);
       (*launches)++;
     }
-    (*launches)++;
   } else {
     cudaError_t e = cudaMemsetAsync(a.k_mean, 0, sizeof(float) * (size_t)bhk * D, stream);
     if (e != cudaSuccess) return e;
@@ -419,11 +428,20 @@ cudaError_t launch_prologue_t(const PrologueArgs& a, cudaStream_t stream, int* l
       if (e != cudaSuccess) return e;
       configured[dev] = true;
     }
-    const int items = (bhq + bhk) * nblk;
-    int grid = (dev < 64 ? sm_count[dev] : 148) * P::CTAS_PER_SM;
-    if (grid > items) grid = items;
-    kern<<<grid, 256, P::SMEM_BYTES, stream>>>(a.q, a.k, a.k_mean, a.q8, a.k8, a.q_scale, a.k_scale, a.S, bhq, bhk,
-                                               a.smooth, a.fp8, a.status, a.sticky);
+    const int resident = (dev < 64 ? sm_count[dev] : 148) * P::CTAS_PER_SM;
+    auto launch = [&](int part, int items) {
+      kern<<<items < resident ? items : resident, 256, P::SMEM_BYTES, stream>>>(
+          a.q, a.k, a.k_mean, a.q8, a.k8, a.q_scale, a.k_scale, a.S, bhq, bhk, a.smooth, a.fp8, part, (float*)a.k8, a.status,
+          a.sticky);
+    };
+    if (two_part) {  // the span sums lie in the place of K's 8-bit copy, which only the last launch writes
+      launch(PART_Q_AND_SUMS, (bhq + bhk) * nblk);
+      k_mean_of_spans_kernel<D><<<bhk, D, 0, stream>>>((const float*)a.k8, a.k_mean, a.S, nblk);
+      launch(PART_K, bhk * nblk);
+      (*launches) += 2;
+    } else {
+      launch(PART_ALL, (bhq + bhk) * nblk);
+    }
   }
   (*launches)++;
   return cudaGetLastError();
