@@ -129,8 +129,14 @@ __global__ void __launch_bounds__(D) k_mean_of_spans_kernel(const float* __restr
                                                             int S, int nspan) {
   const float* at = span_sums + (size_t)blockIdx.x * nspan * D + threadIdx.x;
   float total = 0.f;
-#pragma unroll 16
-  for (int sp = 0; sp < nspan; sp++) total += at[(size_t)sp * D];
+  for (int sp = 0; sp < nspan; sp += 16) {  // 16 loads in flight at a time, the last batch included
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = sp + i < nspan ? at[(size_t)(sp + i) * D] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (sp + i < nspan) total += v[i];
+  }
   k_mean[(size_t)blockIdx.x * D + threadIdx.x] = total * (1.0f / (float)S);
 }
 
@@ -173,8 +179,8 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const void* __restri
 // shared-memory ring with a bulk copy while the CTA reduces and stores block i, so that each SM keeps
 // tens of KB of reads in flight the whole time instead of one load-reduce-store round per CTA.
 // Needs 16-byte aligned Q and K.
-// With smoothing, K can only be quantised when its mean is known, but Q can be before: sequences of more than
-// MEAN_SLOTS spans take two launches of this kernel, Q blocks quantised and K blocks summed (PART_Q_AND_SUMS), and after
+// With smoothing, K can only be quantised when its mean is known, but Q can be before: sequences of 16
+// spans and more take two launches of this kernel, Q blocks quantised and K blocks summed (PART_Q_AND_SUMS), and after
 // k_mean_of_spans_kernel the K blocks quantised (PART_K).  The sum pass over K then streams beside Q's instead of
 // in a launch of its own.  Measured, mean and quantisation: 16 K heads of S=3001 with 64 of Q 48
 // us (cluster mean) -> 31, B=4 H=32 S=8192 214 -> 208.
@@ -394,7 +400,9 @@ cudaError_t launch_prologue_t(const PrologueArgs& a, cudaStream_t stream, int* l
   const int nblk = (a.S + 127) / 128;
   const int bhq = a.B * a.Hq, bhk = a.B * a.Hkv;
   *launches = 0;
-  const bool two_part = a.smooth && a.block != 1 && nblk > MEAN_SLOTS;
+  // Below 16 spans the two more launches cost more than the mean's rounds of MEAN_SLOTS spans do (B=2, 64 + 16 heads of
+  // S=1500: 20.6 us against 26.7; S=2000 27.7 against 26.7; S=5000 61 against 51).
+  const bool two_part = a.smooth && a.block != 1 && nblk >= 4 * MEAN_SLOTS;
   if (a.smooth) {
     if (!two_part) {
       k_mean_kernel<DTYPE, D><<<bhk, MEAN_SLOTS * D, 0, stream>>>(a.k, a.k_mean, a.S);
