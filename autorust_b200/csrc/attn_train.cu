@@ -110,13 +110,14 @@ __device__ __forceinline__ void p_and_ds(float s, float t, float scale, const fl
   ds = p * (t - delta);
 }
 
-// dQ: one CTA per (64 queries, batch x head); walks the keys 64 at a time.
-template <int D>
+// dQ: one CTA per (64 queries, batch x head); walks the keys 64 at a time.  (GROUPED: cta_order.cuh; known at compile time,
+// as the plain form spills with the choice in it, 2 % at D = 128.)
+template <int D, bool GROUPED>
 __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__ Q, const float* __restrict__ K,
                                                        const float* __restrict__ V, const float* __restrict__ dO,
                                                        const float* __restrict__ LSE, const float* __restrict__ delta,
                                                        const float* __restrict__ M, float* __restrict__ dQ, int N, int Hq,
-                                                       int Hkv, int grouped, int causal) {
+                                                       int Hkv, int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
   float* sQ = smem_t;
@@ -127,9 +128,9 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int bh = cta_head(grouped);
-  int tile = cta_tile(grouped);
-  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
+  const int bh = cta_head(GROUPED);
+  int tile = cta_tile(GROUPED);
+  if (causal) tile = cta_tiles(GROUPED) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * BT;
@@ -201,13 +202,12 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
 
 // dK, dV: one CTA per (64 keys, batch x kv head); walks the query heads of the group and their query tiles in a
 // fixed order, so the sums have one writer and one order.
-template <int D>
+template <int D, bool GROUPED>
 __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict__ Q, const float* __restrict__ K,
                                                         const float* __restrict__ V, const float* __restrict__ dO,
                                                         const float* __restrict__ LSE, const float* __restrict__ delta,
                                                         const float* __restrict__ M, float* __restrict__ dK,
-                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int grouped,
-                                                        int causal) {
+                                                        float* __restrict__ dV, int N, int Hq, int Hkv, int causal) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(16) float smem_t[];
   float* sK = smem_t;
@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int kvbh = cta_head(grouped);
-  const int tile = cta_tile(grouped);  // (under a causal mask the first key tile sees the most queries)
+  const int kvbh = cta_head(GROUPED);
+  const int tile = cta_tile(GROUPED);  // (under a causal mask the first key tile sees the most queries)
   const int b = kvbh / Hkv, hk = kvbh - b * Hkv;
   const int group = Hq / Hkv;
   const int k0 = tile * BT;
@@ -588,35 +588,39 @@ cudaError_t configure() {
   return e;
 }
 
-// The 128-row tiles take one CTA per SM, the 64-row ones work at about 0.6 of their rate: the form that ends first.
-bool worth_it(int S, int heads) {
+// The 128-row tiles do their rows about 5 % faster than the 64-row ones, of which an SM holds two: the form whose
+// rounds come to fewer rows per SM (B=6 Hq=4 S=848: dQ 2 x 128 against 3 x 64, a step 7 % slower in the wide form).
+// Under a causal mask they want two rounds at least: one round ends with its heaviest tile.
+bool worth_it(int S, int heads, int causal) {
   const long long w = (long long)((S + 127) / 128) * heads, n = (long long)((S + 63) / 64) * heads;
-  return ((w + 147) / 148) * 128 * 6 <= ((n + 147) / 148) * 64 * 10;
+  if (causal && w < 2 * 148) return false;
+  return ((w + 147) / 148) * 128 * 20 <= ((n + 147) / 148) * 64 * 21;
 }
 }  // namespace wide
 
 template <int D>
 cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches) {
   using C = BwdCfg<D>;
-  auto dq_kern = train_dq_kernel<D>;
-  auto dkv_kern = train_dkv_kernel<D>;
-  static bool configured[64] = {};
+  auto dq_kern = a.causal ? train_dq_kernel<D, true> : train_dq_kernel<D, false>;
+  auto dkv_kern = a.causal ? train_dkv_kernel<D, true> : train_dkv_kernel<D, false>;
+  static bool configured[2][64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 64 && !configured[dev]) {
+  const int form = a.causal ? 1 : 0;
+  if (dev < 64 && !configured[form][dev]) {
     e = cudaFuncSetAttribute(dq_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DQ_SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(dkv_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DKV_SMEM);
     if (e != cudaSuccess) return e;
-    configured[dev] = true;
+    configured[form][dev] = true;
   }
   *launches = 0;
   const long long rows = (long long)a.B * a.Hq * a.S;
   train_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(a.o, a.d_o, a.delta, rows, D);
   (*launches)++;
   const int tiles = (a.S + BT - 1) / BT;
-  const bool wide_dq = D == 64 && wide::worth_it(a.S, a.B * a.Hq), wide_dkv = D == 64 && wide::worth_it(a.S, a.B * a.Hkv);
+  const bool wide_dq = D == 64 && wide::worth_it(a.S, a.B * a.Hq, a.causal), wide_dkv = D == 64 && wide::worth_it(a.S, a.B * a.Hkv, a.causal);
   if (wide_dq || wide_dkv) {
     e = wide::configure();
     if (e != cudaSuccess) return e;
@@ -624,21 +628,27 @@ cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches
   const int wide_tiles = (a.S + wide::OWN - 1) / wide::OWN, group = a.Hq / a.Hkv;
   // f32 bytes that stream past a tile: the shared K and V, or Q and dO of the group's heads
   const size_t dq_bytes = (size_t)a.S * D * 8 / (size_t)group, dkv_bytes = (size_t)a.S * D * 8 * (size_t)group;
-  const CtaGrid gq = cta_grid(dq_bytes, a.B * a.Hq, wide_dq ? wide_tiles : tiles);
-  const CtaGrid gk = cta_grid(dkv_bytes, a.B * a.Hkv, wide_dkv ? wide_tiles : tiles);
+  // (the 64-row kernels are grouped exactly under a causal mask: a grid of one head per group is a plain one)
+  auto grid_of = [&](bool is_wide, size_t bytes, int heads) {
+    if (is_wide) return cta_grid(bytes, heads, wide_tiles);
+    if (!a.causal) return CtaGrid{dim3(tiles, heads, 1), 0};
+    const CtaGrid g = cta_grid(bytes, heads, tiles);
+    return g.grouped ? g : CtaGrid{dim3(1, tiles, heads), 1};
+  };
+  const CtaGrid gq = grid_of(wide_dq, dq_bytes, a.B * a.Hq), gk = grid_of(wide_dkv, dkv_bytes, a.B * a.Hkv);
   if (wide_dq)
     wide::train_dq_wide_kernel<<<gq.grid, 256, wide::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
                                                                        a.Hq, a.Hkv, gq.grouped, a.causal);
   else
     dq_kern<<<gq.grid, 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv,
-                                                  gq.grouped, a.causal);
+                                                  a.causal);
   (*launches)++;
   if (wide_dkv)
     wide::train_dkv_wide_kernel<<<gk.grid, 256, wide::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
                                                                          a.dv, a.S, a.Hq, a.Hkv, gk.grouped, a.causal);
   else
     dkv_kern<<<gk.grid, 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv,
-                                                   gk.grouped, a.causal);
+                                                   a.causal);
   (*launches)++;
   return cudaGetLastError();
 }

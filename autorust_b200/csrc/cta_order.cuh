@@ -31,7 +31,7 @@ inline CtaGrid cta_grid(size_t bytes_per_head, int heads, int tiles, int split =
   int group = 1;
   if ((long long)tiles * heads <= 8 * 148 && tiles <= 65535) {
     const size_t fit = HEAD_GROUP_BYTES / (bytes_per_head ? bytes_per_head : 1);
-    for (int d = 2; d <= heads && (size_t)d <= fit; d++)
+    for (int d = fit < (size_t)heads ? (int)fit : heads; d > 1 && group == 1; d--)  // the largest divisor that fits
       if (heads % d == 0) group = d;
   }
   if (group == 1) return {dim3((unsigned)(tiles * split), (unsigned)heads, 1), 0};

@@ -94,7 +94,8 @@ def test_exact_tiles(ops, oracle_lib, b, hq, hkv, n, d, causal):
 
 
 @pytest.mark.parametrize("tc", [False, True])
-@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321),
+@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321), (1, 7, 1, 70),
+                                        (2, 8, 1, 200),
                                         (5, 30, 30, 130)])
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
