@@ -13,6 +13,8 @@ MODE_EXACT_F32, MODE_TF32, MODE_BF16, MODE_SAGE_INT8, MODE_SAGE_FP8, MODE_SAGE_I
 DTYPE_F32, DTYPE_BF16 = 0, 1
 REPLICAS_MULTICAST = -1  # n_replicas: replicas[0] is one address of an NVLink multicast object
 
+PLAN_TRAIN_BACKWARD = 0  # paths of ar_attn_plan
+
 AR_OK = 0
 AR_ERR_UNSUPPORTED = -1
 AR_ERR_NULL = -2
@@ -49,6 +51,7 @@ SYMBOLS = (
     "ar_sage_forward_static",
     "ar_add_layernorm",
     "ar_attn_last_status",
+    "ar_attn_plan",
     "ar_attn_selections",
     "ar_attn_launch_count",
     "ar_attn_strerror",
@@ -119,6 +122,8 @@ def load() -> ctypes.CDLL:
     L.ar_sage_forward_static.restype = ci
     L.ar_attn_last_status.argtypes = [p, p]
     L.ar_attn_last_status.restype = ci
+    L.ar_attn_plan.argtypes = [ci, i64, i64, i64, i64, i64, ci, ctypes.POINTER(ctypes.c_int32)]
+    L.ar_attn_plan.restype = ci
     L.ar_attn_selections.argtypes = [ci]
     L.ar_attn_selections.restype = ctypes.c_uint64
     L.ar_attn_launch_count.restype = ctypes.c_uint64
@@ -126,6 +131,13 @@ def load() -> ctypes.CDLL:
     L.ar_attn_strerror.restype = ctypes.c_char_p
     _lib = L
     return L
+
+
+def plan(path: int, B: int, Hq: int, Hkv: int, S: int, D: int, causal: bool) -> list[int]:
+    """Which form of its kernels a call of these sizes takes (ar_attn_plan); needs no GPU."""
+    out = (ctypes.c_int32 * 8)()
+    check(load().ar_attn_plan(path, B, Hq, Hkv, S, D, int(causal), out), "ar_attn_plan")
+    return list(out)
 
 
 def strerror(rc: int) -> str:

@@ -701,6 +701,28 @@ int ar_attn_last_status(void* workspace, void* cu_stream) {
 }
 
 
+int ar_attn_plan(int path, int64_t B, int64_t Hq, int64_t Hkv, int64_t S, int64_t D, int causal, int32_t* plan) {
+  if (!plan) return AR_ERR_NULL;
+  int rc = check_shape(B, Hq, Hkv, S, D);
+  if (rc != AR_OK) return rc;
+  if ((D != 64 && D != 128) || B * Hq > 65535 || S > (1 << 24)) return AR_ERR_UNSUPPORTED;
+  for (int i = 0; i < 8; i++) plan[i] = 0;
+  auto put_grid = [&](int at, const dim3& g) {
+    plan[at] = (int32_t)g.x;
+    plan[at + 1] = (int32_t)g.y;
+    plan[at + 2] = (int32_t)g.z;
+  };
+  if (path == AR_PLAN_TRAIN_BACKWARD) {
+    const ar::TrainExactPlan p = ar::train_exact_plan((int)B, (int)Hq, (int)Hkv, (int)S, (int)D, causal != 0);
+    plan[0] = p.dq_rows;
+    plan[1] = p.dkv_rows;
+    put_grid(2, p.dq.grid);
+    put_grid(5, p.dkv.grid);
+    return AR_OK;
+  }
+  return AR_ERR_UNSUPPORTED;
+}
+
 uint64_t ar_attn_selections(int mode) { return (mode >= 0 && mode < 6) ? g_selected[mode].load() : 0; }
 uint64_t ar_attn_launch_count(void) { return g_launches.load(); }
 

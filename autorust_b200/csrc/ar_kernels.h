@@ -4,6 +4,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "cta_order.cuh"
+
 namespace ar {
 
 // Tensor-core forward (attn_fwd_tc.cu): bf16 or Sage INT8 QK^T, bf16 PV.
@@ -104,6 +106,12 @@ struct TrainBwdArgs {
   int B, Hq, Hkv, S, D;
   int causal;
 };
+// The forms that such a call takes: rows of a CTA's tile (64 or 128) and grids.
+struct TrainExactPlan {
+  int dq_rows, dkv_rows;
+  CtaGrid dq, dkv;
+};
+TrainExactPlan train_exact_plan(int B, int Hq, int Hkv, int S, int D, int causal);
 // Launches prep, dQ and dK/dV; *launches returns the number of kernels.
 cudaError_t launch_attn_train_backward(const TrainBwdArgs& a, cudaStream_t stream, int* launches);
 // delta[row] = O_row . dO_row over `rows` rows of D floats, and the bf16 copy of dO.

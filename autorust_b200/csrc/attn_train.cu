@@ -601,59 +601,72 @@ bool worth_it(int S, int heads, int causal) {
 template <int D>
 cudaError_t launch_bwd(const TrainBwdArgs& a, cudaStream_t stream, int* launches) {
   using C = BwdCfg<D>;
-  auto dq_kern = a.causal ? train_dq_kernel<D, true> : train_dq_kernel<D, false>;
-  auto dkv_kern = a.causal ? train_dkv_kernel<D, true> : train_dkv_kernel<D, false>;
-  static bool configured[2][64] = {};
+  const TrainExactPlan p = train_exact_plan(a.B, a.Hq, a.Hkv, a.S, a.D, a.causal);
+  const bool wide_dq = p.dq_rows == wide::OWN, wide_dkv = p.dkv_rows == wide::OWN;
+  auto dq_kern = p.dq.grouped ? train_dq_kernel<D, true> : train_dq_kernel<D, false>;
+  auto dkv_kern = p.dkv.grouped ? train_dkv_kernel<D, true> : train_dkv_kernel<D, false>;
+  static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const int form = a.causal ? 1 : 0;
-  if (dev < 64 && !configured[form][dev]) {
-    e = cudaFuncSetAttribute(dq_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DQ_SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(dkv_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DKV_SMEM);
-    if (e != cudaSuccess) return e;
-    configured[form][dev] = true;
+  if (dev < 64 && !configured[dev]) {
+    for (auto k : {train_dq_kernel<D, false>, train_dq_kernel<D, true>}) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DQ_SMEM);
+      if (e != cudaSuccess) return e;
+    }
+    for (auto k : {train_dkv_kernel<D, false>, train_dkv_kernel<D, true>}) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::DKV_SMEM);
+      if (e != cudaSuccess) return e;
+    }
+    configured[dev] = true;
   }
   *launches = 0;
   const long long rows = (long long)a.B * a.Hq * a.S;
   train_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(a.o, a.d_o, a.delta, rows, D);
   (*launches)++;
-  const int tiles = (a.S + BT - 1) / BT;
-  const bool wide_dq = D == 64 && wide::worth_it(a.S, a.B * a.Hq, a.causal), wide_dkv = D == 64 && wide::worth_it(a.S, a.B * a.Hkv, a.causal);
   if (wide_dq || wide_dkv) {
     e = wide::configure();
     if (e != cudaSuccess) return e;
   }
-  const int wide_tiles = (a.S + wide::OWN - 1) / wide::OWN, group = a.Hq / a.Hkv;
-  // f32 bytes that stream past a tile: the shared K and V, or Q and dO of the group's heads
-  const size_t dq_bytes = (size_t)a.S * D * 8 / (size_t)group, dkv_bytes = (size_t)a.S * D * 8 * (size_t)group;
-  // (the 64-row kernels are grouped exactly under a causal mask: a grid of one head per group is a plain one)
-  auto grid_of = [&](bool is_wide, size_t bytes, int heads) {
-    if (is_wide) return cta_grid(bytes, heads, wide_tiles);
-    if (!a.causal) return CtaGrid{dim3(tiles, heads, 1), 0};
-    const CtaGrid g = cta_grid(bytes, heads, tiles);
-    return g.grouped ? g : CtaGrid{dim3(1, tiles, heads), 1};
-  };
-  const CtaGrid gq = grid_of(wide_dq, dq_bytes, a.B * a.Hq), gk = grid_of(wide_dkv, dkv_bytes, a.B * a.Hkv);
   if (wide_dq)
-    wide::train_dq_wide_kernel<<<gq.grid, 256, wide::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S,
-                                                                       a.Hq, a.Hkv, gq.grouped, a.causal);
+    wide::train_dq_wide_kernel<<<p.dq.grid, 256, wide::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq,
+                                                                         a.S, a.Hq, a.Hkv, p.dq.grouped, a.causal);
   else
-    dq_kern<<<gq.grid, 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv,
+    dq_kern<<<p.dq.grid, 256, C::DQ_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dq, a.S, a.Hq, a.Hkv,
                                                   a.causal);
   (*launches)++;
   if (wide_dkv)
-    wide::train_dkv_wide_kernel<<<gk.grid, 256, wide::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
-                                                                         a.dv, a.S, a.Hq, a.Hkv, gk.grouped, a.causal);
+    wide::train_dkv_wide_kernel<<<p.dkv.grid, 256, wide::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk,
+                                                                            a.dv, a.S, a.Hq, a.Hkv, p.dkv.grouped, a.causal);
   else
-    dkv_kern<<<gk.grid, 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv,
+    dkv_kern<<<p.dkv.grid, 256, C::DKV_SMEM, stream>>>(a.q, a.k, a.v, a.d_o, a.lse, a.delta, a.mask, a.dk, a.dv, a.S, a.Hq, a.Hkv,
                                                    a.causal);
   (*launches)++;
   return cudaGetLastError();
 }
 
 }  // namespace
+
+TrainExactPlan train_exact_plan(int B, int Hq, int Hkv, int S, int D, int causal) {
+  const int group = Hq / Hkv;
+  TrainExactPlan p;
+  p.dq_rows = D == 64 && wide::worth_it(S, B * Hq, causal) ? wide::OWN : BT;
+  p.dkv_rows = D == 64 && wide::worth_it(S, B * Hkv, causal) ? wide::OWN : BT;
+  // The 64-row kernels take a grouped grid under a causal mask, of one head per group where cta_grid gives a plain one;
+  // that grid has the tiles in y, and a sequence with more than y holds stays plain.
+  auto grid_of = [&](int rows, size_t bytes, int heads) {
+    const int tiles = (S + rows - 1) / rows;
+    const CtaGrid plain{dim3((unsigned)tiles, (unsigned)heads, 1), 0};
+    if (rows == BT && !causal) return plain;
+    const CtaGrid g = cta_grid(bytes, heads, tiles);
+    if (rows != BT || g.grouped) return g;
+    return tiles <= 65535 ? CtaGrid{dim3(1, (unsigned)tiles, (unsigned)heads), 1} : plain;
+  };
+  // f32 bytes that stream past a tile: the shared K and V, or Q and dO of the group's heads
+  p.dq = grid_of(p.dq_rows, (size_t)S * D * 8 / (size_t)group, B * Hq);
+  p.dkv = grid_of(p.dkv_rows, (size_t)S * D * 8 * (size_t)group, B * Hkv);
+  return p;
+}
 
 cudaError_t launch_attn_train_backward(const TrainBwdArgs& a, cudaStream_t stream, int* launches) {
   if (a.D == 64) return launch_bwd<64>(a, stream, launches);
