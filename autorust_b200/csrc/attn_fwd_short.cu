@@ -2,8 +2,12 @@
 // tokens: the semantics of attn_fwd_tc.cu's bf16 mode with the whole key range in one pass.
 //
 // All scores of a query tile fit the TMEM columns of half an SM: S = Q K^T is one MMA chain of N = S columns (rounded up
-// to 16), the softmax sees a row's true maximum before its first exponential, and P V is one chain of K = S.  There is
-// no online rescaling, no key loop and no padding to 128 keys.
+// to 16), the softmax has seen all of a row's scores before its first exponential, and P V is one chain of K = S.  There
+// is no rescaling of O, no key loop and no padding to 128 keys.  The arithmetic is that of the two 128-key steps of
+// attn_fwd_tc.cu, so that a row's bits do not depend on which of the kernels served it: the maximum of the first 128 keys
+// is the reference unless a later score exceeds it by RESCALE_THRESHOLD (only then do the roundings of P differ), a
+// step's row sum is kept in two accumulators, and only a step of 128 visible keys has a quarter of its exponentials on
+// the FMA pipe (1.1e-4; the row sum and the log-sum-exp of shorter sequences keep the accuracy of the MUFU unit).
 //
 //   persistent CTA, two per SM, 192 threads; its items are (batch x head, tile of 128 queries)
 //     warps 0-3  softmax and epilogue (thread r owns row r = TMEM lane r)
@@ -27,6 +31,7 @@ using namespace arptx;
 constexpr int BM = 128, D = 64, KEYS = 256;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float NEG = -1e30f * LOG2E;  // the reference's finite sentinel in the log2 domain
+constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units, as in attn_fwd_tc.cu
 constexpr int NUM_THREADS = 192;
 constexpr int W_PROD = 4, W_MMA = 5;
 constexpr int Q_BYTES = BM * D * 2, KV_BYTES = KEYS * D * 2;
@@ -35,10 +40,11 @@ constexpr int NUM_BARS = 8;
 constexpr int SMEM_BYTES = Q_BYTES + 2 * KV_BYTES + STAGE_BYTES + NUM_BARS * 8 + 16 + 1024;
 static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
 
-// Exponentials of 32 columns of a row: P (bf16 pairs) into pk, the unrounded values added to sum.  POLY: a quarter on
-// the FMA pipe (columns that may be -inf take the MUFU path, whose 2^-inf is exactly 0).
+// Exponentials of 32 columns of a row: P (bf16 pairs) into pk, the unrounded values added to the two sums.  POLY: a
+// quarter on the FMA pipe (columns that may be -inf take the MUFU path, whose 2^-inf is exactly 0).
 template <bool POLY>
-__device__ __forceinline__ void exp_chunk(const uint32_t* sv, uint64_t c2, uint64_t negm2, uint32_t (&pk)[16], uint64_t& sum) {
+__device__ __forceinline__ void exp_chunk(const uint32_t* sv, uint64_t c2, uint64_t negm2, uint32_t (&pk)[16],
+                                          uint64_t (&sum)[2]) {
 #pragma unroll
   for (int i = 0; i < 16; i++) {
     const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), c2, negm2);
@@ -47,7 +53,7 @@ __device__ __forceinline__ void exp_chunk(const uint32_t* sv, uint64_t c2, uint6
       exp2_poly_x2(x2, p0, p1);
     else
       exp2_mufu_x2(x2, p0, p1);
-    sum = add_f32x2(sum, pack_f32x2(p0, p1));
+    sum[i & 1] = add_f32x2(sum[i & 1], pack_f32x2(p0, p1));
     pk[i] = pack_bf16x2(p0, p1);
   }
 }
@@ -216,17 +222,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       const bool rows_in = it.q0 + warp * 32 < N;       // the warp has rows inside the sequence
       const int visible = causal ? min(N, row + 1) : N;  // keys this row sees
       const int chunks = (it.keys + 31) >> 5;            // columns past the last key may hold anything: excluded below
-      // (uniform) no lane of the CTA excludes a column before this chunk
-      const int whole = causal ? it.q0 >> 5 : N >> 5;
+      // (uniform) no lane of the CTA excludes a column before chunk `whole`; the 128-key steps before chunk `poly` are
+      // whole ones
+      const int whole = causal ? it.q0 >> 5 : N >> 5, poly = whole & ~3;
       float m = NEG, l = 0.f;
       do {  // (left early by a warp whose wait ran out or whose rows lie past the sequence end)
       ok = __all_sync(0xffffffffu, mbar_wait(s_full, n & 1, wctx, 0x66));
       if (!ok) break;
       tc_fence_after();
       if (rows_in) {
-        // the row's maximum
+        // the row's maximum over the first 128 keys, and over the others
         uint32_t sa[32], sb[32];
-        float mx = __uint_as_float(0xff800000u);
+        float mx = __uint_as_float(0xff800000u), first = mx;
 #pragma unroll 1
         for (int q = 0; q < chunks; q += 2) {
           tmem_ld32(tS + q * 32, sa);
@@ -238,15 +245,26 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
             exclude(sb, visible - q * 32 - 32);
           }
           mx = max_chunk(sb, max_chunk(sa, mx));
+          if (q < 4) {
+            first = mx;
+            if (q == 2) mx = __uint_as_float(0xff800000u);
+          }
         }
-        m = fmaxf(m, mx * c);
+        m = fmaxf(m, first * c);
+        if (chunks > 4 && mx * c > m + RESCALE_THRESHOLD) m = mx * c;
         const uint64_t negm2 = pack_f32x2(-m, -m);
-        uint64_t sum = pack_f32x2(0.f, 0.f);
+        uint64_t sum[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
+        auto end_step = [&]() {
+          float lo, hi;
+          unpack_f32x2(add_f32x2(sum[0], sum[1]), lo, hi);
+          l += lo + hi;
+          sum[0] = sum[1] = pack_f32x2(0.f, 0.f);
+        };
         // P of chunk q goes to columns [16 q, 16 q + 16): the scores there have been read.  The next chunk's scores are
         // on their way during this one's exponentials.
         auto chunk = [&](uint32_t(&sv)[32], int q) {
           uint32_t pk[16];
-          if (q < whole) {
+          if (q < poly) {
             exp_chunk<true>(sv, c2, negm2, pk, sum);
           } else {
             exclude(sv, visible - q * 32);
@@ -266,11 +284,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
             chunk(sb, q + 1);
             if (q + 2 < chunks) tmem_wait_ld32(sa);
           }
+          if (q == 2) end_step();
         }
         tmem_wait_st();
-        float lo, hi;
-        unpack_f32x2(sum, lo, hi);
-        l = lo + hi;
+        end_step();
       }
       tc_fence_before();
       mbar_arrive(p_full);

@@ -53,7 +53,39 @@ def test_bf16_short_sequences_many_items_per_cta(ops, oracle_lib):
     assert torch.equal(out[-1:], one)
 
 
-@pytest.mark.parametrize("mode,d", [("bf16", 64), ("bf16", 128), ("tf32", 64), ("sage", 128), ("sage_rows", 64)])
+@pytest.mark.parametrize("n", [1, 33, 100, 127, 128, 200, 256])
+@pytest.mark.parametrize("causal", [False, True])
+def test_short_log_sum_exp(ops, n, causal):
+    """The row sums behind the training forward's log-sum-exp against float64 on the same bf16 operands.  Without a step
+    of 128 visible keys every exponential is the MUFU unit's (2^-22) and the bound is that of f32 sums over values of a
+    few units, 5e-6; a whole step has a quarter of its exponentials within 1.1e-4."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(2, 4, n, 64, device="cuda", generator=g) for _ in range(3))
+    _, lse = ops.train_forward(q, k, v, causal=causal, tensor_cores=True)
+    s = q.bfloat16().double() @ k.bfloat16().double().transpose(-1, -2) / 8.0
+    if causal:
+        s.masked_fill_(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    err = (lse.double() - torch.logsumexp(s, -1)).abs()
+    whole = torch.arange(n, device="cuda") >= 128 if causal else torch.full((n,), n >= 128, device="cuda")
+    assert err[..., ~whole].max().item() <= 5e-6 if (~whole).any() else True
+    assert err[..., whole].max().item() <= 3.5e-5 if whole.any() else True
+
+
+@pytest.mark.parametrize("n", [40, 128, 129, 200, 256])
+def test_short_and_long_kernel_give_a_row_the_same_bits(ops, n):
+    """A causal row sees the same keys in a call of n tokens (the one-pass kernel) and in one of 300 (the key loop): the
+    same steps, references and sums."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(1, 3, 300, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    long = ops.attn_forward("bf16", q, k, v, None, True)
+    short = ops.attn_forward("bf16", *(t[:, :, :n].contiguous() for t in (q, k, v)), None, True)
+    assert torch.equal(short, long[:, :, :n])
+
+
+@pytest.mark.parametrize("mode,d", [("bf16", 64), ("bf16", 128), ("tf32", 64), ("sage_fp8", 64), ("sage_fp8", 128), ("sage", 128),
+                                    ("sage_rows", 64)])
 @pytest.mark.parametrize("n", [1, 31, 33, 100, 127, 129, 260, 389])
 @pytest.mark.parametrize("causal", [False, True])
 def test_mask_ring(ops, oracle_lib, mode, d, n, causal):
