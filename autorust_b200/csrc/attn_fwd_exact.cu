@@ -127,6 +127,9 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     }
     group_sync();  // the group is done with this K tile
     load_rows(sK, C::LDQ, kb, min(k0 + GROUPS * BK, N));  // (past the last tile: zeros, nothing is read)
+    // Excluded keys get the finite sentinel, which a row whose visible keys all carry -1e30 counts along.  Under a causal
+    // mask a row counts them up to the end of the 64 keys its diagonal lies in; a tile that reaches further gives them
+    // no weight, so that such a row has the same value whatever tile height its call takes.
     const bool bounds = k0 + BK > N || (causal && k0 + BK - 1 > q0);
 #pragma unroll
     for (int i = 0; i < RQ; i++) {
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
         const int key = k0 + tx + TX * jj;
         float x = s[i][jj] * scale;
         if (M != nullptr && row < N && key < N) x += M[(size_t)row * N + key];
-        if (bounds && (key >= N || (causal && key > row))) x = NEG;
+        if (bounds && (key >= N || (causal && key > row))) x = causal && k0 > row ? -INFINITY : NEG;
         s[i][jj] = x;
         mx = fmaxf(mx, x);
       }

@@ -140,6 +140,31 @@ def test_training_steps(ops, oracle_lib, tc, b, hq, hkv, n, d, causal):
     d_o = rng.standard_normal(q.shape, dtype=np.float32)
     mask = sawtooth_mask(n) if n == 129 else None
     want = dict(zip(("o", "lse", "dq", "dk", "dv"), oracle_lib.attn_train(q, k, v, d_o, mask, causal)))
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n", [40, 100, 200, 330])
+def test_exact_causal_rows_without_visible_keys(ops, n, d):
+    """Left padding under a causal mask: a row whose visible keys all carry -1e30 averages V over the keys up to the end of
+    the 64 its diagonal lies in (those past the sequence end count as zeros), in every batch and head and whatever
+    tile height B * H * S selects.  Other rows are the attention over their visible keys."""
+    import torch
+    pad = n - n // 3
+    mask = torch.zeros(n, n, device="cuda")
+    mask[:, :pad] = -1e30
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q1, k1, v1 = (torch.randn(1, 1, n, d, device="cuda", generator=g) for _ in range(3))
+    s = q1[0, 0].double() @ k1[0, 0].double().T / d ** 0.5 + mask.double()
+    s.masked_fill_(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.softmax(s, -1) @ v1[0, 0].double()
+    for row in range(pad):
+        end = (row // 64 + 1) * 64
+        want[row] = v1[0, 0, :end].double().sum(0) / end
+    for heads in (1, 6, 24, 60, 148, 400):
+        q, k, v = (t.expand(1, heads, n, d).contiguous() for t in (q1, k1, v1))
+        got = ops.attn_forward("exact", q, k, v, mask, True)
+        # the outputs are averages of N(0,1) values, below about 5: the exact mode's 1e-5 of the largest value
+        assert (got[0].double() - want).abs().max().item() <= 1e-5, heads
+
+
     tq, tk, tv, tdo = map(to_dev, (q, k, v, d_o))
     tm = None if mask is None else to_dev(mask)
     o, lse = ops.train_forward(tq, tk, tv, tm, causal, tensor_cores=tc)
