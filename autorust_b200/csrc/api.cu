@@ -88,13 +88,13 @@ uint32_t* status_ptr(void* workspace) {
 // The status word of a launch that no earlier kernel of the call clears.  The caller's word is cleared on the stream.
 // The library's word is not: the launch gets a ticket instead, which saves the stream a memset of its own in front of a
 // kernel of 20 microseconds.  A captured call would replay its ticket, so that one clears the word as well.
+std::atomic<uint32_t> g_next_ticket{0};
 bool prepare_status(ar::TcArgs& a, bool callers_word, cudaStream_t stream) {
   if (!callers_word) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return false;
     if (capture == cudaStreamCaptureStatusNone) {
-      static std::atomic<uint32_t> next{0};
-      a.ticket = (next.fetch_add(1) & 0x3fffffffu) + 1u;  // 1 .. 2^30: never 0, never the bit an OR-ed status carries
+      a.ticket = (g_next_ticket.fetch_add(1) & 0x3fffffffu) + 1u;  // 1 .. 2^30: never 0, never the bit an OR-ed status carries
       return true;
     }
   }
@@ -696,7 +696,8 @@ int ar_attn_last_status(void* workspace, void* cu_stream) {
   uint32_t host = 0;
   if (cudaStreamSynchronize((cudaStream_t)cu_stream) != cudaSuccess) return AR_ERR_CUDA;
   if (cudaMemcpy(&host, status, sizeof(host), cudaMemcpyDeviceToHost) != cudaSuccess) return AR_ERR_CUDA;
-  if (host != 0 && !workspace && cudaMemset(status, 0, sizeof(uint32_t)) != cudaSuccess) return AR_ERR_CUDA;
+  // (word 0 as well: the ticket that an expired launch left there must not meet a later launch with the same number)
+  if (host != 0 && !workspace && cudaMemset(library_words(), 0, 2 * sizeof(uint32_t)) != cudaSuccess) return AR_ERR_CUDA;
   return host == 0 ? AR_OK : AR_ERR_DEVICE_WAIT;
 }
 
@@ -741,5 +742,10 @@ const char* ar_attn_strerror(int status) {
     default: return "unknown status";
   }
 }
+
+#ifdef AR_WAIT_TEST
+// test builds only: the number the next launch without a workspace takes its ticket from
+void ar_test_next_ticket(uint32_t n) { g_next_ticket.store(n); }
+#endif
 
 }  // extern "C"

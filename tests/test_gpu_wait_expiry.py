@@ -40,6 +40,17 @@ CHILD = textwrap.dedent('''
     torch.cuda.synchronize()
     assert ops.last_status(None) == _abi.AR_ERR_DEVICE_WAIT, "the expiry was not reported"
     assert ops.last_status(None) == _abi.AR_OK, "reading the library's accumulator clears it"
+    # the expired launch's number has been cleared with the accumulator: a launch that carries it again is not lost
+    L.ar_test_next_ticket(77)
+    ops.attn_forward("bf16", q, k, v)
+    assert ops.last_status(None) == _abi.AR_ERR_DEVICE_WAIT
+    assert L.ar_test_skip_k_tile(-1) == 0
+    L.ar_test_next_ticket(77)
+    out.zero_()
+    ops.attn_forward("bf16", q, k, v, out=out)
+    assert ops.last_status(None) == _abi.AR_OK
+    assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
+    assert L.ar_test_skip_k_tile(1) == 0
     # the Sage path reports to its workspace's word and to the accumulator alike
     ws = torch.empty(ops.workspace_bytes("sage", q, k), dtype=torch.uint8, device="cuda")
     ops.attn_forward("sage", q, k, v, workspace=ws)
