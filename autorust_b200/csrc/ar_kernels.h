@@ -131,6 +131,12 @@ struct TrainBwdTcArgs {
   uint32_t* status;
   uint32_t* sticky;
 };
+// The forms that such a call takes.
+struct TrainTcPlan {
+  int small_dq, small_dkv;  // D = 64: the form with two CTAs per SM
+  int split;                // CTAs of a cluster that share a key tile's query heads (dK/dV)
+};
+TrainTcPlan train_tc_plan(int B, int Hq, int Hkv, int S, int D, int causal);
 // Launches dQ and dK/dV; *launches is incremented by the number of kernels.
 cudaError_t launch_attn_train_backward_tc(const TrainBwdTcArgs& a, cudaStream_t stream, int* launches);
 

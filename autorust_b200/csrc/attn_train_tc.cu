@@ -14,9 +14,9 @@
 //                 P^T, dS^T -> bf16 in TMEM
 //                 dV += P^T dO, dK += dS^T Q       (dO and Q consumed MN-major from the tiles S^T and dP^T read K-major)
 //
-// One CTA per SM.  A step's scores and dP take 128 TMEM columns, and the columns that the accumulators leave hold
-// STAGES = 3 steps (2 for dK/dV at D = 128), each with an element-wise warpgroup of its own (thread = TMEM lane).  The
-// MMA warp keeps STAGES steps of S and dP issued ahead, so that the tensor pipe works on later steps while the
+// A step's scores and dP take 128 TMEM columns, and the columns that the accumulators leave hold STAGES = 3 steps (2 for
+// dK/dV at D = 128), each with an element-wise warpgroup of its own (thread = TMEM lane); one CTA per SM.  SMALL (D = 64):
+// 256 columns, one step and one element-wise warpgroup, two CTAs per SM, for short walks in several rounds.  The MMA warp keeps STAGES steps of S and dP issued ahead, so that the tensor pipe works on later steps while the
 // warpgroups are on theirs:  ... dQ(n), S/dP(n + STAGES), dQ(n + 1), S/dP(n + 1 + STAGES) ...  MMAs of one thread
 // execute in issue order, which is what lets S(n + STAGES) overwrite the columns dQ(n) has read.
 // Floor of a step per SM at D = 64: S and dP 384 cycles of the tensor pipe (N = 64 with both operands from shared memory
@@ -37,6 +37,7 @@
 #include "ar_ptx.cuh"
 #include "cta_order.cuh"
 
+#include <cmath>
 #include <cooperative_groups.h>
 
 namespace ar {
@@ -47,52 +48,54 @@ constexpr int T = 128;  // rows a CTA owns: queries (dQ) or keys (dK/dV)
 constexpr int NH = 64;  // rows streamed per step: keys (dQ) or queries (dK/dV)
 constexpr float LOG2E = 1.4426950408889634f;
 
-template <int D, bool DKV>
+template <int D, bool DKV, bool SMALL>
 struct TcBwd {
   static constexpr int ROW_BYTES = D * 2;
   static constexpr int OWN_BYTES = T * ROW_BYTES;     // one tile of the CTA's own rows (two: Q and dO, or K and V)
   static constexpr int STREAM_BYTES = NH * ROW_BYTES; // one streamed tile (two per step)
   static constexpr int ACC_COLS = DKV ? 2 * D : D;    // TMEM columns of the gradient accumulators
-  static constexpr int STAGES = (512 - ACC_COLS) / (2 * NH) < 3 ? (512 - ACC_COLS) / (2 * NH) : 3;
-  static constexpr int SLOTS = D == 64 ? 6 : 4;       // streamed steps in shared memory; STAGES + 1 keep the MMAs fed
+  static constexpr int TMEM_COLS = SMALL ? 256 : 512;
+  static constexpr int MIN_CTAS = SMALL ? 2 : 1;
+  static constexpr int STAGES = (TMEM_COLS - ACC_COLS) / (2 * NH) < 3 ? (TMEM_COLS - ACC_COLS) / (2 * NH) : 3;
+  static constexpr int SLOTS = D == 64 && !SMALL ? 6 : 4;  // streamed steps in shared memory; STAGES + 1 keep the MMAs fed
   static_assert(SLOTS > STAGES, "a slot beyond the steps in flight");
   static constexpr int ROWVALS_BYTES = STAGES * 2 * 2 * NH * 4;  // dK/dV: LSE and D_i of a step's queries, double-buffered
   static constexpr int NUM_BARS = 2 + 2 * SLOTS + 2 * STAGES;
   static constexpr int SMEM_BYTES = 2 * OWN_BYTES + SLOTS * 2 * STREAM_BYTES + ROWVALS_BYTES + NUM_BARS * 8 + 16 + 1024;
-  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+  static_assert(MIN_CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory budget");
   static_assert(ACC_COLS * T * 4 <= 2 * OWN_BYTES + SLOTS * 2 * STREAM_BYTES, "accumulators pass through the tiles");
   static constexpr int KSTEPS_D = D / 16;             // k-steps of a product over d
   static constexpr int KSTEPS_NH = NH / 16;           // k-steps of a product over one step's rows
   static constexpr uint32_t IDESC_SS = make_idesc(1, 1, 1, 0, 0, T, NH);  // bf16 x bf16 -> f32, both K-major, N = NH
   static constexpr uint32_t IDESC_TS = make_idesc(1, 1, 1, 0, 1, T, D);   // A from TMEM, B MN-major, N = D
-  static constexpr int W_PROD = 4 * STAGES, W_MMA = W_PROD + 1;           // two more warps complete the last warpgroup
-  static constexpr int NUM_THREADS = 128 * STAGES + 128;
+  static constexpr int W_PROD = 4 * STAGES, W_MMA = W_PROD + 1;
+  static constexpr int NUM_THREADS = 128 * STAGES + (SMALL ? 64 : 128);   // (two more warps complete the last warpgroup)
   // registers per thread: launched with LAUNCH_REGS, then (two stages) moved from the last warpgroup to the others
+  static constexpr bool MOVE_REGS = STAGES == 2;
   static constexpr int LAUNCH_REGS = STAGES == 3 ? 128 : 168;
-  static constexpr int EW_REGS = STAGES == 3 ? 128 : 192;
-  static constexpr int SERVICE_REGS = STAGES == 3 ? 128 : 120;
-  static_assert(128 * STAGES * EW_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
-  static_assert(LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
+  static constexpr int EW_REGS = 192, SERVICE_REGS = 120;
+  static_assert(!MOVE_REGS || 128 * STAGES * EW_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
+  static_assert(MIN_CTAS * LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
 };
 
 // D[tmem, 128 x NH] = A[128 x D] B[NH x D]^T, both tiles K-major (rows of 128-byte boxes, 128-byte swizzle)
-template <int D, bool DKV>
+template <int D, bool DKV, bool SMALL>
 __device__ __forceinline__ void mma_abt(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi) {
   if (!elect_one()) return;
 #pragma unroll
-  for (int s = 0; s < TcBwd<D, DKV>::KSTEPS_D; s++) {
+  for (int s = 0; s < TcBwd<D, DKV, SMALL>::KSTEPS_D; s++) {
     const uint32_t a = a_lo + (((s >> 2) * (T * 128) + (s & 3) * 32) >> 4);
     const uint32_t b = b_lo + (((s >> 2) * (NH * 128) + (s & 3) * 32) >> 4);
-    mma_ss_lohi<KIND_F16>(d_tmem, a, hi, b, hi, TcBwd<D, DKV>::IDESC_SS, s > 0);
+    mma_ss_lohi<KIND_F16>(d_tmem, a, hi, b, hi, TcBwd<D, DKV, SMALL>::IDESC_SS, s > 0);
   }
 }
 // D[tmem, 128 x D] (+)= A[tmem, 128 x NH bf16] B[NH x D], B consumed MN-major from a row-major tile
-template <int D, bool DKV>
+template <int D, bool DKV, bool SMALL>
 __device__ __forceinline__ void mma_tb(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, bool acc) {
   if (!elect_one()) return;
 #pragma unroll
-  for (int s = 0; s < TcBwd<D, DKV>::KSTEPS_NH; s++)
-    mma_ts_lohi<KIND_F16>(d_tmem, a_tmem + s * 8, b_lo + s * (2048 >> 4), b_hi, TcBwd<D, DKV>::IDESC_TS,
+  for (int s = 0; s < TcBwd<D, DKV, SMALL>::KSTEPS_NH; s++)
+    mma_ts_lohi<KIND_F16>(d_tmem, a_tmem + s * 8, b_lo + s * (2048 >> 4), b_hi, TcBwd<D, DKV, SMALL>::IDESC_TS,
                           (acc || s > 0) ? 1u : 0u);
 }
 
@@ -109,14 +112,14 @@ __device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* m, ui
 // tiles K, V), Q and dO of the group's query heads stream.
 // dK/dV with split > 1: a cluster of `split` CTAs shares a key tile, each walks its part of the group's query heads, and
 // the CTAs add their accumulators through distributed shared memory, column by column in rank order.
-template <int D, bool DKV>
-__global__ void __launch_bounds__(TcBwd<D, DKV>::NUM_THREADS, 1)
+template <int D, bool DKV, bool SMALL>
+__global__ void __launch_bounds__(TcBwd<D, DKV, SMALL>::NUM_THREADS, TcBwd<D, DKV, SMALL>::MIN_CTAS)
 train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const float* __restrict__ LSE, const float* __restrict__ delta, const float* __restrict__ mask,
                     float* __restrict__ out0, float* __restrict__ out1, int N, int Hq, int Hkv, int grouped, int split,
                     int causal, uint32_t* status, uint32_t* sticky) {
-  using C = TcBwd<D, DKV>;
+  using C = TcBwd<D, DKV, SMALL>;
   constexpr int ST = C::STAGES, SL = C::SLOTS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -170,7 +173,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     fence_mbar_init();
   }
   if (warp == C::W_MMA) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -194,7 +197,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   };
 
-  if constexpr (C::EW_REGS > C::LAUNCH_REGS) {
+  if constexpr (C::MOVE_REGS) {
     if (warp >= C::W_PROD) setmaxnreg_dec<C::SERVICE_REGS>();
   }
   if (warp == C::W_PROD) {
@@ -235,8 +238,8 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (!__all_sync(0xffffffffu, mbar_wait(&slot_full[n % SL], (n / SL) & 1, wctx, 0x52))) return false;
       tc_fence_after();
       const uint32_t x = ring0 + (n % SL) * (2 * C::STREAM_BYTES >> 4), y = x + (C::STREAM_BYTES >> 4);
-      mma_abt<D, DKV>(tb + st * 2 * NH, a0, (uint32_t)k_proto | x, k_hi);       // S = Q K^T     | S^T = K Q^T
-      mma_abt<D, DKV>(tb + st * 2 * NH + NH, a1, (uint32_t)k_proto | y, k_hi);  // dP = dO V^T   | dP^T = V dO^T
+      mma_abt<D, DKV, SMALL>(tb + st * 2 * NH, a0, (uint32_t)k_proto | x, k_hi);       // S = Q K^T     | S^T = K Q^T
+      mma_abt<D, DKV, SMALL>(tb + st * 2 * NH + NH, a1, (uint32_t)k_proto | y, k_hi);  // dP = dO V^T   | dP^T = V dO^T
       commit_one(&s_full[st]);
       return true;
     };
@@ -249,10 +252,10 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint32_t x = ring0 + (n % SL) * (2 * C::STREAM_BYTES >> 4), y = x + (C::STREAM_BYTES >> 4);
       const uint32_t s_cols = tb + st * 2 * NH, p_cols = s_cols + NH;
       if constexpr (DKV) {
-        mma_tb<D, DKV>(tb + col_acc, s_cols, (uint32_t)mn_proto | y, mn_hi, n > 0);      // dV += P^T dO
-        mma_tb<D, DKV>(tb + col_acc + D, p_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);  // dK += dS^T Q
+        mma_tb<D, DKV, SMALL>(tb + col_acc, s_cols, (uint32_t)mn_proto | y, mn_hi, n > 0);      // dV += P^T dO
+        mma_tb<D, DKV, SMALL>(tb + col_acc + D, p_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);  // dK += dS^T Q
       } else {
-        mma_tb<D, DKV>(tb + col_acc, s_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);      // dQ += dS K
+        mma_tb<D, DKV, SMALL>(tb + col_acc, s_cols, (uint32_t)mn_proto | x, mn_hi, n > 0);      // dQ += dS K
       }
       commit_one(&slot_empty[n % SL]);
       if (n + ST < steps) ok = scores(n + ST);
@@ -260,7 +263,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (ok) commit_one(acc_full);
   } else if (warp < C::W_PROD) {
     // element-wise: warpgroup wg takes steps wg, wg + STAGES, ...; thread r owns the CTA's row row0 + r
-    if constexpr (C::EW_REGS > C::LAUNCH_REGS) setmaxnreg_inc<C::EW_REGS>();
+    if constexpr (C::MOVE_REGS) setmaxnreg_inc<C::EW_REGS>();
     const int wg = warp >> 2;
     const int r = tid & 127;
     const int row = row0 + r;
@@ -303,9 +306,10 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         break;
       }
       tc_fence_after();
-      // a step whose 128 x 64 block lies inside the sequence, on the visible side of the causal diagonal and under no
-      // additive mask needs none of the per-element tests: two lanes per instruction
-      const bool interior = mask == nullptr && row0 + T <= N && c0 + NH <= N &&
+      // a step whose 64 streamed rows lie inside the sequence, on the visible side of the causal diagonal and under no
+      // additive mask needs none of the per-element tests: two lanes per instruction.  (The CTA's own rows past the end
+      // may hold anything: a row of P or dS reaches its own row of the accumulators only, and that one is not stored.)
+      const bool interior = mask == nullptr && c0 + NH <= N &&
                             (!causal || (DKV ? row0 + T - 1 <= c0 : c0 + NH - 1 <= row0));
       // 16 columns at a time, the next 16 on their way meanwhile: [0, 16) of a buffer are scores, [16, 32) dP
       uint32_t buf[2][32];
@@ -422,7 +426,7 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == C::W_MMA) tmem_dealloc(tb, 512);
+  if (warp == C::W_MMA) tmem_dealloc(tb, C::TMEM_COLS);
 }
 
 // delta[row] = O_row . dO_row and the bf16 copy of dO in one pass over both: D / 4 lanes per row.
@@ -460,10 +464,10 @@ __global__ void __launch_bounds__(256) train_convert_kernel(const float* __restr
   }
 }
 
-template <int D, bool DKV>
-cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
-  using C = TcBwd<D, DKV>;
-  auto kern = train_bwd_tc_kernel<D, DKV>;
+template <int D, bool DKV, bool SMALL>
+cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, int split, cudaStream_t stream) {
+  using C = TcBwd<D, DKV, SMALL>;
+  auto kern = train_bwd_tc_kernel<D, DKV, SMALL>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -476,14 +480,6 @@ cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
   const int heads = a.B * (DKV ? a.Hkv : a.Hq), group = a.Hq / a.Hkv, tiles = (a.S + T - 1) / T;
   // bf16 bytes that stream past a tile: Q and dO of the group's heads, or the shared K and V
   const size_t head_bytes = (size_t)a.S * D * 4 * (DKV ? group : 1) / (DKV ? 1 : group);
-  // dK/dV of a GQA group: few CTAs with `group` times a head's steps each.  Below four of them per SM the query heads of
-  // the group are dealt out over a cluster (its largest divisor up to 8), so that the last CTA to end -- under a causal
-  // mask the one of the first keys -- has a `split`-th of the work.
-  // Measured, B=2 Hq=16 Hkv=4 S=1531 D=128 causal: 168 us for dK/dV before the steps in flight and the split, 93 with both.
-  int split = 1;
-  if (DKV && (long long)tiles * heads < 4 * 148)
-    for (int d = 2; d <= 8; d++)
-      if (group % d == 0) split = d;
   cudaLaunchConfig_t cfg = {};
   const CtaGrid g = cta_grid(head_bytes, heads, tiles, split);
   cfg.gridDim = g.grid;
@@ -504,12 +500,73 @@ cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
+// The forms that end first by estimate, in microseconds, from measurements of every form at 536 shapes (S = 64 to 8192, 12
+// to 1500 heads, groups of 1 to 16).  Over those shapes the choice lies 0.3 % on average above the best of the forms, and
+// none is slower than two CTAs per SM without steps issued ahead, which used to serve every D = 64 call.
+TrainTcPlan train_tc_plan(int B, int Hq, int Hkv, int S, int D, int causal) {
+  TrainTcPlan p{0, 0, 1};
+  const int group = Hq / Hkv, tiles = (S + T - 1) / T, steps = (S + NH - 1) / NH;
+  // steps of the average tile and, under a causal mask, of the heaviest one, before which no launch ends
+  const double mean = causal ? 0.5 * (steps + 2 < 2 * steps ? steps + 2 : 2 * steps) : steps;
+  const double most = causal ? steps : 0.0;
+  // D = 64, two CTAs per SM: one CTA's set-up and hand-overs run under the other's, which is worth 2 to 3 us per pair; a
+  // CTA that is alone on its SM takes nearly twice as long per step.  So: short walks in more than one round of CTAs
+  // (768 heads of S=197: 254 us with one CTA per SM, 216 with two; 24 heads of S=768: 33 and 47).
+  struct Form {
+    double set_up, step;              // one CTA per SM
+    double pair_set_up, pair_step;    // two: both CTAs
+    double alone_set_up, alone_step;  // ... and one that has its SM to itself
+  };
+  auto two_per_sm = [&](const Form& f, long long ctas, int heads) {
+    if (D != 64 || ctas <= 148) return 0;
+    const double one = (double)((ctas + 147) / 148) * (f.set_up + f.step * mean * heads);
+    const long long rest = ctas % 296;
+    double two = (double)(ctas / 296) * (f.pair_set_up + f.pair_step * mean * heads);
+    if (rest > 148)
+      two += f.pair_set_up + f.pair_step * mean * heads;
+    else if (rest > 0)
+      two += f.alone_set_up + f.alone_step * mean * heads;
+    const double one_least = f.set_up + f.step * most * heads, two_least = f.pair_set_up + f.pair_step * most * heads;
+    return (two > two_least ? two : two_least) < (one > one_least ? one : one_least) ? 1 : 0;
+  };
+  p.small_dq = two_per_sm({3.5, 0.54, 5.0, 1.08, 2.9, 1.06}, (long long)tiles * B * Hq, 1);
+  // dK/dV of a GQA group: few CTAs with `group` times a head's steps each.  The query heads of the group may be dealt out
+  // over a cluster, so that the last CTA to end has a `split`-th of the work; each CTA then pays its own set-up, two
+  // cluster barriers and the sum over the ranks, and clusters of some sizes leave SMs of an 18-SM group idle.  It pays
+  // where less than a round of CTAs has long walks (B=1 Hq=16 Hkv=2 S=1531 D=64: 193 us, 87 over four) and costs where
+  // there are several rounds (B=36 Hq=64 Hkv=8 S=256: 406 us, 841 over eight).
+  const long long ctas = (long long)tiles * B * Hkv;
+  double least = 0.0;
+  for (int split = 1; split <= 8; split++) {
+    if (group % split != 0) continue;
+    const double set_up = split == 1 ? 4.0 : 4.0 + 2.0 * sqrt((double)split), step = D == 64 ? 0.78 : 1.08;
+    const int resident = split == 1 ? 148 : 8 * (18 / split) * split, heads = group / split;
+    const double rounds = (double)(ctas * split) / resident, heaviest = set_up + step * heads * steps;
+    double t = ceil(rounds) * heaviest;
+    if (causal) {
+      t = 1.15 * rounds * (set_up + step * heads * 0.5 * (steps + 2));
+      if (t < heaviest) t = heaviest;
+    }
+    if (split == 1 || t < least * (p.split == 1 ? 0.97 : 1.0)) {
+      least = t;
+      p.split = split;
+    }
+  }
+  if (p.split == 1) p.small_dkv = two_per_sm({4.0, 0.66, 4.8, 1.72, 3.1, 1.5}, ctas, group);
+  return p;
+}
+
 cudaError_t launch_attn_train_backward_tc(const TrainBwdTcArgs& a, cudaStream_t stream, int* launches) {
   if (a.D != 64 && a.D != 128) return cudaErrorInvalidValue;
-  cudaError_t e = a.D == 64 ? launch_bwd_tc<64, false>(a, stream) : launch_bwd_tc<128, false>(a, stream);
+  const TrainTcPlan p = train_tc_plan(a.B, a.Hq, a.Hkv, a.S, a.D, a.causal);
+  cudaError_t e = a.D == 128   ? launch_bwd_tc<128, false, false>(a, 1, stream)
+                  : p.small_dq ? launch_bwd_tc<64, false, true>(a, 1, stream)
+                               : launch_bwd_tc<64, false, false>(a, 1, stream);
   if (e != cudaSuccess) return e;
   (*launches)++;
-  e = a.D == 64 ? launch_bwd_tc<64, true>(a, stream) : launch_bwd_tc<128, true>(a, stream);
+  e = a.D == 128    ? launch_bwd_tc<128, true, false>(a, p.split, stream)
+      : p.small_dkv ? launch_bwd_tc<64, true, true>(a, p.split, stream)
+                    : launch_bwd_tc<64, true, false>(a, p.split, stream);
   if (e != cudaSuccess) return e;
   (*launches)++;
   return cudaSuccess;

@@ -21,3 +21,22 @@ def test_exact_backward_grids_fit(b, hq, hkv, s, causal, d):
     for rows, heads, (x, y, z) in ((dq_rows, b * hq, grids[:3]), (dkv_rows, b * hkv, grids[3:])):
         assert 1 <= y <= 65535 and 1 <= z <= 65535 and 1 <= x < 1 << 31
         assert x * y * z == -(-s // rows) * heads
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_tc_backward_forms(causal):
+    """Two CTAs per SM for many short walks at D = 64, one CTA per SM elsewhere; a cluster per GQA group only where the key
+    tiles alone would leave SMs idle over long walks."""
+    plan = lambda *sizes: _abi.plan(_abi.PLAN_TRAIN_BACKWARD_TC, *sizes, causal)[:3]
+    assert plan(1, 768, 768, 64, 64) == [1, 1, 1]
+    assert plan(1, 768, 768, 197, 64) == [1, 1, 1]
+    assert plan(1, 768, 768, 197, 128) == [0, 0, 1]
+    assert plan(1, 24, 24, 768, 64) == [0, 0, 1]      # 144 CTAs: one round
+    assert plan(1, 1, 1, 1, 64) == [0, 0, 1]
+    assert plan(1, 16, 2, 1531, 64)[2] >= 4           # 24 key tiles, 8 query heads each
+    assert plan(1, 16, 2, 1531, 128)[2] >= 4
+    for b, hq, hkv, s, d in ((36, 64, 8, 256, 64), (16, 64, 8, 512, 64), (8, 56, 8, 1000, 64), (16, 40, 8, 384, 128),
+                             (36, 16, 8, 197, 128), (8, 64, 8, 197, 64)):
+        assert plan(b, hq, hkv, s, d)[2] == 1
+    group = plan(3, 21, 3, 500, 64)[2]
+    assert 7 % group == 0
