@@ -838,7 +838,7 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
   // completion reports want pairs to finish one by one
   const size_t head_bytes = a.progress.count != nullptr ? ~(size_t)0
                                                         : (size_t)a.S * D * (C::QK_ESIZE + C::V_ESIZE) / (size_t)(a.Hq / a.Hkv);
-  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + TILES * BM - 1) / (TILES * BM));
+  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + TILES * BM - 1) / (TILES * BM), a.causal || a.S % (TILES * BM) != 0);
   if constexpr (MODE != TC_SAGE) {
     if (a.mask != nullptr) return launch_grid<MODE, D, ROWS, true, ORDER_ARG>(a, g, stream);
   }

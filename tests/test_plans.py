@@ -40,3 +40,14 @@ def test_tc_backward_forms(causal):
         assert plan(b, hq, hkv, s, d)[2] == 1
     group = plan(3, 21, 3, 500, 64)[2]
     assert 7 % group == 0
+
+
+def test_grids_are_grouped_only_where_tiles_differ():
+    """Heaviest tiles first for the heads of a group: under a causal mask or with a partial tile.  Tiles of one weight keep
+    the grid of (tiles, heads), whose CTAs side by side share few heads' K and V."""
+    grid = lambda *sizes: tuple(_abi.plan(_abi.PLAN_TRAIN_BACKWARD, *sizes)[2:5])
+    assert grid(1, 148, 148, 256, 64, False) == (2, 148, 1)
+    heads_of_a_group, tiles, groups = grid(1, 148, 148, 250, 64, False)
+    assert (heads_of_a_group * groups, tiles) == (148, 2) and heads_of_a_group > 1
+    heads_of_a_group, tiles, groups = grid(1, 20, 20, 512, 64, True)
+    assert (heads_of_a_group * groups, tiles) == (20, 8) and heads_of_a_group > 1
