@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256) train_dq_kernel(const float* __restrict__
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int bh = cta_head(GROUPED);
   int tile = cta_tile(GROUPED);
-  if (causal) tile = cta_tiles(GROUPED) - 1 - tile;  // the last query tile sees the most keys
+  if (GROUPED && causal) tile = cta_tiles(GROUPED) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * BT;
@@ -219,11 +219,10 @@ __global__ void __launch_bounds__(256) train_dkv_kernel(const float* __restrict_
   float* sL = sDS + BT * C::LDP;
   float* sDl = sL + BT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int kvbh = cta_head(GROUPED);
-  const int tile = cta_tile(GROUPED);  // (under a causal mask the first key tile sees the most queries)
+  const int kvbh = GROUPED ? cta_head(1) : blockIdx.y;
   const int b = kvbh / Hkv, hk = kvbh - b * Hkv;
   const int group = Hq / Hkv;
-  const int k0 = tile * BT;
+  const int k0 = (GROUPED ? blockIdx.y : blockIdx.x) * BT;  // (under a causal mask the first key tile sees the most queries)
   const float scale = 1.0f / sqrtf((float)D);
   constexpr int OD = D / 64;
   load_tile<D>(sK, K + (size_t)kvbh * N * D, k0, N, tid);
@@ -590,10 +589,11 @@ cudaError_t configure() {
 
 // The 128-row tiles do their rows about 5 % faster than the 64-row ones, of which an SM holds two: the form whose
 // rounds come to fewer rows per SM (B=6 Hq=4 S=848: dQ 2 x 128 against 3 x 64, a step 7 % slower in the wide form).
-// Under a causal mask they want two rounds at least: one round ends with its heaviest tile.
+// Under a causal mask they want more than four rounds: their heaviest tiles, twice as long, end the launch (96 heads of
+// S=700: 764 us against 702 with 64 rows; 96 of S=848, 4.5 rounds: 1110 against 1230).
 bool worth_it(int S, int heads, int causal) {
   const long long w = (long long)((S + 127) / 128) * heads, n = (long long)((S + 63) / 64) * heads;
-  if (causal && w < 2 * 148) return false;
+  if (causal) return w > 4 * 148 + 74;
   return ((w + 147) / 148) * 128 * 20 <= ((n + 147) / 148) * 64 * 21;
 }
 }  // namespace wide
