@@ -366,8 +366,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
 
 }  // namespace
 
+// Up to one item per SM a launch is one chain of latencies, which the key loop's one-tile form gets through sooner: it reads
+// the scores once, into 128 registers, and hands P over in halves (12 heads of S=128: 5.3 us against 5.7, causal 5.8 and
+// 6.3, S=256 6.4 and 6.9).  With more, items under way side by side count.
 bool attn_short_takes(const TcArgs& a) {
-  return a.mode == TC_BF16 && a.D == D && a.S <= KEYS && a.mask == nullptr;
+  return a.mode == TC_BF16 && a.D == D && a.S <= KEYS && a.mask == nullptr &&
+         (long long)((a.S + BM - 1) / BM) * a.B * a.Hq > 148;
 }
 
 template <bool EXTRA>

@@ -50,6 +50,10 @@ using namespace arptx;
 __device__ int g_test_skip_k_tile = -1;
 #endif
 
+// Lengths up to which a call of the D = 64 bf16 kernel takes CTAs of one query tile instead of two: 128 with a mask (768
+// heads of S=100: 38.5 -> 25.3 us).  Without one, up to 256: what attn_short_takes leaves of those.
+constexpr int ONE_TILE_MASKED = 128, ONE_TILE_PLAIN = 256;
+
 constexpr int BM = 128;  // query rows per tile
 constexpr int BN = 128;  // keys per step
 constexpr int NPART = 2;  // P of a step is handed to the MMA warp in two halves of 64 keys
@@ -60,16 +64,22 @@ constexpr float LOG2E = 1.4426950408889634f;
 // masked row, as in the reference).
 constexpr float NEG = -1e30f * LOG2E;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
-// Two query tiles, 384 threads: softmax warpgroup 0, softmax warpgroup 1, {TMA producer, MMA issuer, 2 idle warps}; one CTA
-// per SM (all 512 TMEM columns).  setmaxnreg moves registers inside the pool the CTA was launched with (168 per thread);
-// an increase that the pool cannot cover waits forever.
-constexpr int TILES = 2;
-constexpr int NUM_THREADS = 128 * TILES + 128;
-constexpr int LAUNCH_REGS = 168;
-constexpr int SOFTMAX_REGS = 216;  // softmax warps after setmaxnreg
-constexpr int SERVICE_REGS = 72;   // the last warpgroup
-static_assert(TILES * 128 * SOFTMAX_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
-static_assert(LAUNCH_REGS * NUM_THREADS <= 65536, "register file of the SM");
+// Shape of a CTA.  TILES = 2: two query tiles, 384 threads -- softmax warpgroup 0, softmax warpgroup 1, {TMA producer, MMA
+// issuer, 2 idle warps}; one CTA per SM (all 512 TMEM columns).  TILES = 1: one query tile, 256 threads, 256 TMEM columns
+// and at most half of the shared memory and registers, so that two CTAs share an SM: for short sequences, whose second
+// warpgroup would have little to do.
+// setmaxnreg moves registers inside the pool the CTA was launched with (168 per thread for 384 threads, 128 per
+// thread for 256 threads at two CTAs per SM); an increase that the pool cannot cover waits forever.
+template <int TILES>
+struct Shape {
+  static constexpr int NUM_THREADS = 128 * TILES + 128;
+  static constexpr int MIN_CTAS = TILES == 1 ? 2 : 1;
+  static constexpr int LAUNCH_REGS = TILES == 1 ? 128 : 168;
+  static constexpr int SOFTMAX_REGS = TILES == 1 ? 208 : 216;  // softmax warps after setmaxnreg
+  static constexpr int SERVICE_REGS = TILES == 1 ? 48 : 72;    // the last warpgroup
+  static_assert(TILES * 128 * SOFTMAX_REGS + 128 * SERVICE_REGS <= LAUNCH_REGS * NUM_THREADS, "register pool of the CTA");
+  static_assert(LAUNCH_REGS * NUM_THREADS * MIN_CTAS <= 65536, "register file of the SM");
+};
 
 // Largest scale c of an INT8 step that may fold its conversion: (12582912 + 127 * 127 * 128) * c < 2^14.
 constexpr float FOLD_MAX_C = 1.0e-3f;
@@ -340,7 +350,7 @@ __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float
   l += lsum + lsum_hi;
 }
 
-template <int MODE, int D, bool MASKED = false>
+template <int MODE, int D, bool MASKED = false, int TILES = 2>
 struct Cfg {
   static constexpr bool QUANT = MODE == TC_SAGE || MODE == TC_SAGE_FP8;  // 8-bit Q and K with per-block scales
   static constexpr int QK_ESIZE = QUANT ? 1 : MODE == TC_TF32 ? 4 : 2;
@@ -364,16 +374,15 @@ struct Cfg {
   static constexpr int V_TILE_BYTES = BN * D * V_ESIZE;
   static constexpr int PV_KSTEPS = MODE == TC_TF32 ? BN / 8 : BN / 16;
   static constexpr int STAGES =
-      MASKED ? 2 : ((2 * Q_TILE_STRIDE + 3 * (QK_TILE_BYTES + V_TILE_BYTES) <= 200 * 1024) ? 3 : 2);
+      TILES == 1 ? (MASKED ? 1 : 2) : MASKED ? 2 : ((2 * Q_TILE_STRIDE + 3 * (QK_TILE_BYTES + V_TILE_BYTES) <= 200 * 1024) ? 3 : 2);
   static constexpr int SMEM_TILES = TILES * Q_TILE_STRIDE + STAGES * (QK_TILE_BYTES + V_TILE_BYTES);
   // chunks of the additive mask in flight per softmax warp (4 KB each): as many of a step's four as fit
-  static constexpr int MASK_RING = !MASKED ? 0 : (224 * 1024 - SMEM_TILES) / (TILES * 4 * 4096) >= 4 ? 4
-                                             : (224 * 1024 - SMEM_TILES) / (TILES * 4 * 4096) >= 2   ? 2
-                                                                                                     : 1;
+  static constexpr int RING_FITS = ((TILES == 1 ? 110 : 224) * 1024 - SMEM_TILES) / (TILES * 4 * 4096);
+  static constexpr int MASK_RING = !MASKED ? 0 : RING_FITS >= 4 ? 4 : RING_FITS >= 2 ? 2 : 1;
   static constexpr int MASK_BYTES = MASK_RING * TILES * 4 * 4096;
   static constexpr int NUM_BARS = 2 + 4 * STAGES + 4 + 2 * NPART;
   static constexpr int SMEM_BYTES = SMEM_TILES + MASK_BYTES + NUM_BARS * 8 + 16 + 1024;  // + alignment slack
-  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+  static_assert(SMEM_BYTES <= (TILES == 1 ? 113 : 227) * 1024, "shared memory budget");
   static constexpr int QK_KIND = MODE == TC_SAGE ? KIND_I8 : MODE == TC_SAGE_FP8 ? KIND_F8 : MODE == TC_TF32 ? KIND_TF32 : KIND_F16;
   static constexpr uint32_t IDESC_QK = MODE == TC_SAGE       ? make_idesc(2, 1, 1, 0, 0, BM, BN)  // s8 x s8 -> s32
                                        : MODE == TC_SAGE_FP8 ? make_idesc(1, 0, 0, 0, 0, BM, BN)  // e4m3 x e4m3 -> f32
@@ -385,15 +394,15 @@ struct Cfg {
 // ROWS: Sage with one scale per query row and per key row; MASKED: an additive mask (instantiations of their own, so
 // that the plain kernel carries none of either).
 // ORDER: the grid of cta_order.cuh, known when the plain kernel is compiled for the same reason; the heaviest query block is the last one of a causal call, else the partial one comes last.
-template <int MODE, int D, bool ROWS, bool MASKED, int ORDER>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+template <int MODE, int D, bool ROWS, bool MASKED, int ORDER, int TILES>
+__global__ void __launch_bounds__(Shape<TILES>::NUM_THREADS, Shape<TILES>::MIN_CTAS)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ out, const float* __restrict__ mask,
                    const float* __restrict__ q_scale, const float* __restrict__ k_scale, int N, int Hq, int Hkv,
                    int grouped_arg, int causal, int out_f32, int token_major, long long o_sb, long long o_sh, long long o_ss,
                    const OutReplicas reps, const OutProgress progress, float* __restrict__ lse_out, uint32_t* status,
                    uint32_t* sticky, uint32_t ticket) {
-  using C = Cfg<MODE, D, MASKED>;
+  using C = Cfg<MODE, D, MASKED, TILES>;
   constexpr int ST = C::STAGES;
   const bool grouped = ORDER == ORDER_ARG ? grouped_arg != 0 : ORDER == ORDER_GROUPED;
   constexpr int W_PROD = 4 * TILES;     // warp that loads
@@ -517,7 +526,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after();
   const uint32_t tb = *tmem_slot;
 
-  if (warp >= W_PROD) setmaxnreg_dec<SERVICE_REGS>();
+  if (warp >= W_PROD) setmaxnreg_dec<Shape<TILES>::SERVICE_REGS>();
   if (warp == W_PROD) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -636,7 +645,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     }
   } else if (warp < W_PROD) {
     // ------------------------------------------------------------ softmax warps
-    setmaxnreg_inc<SOFTMAX_REGS>();
+    setmaxnreg_inc<Shape<TILES>::SOFTMAX_REGS>();
     const int t = warp >> 2;
     const int r = tid & 127;
     const int row = q0 + t * BM + r;
@@ -812,10 +821,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int MODE, int D, bool ROWS, bool MASKED, int ORDER>
+template <int MODE, int D, bool ROWS, bool MASKED, int ORDER, int TILES = 2>
 cudaError_t launch_grid(const TcArgs& a, const CtaGrid& g, cudaStream_t stream) {
-  using C = Cfg<MODE, D, MASKED>;
-  auto kern = attn_fwd_tc_kernel<MODE, D, ROWS, MASKED, ORDER>;
+  using C = Cfg<MODE, D, MASKED, TILES>;
+  auto kern = attn_fwd_tc_kernel<MODE, D, ROWS, MASKED, ORDER, TILES>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -825,10 +834,9 @@ cudaError_t launch_grid(const TcArgs& a, const CtaGrid& g, cudaStream_t stream) 
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  kern<<<g.grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale, a.k_scale, a.S, a.Hq,
-                                                       a.Hkv, g.grouped, a.causal, a.out_f32, a.token_major, a.o_sb, a.o_sh,
-                                                       a.o_ss, a.replicas, a.progress, a.lse_out, a.status, a.sticky,
-                                                       a.ticket);
+  kern<<<g.grid, Shape<TILES>::NUM_THREADS, C::SMEM_BYTES, stream>>>(
+      a.tm_q, a.tm_k, a.tm_v, a.out, a.mask, a.q_scale, a.k_scale, a.S, a.Hq, a.Hkv, g.grouped, a.causal, a.out_f32,
+      a.token_major, a.o_sb, a.o_sh, a.o_ss, a.replicas, a.progress, a.lse_out, a.status, a.sticky, a.ticket);
   return cudaGetLastError();
 }
 
@@ -838,7 +846,14 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
   // completion reports want pairs to finish one by one
   const size_t head_bytes = a.progress.count != nullptr ? ~(size_t)0
                                                         : (size_t)a.S * D * (C::QK_ESIZE + C::V_ESIZE) / (size_t)(a.Hq / a.Hkv);
-  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + TILES * BM - 1) / (TILES * BM), a.causal || a.S % (TILES * BM) != 0);
+  if constexpr (MODE == TC_BF16 && D == 64) {
+    if (a.S <= (a.mask != nullptr ? ONE_TILE_MASKED : ONE_TILE_PLAIN)) {
+      const CtaGrid g = {dim3((unsigned)((a.S + BM - 1) / BM), (unsigned)(a.B * a.Hq), 1), 0};
+      return a.mask != nullptr ? launch_grid<MODE, D, ROWS, true, ORDER_PLAIN, 1>(a, g, stream)
+                               : launch_grid<MODE, D, ROWS, false, ORDER_PLAIN, 1>(a, g, stream);
+    }
+  }
+  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + 2 * BM - 1) / (2 * BM), a.causal || a.S % (2 * BM) != 0);
   if constexpr (MODE != TC_SAGE) {
     if (a.mask != nullptr) return launch_grid<MODE, D, ROWS, true, ORDER_ARG>(a, g, stream);
   }

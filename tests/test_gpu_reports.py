@@ -17,7 +17,7 @@ def _words(torch, n):
 
 @pytest.mark.parametrize("mode,B,Hq,Hkv,S,D,causal", [
     ("bf16", 2, 4, 4, 700, 128, True),
-    ("bf16", 3, 4, 2, 197, 64, False),   # the one-tile form of short sequences
+    ("bf16", 3, 4, 2, 197, 64, False),   # the one-pass kernel of short sequences
     ("sage", 1, 6, 3, 1000, 128, False),
     ("sage_fp8", 1, 4, 4, 300, 64, True),
 ])
