@@ -153,6 +153,10 @@ struct PrologueArgs {
   uint32_t* status = nullptr;  // device word a bounded wait that ran out is recorded in; cleared by the caller
   uint32_t* sticky = nullptr;  // the library's accumulator of the same bits
 };
+// How the K mean of a smoothed call is added up: by one CTA per K head, by a cluster per K head, or from span sums that
+// a launch of the quantiser leaves.  The same bits.
+enum { SAGE_MEAN_ONE_CTA, SAGE_MEAN_CLUSTER, SAGE_MEAN_SPANS };
+int sage_mean_form(int dtype, int kv_heads, int S);
 // Returns the number of kernels launched through *launches.
 cudaError_t launch_sage_prologue(const PrologueArgs& a, cudaStream_t stream, int* launches);
 // [BH, S, D] f32 -> [BH, D, S_pad] f32 (S_pad = S rounded up to 4; the padding is zeroed): the K-major V

@@ -16,6 +16,7 @@
 // subtraction, and the division and reciprocal are IEEE.
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 namespace ar {
@@ -122,6 +123,81 @@ __global__ void __launch_bounds__(MEAN_SLOTS * D) k_mean_kernel(const void* __re
   if (tid < D) k_mean[(size_t)blockIdx.x * D + tid] = total * (1.0f / (float)S);
 }
 
+// The same mean with the spans of one (batch, kv head) pair spread over a cluster of MEAN_CLUSTER CTAs, so
+// that a handful of heads still fills the GPU.  Every CTA leaves the sums of its spans in its own shared
+// memory; CTA 0 of the cluster then adds all of them in span order through distributed shared memory --
+// the order, and therefore every bit, of the single-CTA kernel.  grid = (MEAN_CLUSTER, B * Hkv).
+constexpr int MEAN_CLUSTER = 8;
+template <int DTYPE, int D>
+__global__ void __launch_bounds__(MEAN_SLOTS * D) k_mean_cluster_kernel(const void* __restrict__ K,
+                                                                        float* __restrict__ k_mean, int S, int per) {
+  namespace cg = cooperative_groups;
+  constexpr int CH = D / 8;
+  __shared__ float run_sums[MEAN_SLOTS][8][D];
+  extern __shared__ float my_spans[];  // [per][D]: sums of the spans this CTA owns; then [nspan][D], used by CTA 0
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x;
+  const int slot = tid / D;
+  const int g = (tid % D) / CH;
+  const int c = tid % CH;
+  const size_t base = (size_t)blockIdx.y * S * D;
+  const int nspan = (S + 127) / 128;
+  const int first = rank * per, last = min(nspan, first + per);
+  for (int span0 = first; span0 < last; span0 += MEAN_SLOTS) {
+    const int span = span0 + slot;
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[i] = 0.f;
+    if (span < last) {
+      const int t0 = span * 128 + g * 16;
+#pragma unroll
+      for (int half = 0; half < 2; half++) {
+        float x[8][8];
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+          if (t0 + half * 8 + t < S) load8<DTYPE>(K, base + (size_t)(t0 + half * 8 + t) * D + c * 8, x[t]);
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+          if (t0 + half * 8 + t < S) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) acc[i] += x[t][i];
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) run_sums[slot][g][c * 8 + i] = acc[i];
+    __syncthreads();
+    if (span < last) {
+      // thread (slot, d): the 8 run sums of its span, left to right
+      const int d = tid % D;
+      float sum = 0.f;
+#pragma unroll
+      for (int gg = 0; gg < 8; gg++) sum += run_sums[slot][gg][d];
+      my_spans[(size_t)(span - first) * D + d] = sum;
+    }
+    __syncthreads();  // run_sums is rewritten by the next round
+  }
+  cluster.sync();  // every CTA's span sums are in place
+  if (rank == 0) {
+    // all threads fetch the other CTAs' sums side by side (remote loads are slow one at a time) ...
+    float* all_spans = my_spans + (size_t)per * D;  // [nspan][D]
+    for (int i = tid; i < nspan * D; i += MEAN_SLOTS * D) {
+      const int sp = i / D, r = sp / per;
+      const float* theirs = cluster.map_shared_rank(my_spans, r);
+      all_spans[i] = theirs[(size_t)(sp - r * per) * D + (i - sp * D)];
+    }
+    __syncthreads();
+    // ... and one thread per channel adds them in span order
+    if (tid < D) {
+      float total = 0.f;
+      for (int sp = 0; sp < nspan; sp++) total += all_spans[(size_t)sp * D + tid];
+      k_mean[(size_t)blockIdx.y * D + tid] = total * (1.0f / (float)S);
+    }
+  }
+  cluster.sync();  // nobody's shared memory goes away while CTA 0 reads it
+}
+
 // The mean of longer sequences from the span sums that the quantiser's first launch leaves (see below): one CTA per
 // (batch, kv head) adds them in span order -- the order, and therefore every bit, of the kernel above.
 template <int D>
@@ -180,11 +256,13 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const void* __restri
 // tens of KB of reads in flight the whole time instead of one load-reduce-store round per CTA.
 // Needs 16-byte aligned Q and K.
 // With smoothing, K can only be quantised when its mean is known, but Q can be before: sequences of 16
-// spans and more take two launches of this kernel, Q blocks quantised and K blocks summed (PART_Q_AND_SUMS), and after
+// spans and more (sage_mean_form) take two launches of this kernel, Q blocks quantised and K blocks summed (PART_Q_AND_SUMS), and after
 // k_mean_of_spans_kernel the K blocks quantised (PART_K).  The sum pass over K then streams beside Q's instead of
 // in a launch of its own.  Measured, mean and quantisation: 16 K heads of S=3001 with 64 of Q 48
 // us (cluster mean) -> 31, B=4 H=32 S=8192 214 -> 208.
-enum { PART_ALL, PART_Q_AND_SUMS, PART_K };
+// The part is a template parameter: with it as an argument the plain form lost 2 to 5 % (B=1, 128 heads of 1000 f32
+// tokens, D = 128, with the mean: 45.4 -> 48.0 us).
+enum { PART_ALL, PART_Q_AND_SUMS, PART_SUMS, PART_K };
 template <int DTYPE, int D>
 struct QuantPipe {
   static constexpr int ES = DTYPE == 1 ? 2 : 4;
@@ -226,12 +304,12 @@ __device__ __forceinline__ void load4_shared(const uint8_t* p, float* x) {
   }
 }
 
-template <int DTYPE, int D>
+template <int DTYPE, int D, int PART>
 __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restrict__ Q, const void* __restrict__ K,
                                                             const float* __restrict__ k_mean, int8_t* __restrict__ q8,
                                                             int8_t* __restrict__ k8, float* __restrict__ q_scale,
                                                             float* __restrict__ k_scale, int S, int BHq, int BHk,
-                                                            int smooth, int fp8, int part, float* __restrict__ span_sums,
+                                                            int smooth, int fp8, float* __restrict__ span_sums,
                                                             uint32_t* status, uint32_t* sticky) {
   using P = QuantPipe<DTYPE, D>;
   constexpr int CH = D / 8;
@@ -241,12 +319,13 @@ __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restri
   uint8_t* ring = (uint8_t*)(((uintptr_t)qp_smem_raw + 127) & ~(uintptr_t)127);
   __shared__ uint64_t full[ST];
   __shared__ float warp_max[2][8];
-  __shared__ float run_sums[8][D];
+  constexpr bool SUMS = PART == PART_Q_AND_SUMS || PART == PART_SUMS;
+  __shared__ float run_sums[SUMS ? 8 : 1][D];
   __shared__ uint32_t abort_flag;
   const int tid = threadIdx.x;
   const int nblk = (S + 127) / 128;
   const int q_items = BHq * nblk, items = (BHq + BHk) * nblk;
-  const int first = (part == PART_K ? q_items : 0) + blockIdx.x;
+  const int first = (PART == PART_K || PART == PART_SUMS ? q_items : 0) + blockIdx.x;
   if (tid == 0) {
     abort_flag = 0;
     for (int i = 0; i < ST; i++) arptx::mbar_init(&full[i], 1);
@@ -291,14 +370,14 @@ __global__ void __launch_bounds__(256) quantize_pipe_kernel(const void* __restri
     float mu[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) mu[i] = 0.f;
-    if (is_k && smooth && part != PART_Q_AND_SUMS) {
+    if (is_k && smooth && !SUMS) {
 #pragma unroll
       for (int i = 0; i < 8; i++) mu[i] = k_mean[(size_t)bh * D + c * 8 + i];
     }
     const bool ok = arptx::mbar_wait(&full[stage], (uint32_t)(it / ST) & 1u, arptx::WaitCtx{&abort_flag, status, sticky}, 0x40);
     if (!__syncthreads_and(ok)) break;  // a copy that never lands: the status word says so, the CTA leaves together
     const uint8_t* blockp = ring + stage * P::BLOCK_BYTES;
-    if (is_k && part == PART_Q_AND_SUMS) {
+    if (SUMS && is_k) {
       // thread (run of 16 tokens, 4 channels): the run left to right; then thread d: the 8 runs left to right
       const int g = tid / (D / 4), c4 = tid % (D / 4);
       if (g < 8) {
@@ -395,67 +474,100 @@ __global__ void __launch_bounds__(256) transpose_v_kernel(const float* __restric
     if (s0 + tx < S_pad) dst[(size_t)(d0 + r) * S_pad + s0 + tx] = tile[tx][r];
 }
 
+// One launch of the pipelined quantiser over the items of its part.
+template <int DTYPE, int D, int PART>
+cudaError_t launch_quantize_part(const PrologueArgs& a, int items, cudaStream_t stream, int* launches) {
+  using P = QuantPipe<DTYPE, D>;
+  auto kern = quantize_pipe_kernel<DTYPE, D, PART>;
+  static bool configured[64] = {};
+  static int sm_count[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && !configured[dev]) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  const int resident = (dev < 64 ? sm_count[dev] : 148) * P::CTAS_PER_SM;
+  // the span sums lie in the place of K's 8-bit copy, which only a later launch writes
+  kern<<<items < resident ? items : resident, 256, P::SMEM_BYTES, stream>>>(
+      a.q, a.k, a.k_mean, a.q8, a.k8, a.q_scale, a.k_scale, a.S, a.B * a.Hq, a.B * a.Hkv, a.smooth, a.fp8, (float*)a.k8,
+      a.status, a.sticky);
+  (*launches)++;
+  return cudaGetLastError();
+}
+
 template <int DTYPE, int D>
 cudaError_t launch_prologue_t(const PrologueArgs& a, cudaStream_t stream, int* launches) {
   const int nblk = (a.S + 127) / 128;
   const int bhq = a.B * a.Hq, bhk = a.B * a.Hkv;
   *launches = 0;
-  // Below 16 spans the two more launches cost more than the mean's rounds of MEAN_SLOTS spans do (B=2, 64 + 16 heads of
-  // S=1500: 20.6 us against 26.7; S=2000 27.7 against 26.7; S=5000 61 against 51).
-  const bool two_part = a.smooth && a.block != 1 && nblk >= 4 * MEAN_SLOTS;
-  if (a.smooth) {
-    if (!two_part) {
-      k_mean_kernel<DTYPE, D><<<bhk, MEAN_SLOTS * D, 0, stream>>>(a.k, a.k_mean, a.S);
-      (*launches)++;
-    }
+  cudaError_t e = cudaSuccess;
+  const int mean = a.smooth ? sage_mean_form(a.dtype, bhk, a.S) : SAGE_MEAN_ONE_CTA;
+  const bool spans = mean == SAGE_MEAN_SPANS;
+  if (!a.smooth) {
+    e = cudaMemsetAsync(a.k_mean, 0, sizeof(float) * (size_t)bhk * D, stream);
+  } else if (mean == SAGE_MEAN_CLUSTER) {
+    const int per = (nblk + MEAN_CLUSTER - 1) / MEAN_CLUSTER;  // spans per CTA of a cluster
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(MEAN_CLUSTER, bhk, 1);
+    cfg.blockDim = dim3(MEAN_SLOTS * D, 1, 1);
+    cfg.dynamicSmemBytes = (size_t)(per + nblk) * D * sizeof(float);  // (beside 16 KB, at most 36 spans of 512 bytes)
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = MEAN_CLUSTER;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, k_mean_cluster_kernel<DTYPE, D>, a.k, a.k_mean, a.S, per);
+    (*launches)++;
+  } else if (!spans) {
+    k_mean_kernel<DTYPE, D><<<bhk, MEAN_SLOTS * D, 0, stream>>>(a.k, a.k_mean, a.S);
+    (*launches)++;
+    e = cudaGetLastError();
   } else {
-    cudaError_t e = cudaMemsetAsync(a.k_mean, 0, sizeof(float) * (size_t)bhk * D, stream);
+    // 128-token blocks: beside the quantisation of Q; the other granularity quantises in a kernel of its own
+    e = a.block == 1 ? launch_quantize_part<DTYPE, D, PART_SUMS>(a, bhk * nblk, stream, launches)
+                     : launch_quantize_part<DTYPE, D, PART_Q_AND_SUMS>(a, (bhq + bhk) * nblk, stream, launches);
     if (e != cudaSuccess) return e;
+    k_mean_of_spans_kernel<D><<<bhk, D, 0, stream>>>((const float*)a.k8, a.k_mean, a.S, nblk);
+    (*launches)++;
+    e = cudaGetLastError();
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (a.block == 1) {
     const long long q_rows = (long long)bhq * a.S, all_rows = q_rows + (long long)bhk * a.S;
     const int rows_per_cta = 256 / (D / 8);
     quantize_rows_kernel<DTYPE, D><<<(unsigned)((all_rows + rows_per_cta - 1) / rows_per_cta), 256, 0, stream>>>(
         a.q, a.k, a.k_mean, a.q8, a.k8, a.q_scale, a.k_scale, a.S, q_rows, all_rows, a.smooth, a.fp8);
-  } else {
-    // 128-token blocks: the pipelined kernel, one or two CTAs per SM (its bulk copies need 16-byte aligned sources,
-    // which every caller of this function guarantees)
-    using P = QuantPipe<DTYPE, D>;
-    auto kern = quantize_pipe_kernel<DTYPE, D>;
-    static bool configured[64] = {};
-    static int sm_count[64] = {};
-    int dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 64 && !configured[dev]) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM_BYTES);
-      if (e != cudaSuccess) return e;
-      e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-      if (e != cudaSuccess) return e;
-      configured[dev] = true;
-    }
-    const int resident = (dev < 64 ? sm_count[dev] : 148) * P::CTAS_PER_SM;
-    auto launch = [&](int part, int items) {
-      kern<<<items < resident ? items : resident, 256, P::SMEM_BYTES, stream>>>(
-          a.q, a.k, a.k_mean, a.q8, a.k8, a.q_scale, a.k_scale, a.S, bhq, bhk, a.smooth, a.fp8, part, (float*)a.k8, a.status,
-          a.sticky);
-    };
-    if (two_part) {  // the span sums lie in the place of K's 8-bit copy, which only the last launch writes
-      launch(PART_Q_AND_SUMS, (bhq + bhk) * nblk);
-      k_mean_of_spans_kernel<D><<<bhk, D, 0, stream>>>((const float*)a.k8, a.k_mean, a.S, nblk);
-      launch(PART_K, bhk * nblk);
-      (*launches) += 2;
-    } else {
-      launch(PART_ALL, (bhq + bhk) * nblk);
-    }
+    (*launches)++;
+    return cudaGetLastError();
   }
-  (*launches)++;
-  return cudaGetLastError();
+  // 128-token blocks: the pipelined kernel, one or two CTAs per SM (its bulk copies need 16-byte aligned sources,
+  // which every caller of this function guarantees)
+  return spans ? launch_quantize_part<DTYPE, D, PART_K>(a, bhk * nblk, stream, launches)
+               : launch_quantize_part<DTYPE, D, PART_ALL>(a, (bhq + bhk) * nblk, stream, launches);
 }
 
 }  // namespace
+
+// Below 16 spans of 128 tokens one CTA per K head is as fast as any form.  From there on the span sums, beside the
+// quantisation of Q, where they save a pass over K in a launch of its own.  bf16, mean and quantisation: 64 heads of Q and 16
+// of K, S=3001, D = 128 31 us against 42; B=4 H=32 S=8192 212 against 219; one head of S=20000 17 against 62.  f32
+// tensors keep the other forms where those are ahead: the cluster for up to nine heads of up to 32 spans (8 heads of S=3001,
+// D = 128: 17.3 us, 18.8 from span sums; 18 heads 28.8 and 25.1), one CTA per head from 96 heads on (128 heads of S=3001: 125 us and 130).
+int sage_mean_form(int dtype, int kv_heads, int S) {
+  const int spans = (S + 127) / 128;
+  if (spans < 4 * MEAN_SLOTS) return SAGE_MEAN_ONE_CTA;
+  if (dtype == 0 && kv_heads * MEAN_CLUSTER <= 74 && spans <= 32) return SAGE_MEAN_CLUSTER;
+  if (dtype == 0 && kv_heads >= 96) return SAGE_MEAN_ONE_CTA;
+  return SAGE_MEAN_SPANS;
+}
 
 cudaError_t launch_sage_prologue(const PrologueArgs& a, cudaStream_t stream, int* launches) {
   if (a.dtype == 1 && a.D == 128) return launch_prologue_t<1, 128>(a, stream, launches);

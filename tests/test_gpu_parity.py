@@ -167,13 +167,17 @@ def test_fully_masked_row_returns_mean_of_v(ops, oracle_lib):
 PROLOGUE_SHAPES = [(1, 2, 2, 256, 128, True), (2, 4, 2, 300, 128, True), (1, 2, 2, 197, 64, True),
                    (1, 2, 1, 1000, 128, False), (1, 3, 3, 1, 128, True), (1, 2, 2, 129, 64, False),
                    (1, 2, 2, 4096, 128, True),
-                   # the K mean over a cluster of CTAs with a ragged split of the spans; then too many heads for it
-                   (1, 2, 1, 2500, 128, True), (1, 20, 20, 2048, 64, True)]
+                   # the K mean from span sums (16 spans of 128 tokens and more) on both sides of its limit, few heads and many
+                   (1, 2, 1, 2500, 128, True), (1, 20, 20, 2048, 64, True), (1, 2, 1, 1920, 64, False),
+                   (1, 2, 1, 1921, 64, False), (1, 2, 2, 1920, 128, False), (1, 2, 2, 2049, 128, False),
+                   (1, 2, 1, 1921, 64, True), (1, 100, 100, 1921, 64, False), (1, 2, 1, 4096, 128, False),
+                   (1, 2, 1, 4100, 128, False), (1, 20, 20, 2048, 64, False)]
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,bf16", PROLOGUE_SHAPES)
 @pytest.mark.parametrize("smooth", [True, False])
-def test_sage_prologue_bit_exact(ops, oracle_lib, B, Hq, Hkv, S, D, bf16, smooth):
+@pytest.mark.parametrize("block", [128, 1])
+def test_sage_prologue_bit_exact(ops, oracle_lib, B, Hq, Hkv, S, D, bf16, smooth, block):
     import torch
     q, k, _ = normal_qkv(S + D, B, Hq, Hkv, S, D, k_offset_sigma=2.0)
     if bf16:
@@ -182,8 +186,8 @@ def test_sage_prologue_bit_exact(ops, oracle_lib, B, Hq, Hkv, S, D, bf16, smooth
     else:
         qi, ki = q, k
         tq, tk = to_dev(q), to_dev(k)
-    want = oracle_lib.sage_quantize(qi, ki, 128, smooth)
-    got = ops.sage_quantize(tq, tk, smooth)
+    want = oracle_lib.sage_quantize(qi, ki, block, smooth)
+    got = ops.sage_quantize(tq, tk, smooth, block=block)
     torch.cuda.synchronize()
     for name, g, w in zip(("q8", "k8", "q_scale", "k_scale", "k_mean"), got, want):
         g = g.cpu().numpy()
