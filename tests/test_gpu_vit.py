@@ -40,6 +40,24 @@ def test_vit_exact_f32_path(attn_lib):
     assert (ours - theirs).abs().max().item() <= 1e-4 * max(theirs.abs().max().item(), 1.0)
 
 
+def test_vit_position_embedding_of_one_row(attn_lib):
+    """A position embedding of one row is added to every token, as in the form without the fused passes; any other
+    number of rows than the tokens' is refused."""
+    import torch
+    from autorust_b200.vit import ViT
+    model = ViT(layers=1, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.rand(2, 3, 224, 224, device="cuda", generator=g)
+    row = model.pos[:, :1].clone()
+    model.pos = row.expand(-1, 197, -1).contiguous()
+    want = model.forward(x)
+    model.pos = row
+    assert torch.equal(model.forward(x), want)
+    model.pos = row.expand(-1, 5, -1).contiguous()
+    with pytest.raises(RuntimeError):
+        model.forward(x)
+
+
 def test_vit_view_form_equals_copy_form(attn_lib):
     """One QKV GEMM with the kernel reading and writing [B, S, H, D] views, against the reference's form (separate
     projections, materialised transposes): the attention inputs are the same numbers, so the logits agree to the
