@@ -157,7 +157,7 @@ def attn_forward_views(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: 
     return out
 
 
-def views_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, stream: torch.cuda.Stream):
+def _views_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, stream: torch.cuda.Stream):
     """attn_forward_views (bf16, no mask, not causal) for a caller that makes the same call on many tensors of one layout,
     as the layers of an encoder do: checks and strides are worked out once, the function returned takes the device
     addresses of four tensors that differ from these in their memory only (same shapes, strides, dtype and device -- the
@@ -182,10 +182,10 @@ def views_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Ten
     return call
 
 
-def layernorm_call(x: torch.Tensor, stream: torch.cuda.Stream, eps: float = 1e-5):
+def _layernorm_call(x: torch.Tensor, stream: torch.cuda.Stream, eps: float = 1e-5):
     """add_layernorm for a caller that makes the same call many times: the function returned does x += residual (when
     there is one) and y = LayerNorm(x) * gamma + beta; y has x's layout, the other tensors are checked.  The same
-    terms as views_call."""
+    terms as _views_call."""
     L = _abi.load()
     _check_dense("x", x, x.shape, torch.bfloat16, x.device)
     cols = x.shape[-1]

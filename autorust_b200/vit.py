@@ -128,18 +128,20 @@ class ViT:
             stream = torch.cuda.current_stream()
             n, a = torch.empty_like(x), torch.empty_like(x)
             n2, a2 = n.view(B * S, E), a.view(B * S, E)
-            # q, k, v are views of one [B, S, 3E] product, read in place by the kernel; its output is [B, S, H, D] memory
-            qkv = torch.empty((B, S, 3, H, D), dtype=x.dtype, device=x.device)
-            attention = ops.views_call(*(qkv[:, :, j].transpose(1, 2) for j in range(3)),
-                                       a.view(B, S, H, D).transpose(1, 2), stream)
-            layernorm = ops.layernorm_call(x, stream)
-            a_at, third = a.data_ptr(), E * x.element_size()
+            layernorm = ops._layernorm_call(x, stream)
+            attention, a_at, third = None, a.data_ptr(), E * x.element_size()
             layernorm(x, None, *self.blocks[0]["ln1"], n)
             for i, blk in enumerate(self.blocks):
                 w, bias = blk["qkv"]
                 qkv = F.linear(n2, w, bias)
                 if qkv.shape[1] != 3 * E:
                     raise ValueError("the fused projection must have 3 * embed_dim rows")
+                if attention is None:
+                    # q, k, v are views of one [B, S, 3E] product, read in place by the kernel; its output is
+                    # [B, S, H, D] memory.  Every layer's product has the first one's layout.
+                    heads = qkv.view(B, S, 3, H, D)
+                    attention = ops._views_call(*(heads[:, :, j].transpose(1, 2) for j in range(3)),
+                                                a.view(B, S, H, D).transpose(1, 2), stream)
                 at = qkv.data_ptr()
                 attention(at, at + third, at + 2 * third, a_at)
                 w, bias = blk["o"]
