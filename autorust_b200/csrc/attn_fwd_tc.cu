@@ -94,7 +94,7 @@ constexpr uint32_t POLY_MASK = 0x8888u;  // one pair in four
 // pieces.  Piece p of row r lies at p ^ (r & 7), which keeps both sides free of bank conflicts.  RING chunks are in
 // flight, so the next step's first chunks land under this step's exponentials.  Rows and keys past the sequence end
 // are filled with zeros (the caller excludes those keys).
-// Measured, B=4 H=16 S=789 D=64 with a mask (this and the order of cta_order.cuh): 133 -> 78 us.  Copies by the two warps
+// Measured, B=4 H=16 S=789 D=64 with a mask (this and the order of cta_order.cuh): the kernel 122 -> 78 us.  Copies by the two warps
 // of the last warpgroup that have nothing else to do took 144 us, 16-byte copies from the boundary before each row with
 // a shift on reading 90 us.
 template <int RING>
@@ -191,7 +191,7 @@ __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float
       if (i >= first_out) sv[i] = 0xff800000u;
   }
   if constexpr (EDGE == 3) {
-    // leaves scaled logits in sv and c = 1
+    // (INT8 scores) leaves scaled logits in sv and c = 1
     const float* mrow = (mask != nullptr && row < N) ? mask + (size_t)row * N : nullptr;
     float mx = NEG;
 #pragma unroll
@@ -199,7 +199,7 @@ __device__ __forceinline__ void softmax_step(uint32_t (&sv)[BN], float& m, float
       const int col = col0 + i;
       // kcol: one scale per key
       const float ci = kcol != nullptr ? c * (col < N ? kcol[i] : 0.f) : c;
-      float x = MODE == TC_SAGE ? (float)(int)sv[i] * ci : __uint_as_float(sv[i]) * ci;
+      float x = (float)(int)sv[i] * ci;
       if (mrow != nullptr && col < N) x = fmaf(mrow[col], LOG2E, x);
       if (col >= N || (causal && col > row)) x = NEG;
       sv[i] = __float_as_uint(x);
@@ -692,7 +692,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // INT8 keeps its mask in this kernel, read in place: the interior step of this instantiation loses 2 % with the
         // branch taken out, and as much with the launch ticket (S=8192: 3.07 -> 3.13 ms each; 3.19 ms without both)
         const bool edge = (col0 + BN > N) || (causal && col0 + BN - 1 > q0 + t * BM) || (mask != nullptr) ||
-                          (MODE == TC_SAGE && c >= FOLD_MAX_C) || ROWS;
+                          c >= FOLD_MAX_C || ROWS;
         if (!edge)
           softmax_step<MODE, D, 0>(sv, m, l, c, j, col0, row, N, causal, tS, tO, &p_part[NPART * t]);
         else if (mask == nullptr && !ROWS)
