@@ -28,6 +28,10 @@ namespace ar {
 namespace {
 using namespace arptx;
 
+#ifdef AR_WAIT_TEST
+__device__ int g_test_skip_item = -1;  // test builds only: the item whose V tiles are never requested
+#endif
+
 constexpr int BM = 128, D = 64, KEYS = 256;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float NEG = -1e30f * LOG2E;  // the reference's finite sentinel in the log2 domain
@@ -127,7 +131,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     load_tile(sQ, &tm_q, qk_full, it.q0, it.h, it.b, 0);
     for (int x = 0; x < boxes; x++) load_tile(sK + x * (BM * D * 2), &tm_k, qk_full, x * BM, it.h / group, it.b, 1);
   };
-  auto issue_v = [&](const Item& it) {
+  auto issue_v = [&](const Item& it, int item) {
+#ifdef AR_WAIT_TEST
+    if (item == g_test_skip_item) return;
+#endif
     const int boxes = (it.keys + BM - 1) / BM;
     mbar_arrive_expect_tx(v_full, boxes * (BM * D * 2));
     for (int x = 0; x < boxes; x++) load_tile(sV + x * (BM * D * 2), &tm_v, v_full, x * BM, it.h / group, it.b, 2);
@@ -143,7 +150,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     if (!lost) {
       const Item it = item_at(blockIdx.x);
       issue_qk(it);
-      issue_v(it);
+      issue_v(it, blockIdx.x);
     }
   }
   if (warp == W_MMA) {
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
         issue_qk(it);
         qk_issued++;
         if (!mbar_wait(v_empty, (v_issued - 1) & 1, wctx, 0x61)) break;
-        issue_v(it);
+        issue_v(it, i);
         v_issued++;
       }
       if (*abort_flag) {  // let what was started land before the shared memory goes back
@@ -402,3 +409,9 @@ cudaError_t launch_attn_short(const TcArgs& a, cudaStream_t stream) {
 }
 
 }  // namespace ar
+
+#ifdef AR_WAIT_TEST
+extern "C" int ar_test_skip_short_item(int item) {
+  return cudaMemcpyToSymbol(ar::g_test_skip_item, &item, sizeof(int)) == cudaSuccess ? 0 : -1;
+}
+#endif

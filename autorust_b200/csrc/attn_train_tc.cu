@@ -44,6 +44,10 @@ namespace ar {
 namespace {
 using namespace arptx;
 
+#ifdef AR_WAIT_TEST
+__device__ int g_test_skip_step = -1;  // test builds only: the step whose streamed tiles CTA 0 never requests
+#endif
+
 constexpr int T = 128;  // rows a CTA owns: queries (dQ) or keys (dK/dV)
 constexpr int NH = 64;  // rows streamed per step: keys (dQ) or queries (dK/dV)
 constexpr float LOG2E = 1.4426950408889634f;
@@ -213,6 +217,9 @@ train_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int r = (first + n - g * per_head) * NH;
         const int sh = DKV ? h * G + g0 + g : h / G;       // head of the streamed tensors
         if (n >= SL && !mbar_wait(&slot_empty[sl], ((n / SL) - 1) & 1, wctx, 0x50)) break;
+#ifdef AR_WAIT_TEST
+        if (n == g_test_skip_step && blockIdx.x + blockIdx.y + blockIdx.z == 0) continue;
+#endif
         uint8_t* dst = ring + sl * 2 * C::STREAM_BYTES;
         mbar_arrive_expect_tx(&slot_full[sl], 2 * C::STREAM_BYTES);
         load_rows<D>(dst, DKV ? &tm_q : &tm_k, &slot_full[sl], NH, r, sh, b);
@@ -592,3 +599,9 @@ cudaError_t launch_train_convert(const float* q, const float* k, const float* v,
 }
 
 }  // namespace ar
+
+#ifdef AR_WAIT_TEST
+extern "C" int ar_test_skip_backward_step(int step) {
+  return cudaMemcpyToSymbol(ar::g_test_skip_step, &step, sizeof(int)) == cudaSuccess ? 0 : -1;
+}
+#endif

@@ -79,13 +79,80 @@ CHILD = textwrap.dedent('''
 ''')
 
 
+PRELUDE = textwrap.dedent('''
+    import sys
+    from pathlib import Path
+    sys.path.insert(0, sys.argv[1])
+    import torch
+    from autorust_b200 import _abi
+    _abi.LIB_DIR = Path(sys.argv[1]) / "autorust_b200" / "lib" / "waittest"
+    from autorust_b200 import ops
+    L = _abi.load()
+    g = torch.Generator(device="cuda").manual_seed(0)
+    bits = lambda t: t.view(torch.int16 if t.dtype == torch.bfloat16 else torch.int32)
+''')
+
+# The one-pass kernel: persistent CTAs of more items than are resident, one item's V tiles never requested.
+SHORT_CHILD = PRELUDE + textwrap.dedent('''
+    for B, H, S, items in ((2, 60, 200, 240), (8, 60, 150, 960)):
+        q, k, v = (torch.randn(B, H, S, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+        ref = ops.attn_forward("bf16", q, k, v)
+        torch.cuda.synchronize()
+        assert ops.last_status(None) == _abi.AR_OK
+        skip = items - 3  # the first tile of the second last pair, or the second of the one before
+        assert L.ar_test_skip_short_item(skip) == 0
+        ops.attn_forward("bf16", q, k, v)
+        assert ops.last_status(None) == _abi.AR_ERR_DEVICE_WAIT
+        assert ops.last_status(None) == _abi.AR_OK
+        count = torch.zeros(B * H, dtype=torch.int32, device="cuda")
+        flag = torch.zeros(B * H, dtype=torch.int32).pin_memory()
+        ops.attn_forward("bf16", q, k, v, reports=(count.data_ptr(), flag.data_ptr(), 9))
+        assert ops.last_status(None) == _abi.AR_ERR_DEVICE_WAIT
+        assert int(flag[skip // 2]) == 0 and int(count[skip // 2]) < 2, "an unfinished pair was reported"
+        assert bool(((flag == 9) == (count.cpu() == 2)).all())
+        assert L.ar_test_skip_short_item(-1) == 0
+        again = ops.attn_forward("bf16", q, k, v)
+        assert ops.last_status(None) == _abi.AR_OK
+        assert torch.equal(bits(again), bits(ref))
+    print("wait-expiry ok")
+''')
+
+# The tensor-core backward: CTA 0 of dQ and of dK/dV never requests its second step; with and without a cluster.
+BACKWARD_CHILD = PRELUDE + textwrap.dedent('''
+    for Hq, Hkv, D in ((4, 4, 64), (4, 4, 128), (8, 2, 64), (8, 1, 128), (600, 600, 64)):
+        q, k, v, d_o = (torch.randn(1, h, 300, D, device="cuda", generator=g) for h in (Hq, Hkv, Hkv, Hq))
+        o, lse = ops.train_forward(q, k, v, tensor_cores=True)
+        ref = ops.train_backward(q, k, v, o, d_o, lse, tensor_cores=True)
+        assert ops.last_status(None) == _abi.AR_OK
+        assert L.ar_test_skip_backward_step(1) == 0
+        ops.train_backward(q, k, v, o, d_o, lse, tensor_cores=True)
+        assert ops.last_status(None) == _abi.AR_ERR_DEVICE_WAIT
+        assert ops.last_status(None) == _abi.AR_OK
+        assert L.ar_test_skip_backward_step(-1) == 0
+        again = ops.train_backward(q, k, v, o, d_o, lse, tensor_cores=True)
+        assert ops.last_status(None) == _abi.AR_OK
+        for a, b in zip(ref, again):
+            assert torch.equal(bits(a), bits(b))
+    print("wait-expiry ok")
+''')
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_gpu_stays_usable(attn_lib):
+    _run_child(CHILD)
+
+
+@pytest.mark.parametrize("child", [SHORT_CHILD, BACKWARD_CHILD], ids=["short", "backward"])
+def test_the_bounded_waits_of_the_other_kernels(attn_lib, child):
+    _run_child(child)
+
+
+def _run_child(child):
     import torch
     if not torch.cuda.is_available():
         pytest.fail("needs a CUDA device")
     from autorust_b200 import build
     lib = build.build_wait_test()
     assert lib.exists()
-    proc = subprocess.run([sys.executable, "-c", CHILD, str(ROOT)], capture_output=True, text=True, timeout=600)
+    proc = subprocess.run([sys.executable, "-c", child, str(ROOT)], capture_output=True, text=True, timeout=600)
     assert proc.returncode == 0, proc.stdout + proc.stderr
     assert "wait-expiry ok" in proc.stdout
