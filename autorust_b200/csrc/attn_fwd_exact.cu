@@ -266,7 +266,7 @@ cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
     configured[dev] = true;
   }
   const CtaGrid g = cta_grid((size_t)a.S * D * 8 / (size_t)(a.Hq / a.Hkv), a.B * a.Hq, (a.S + C::BQ - 1) / C::BQ,
-                             a.causal || a.S % C::BQ != 0);
+                             a.causal ? CAUSAL_TILES : a.S % C::BQ != 0);
   kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped,
                                                      a.causal);
   return cudaGetLastError();

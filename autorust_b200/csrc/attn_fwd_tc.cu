@@ -853,7 +853,7 @@ cudaError_t launch_one(const TcArgs& a, cudaStream_t stream) {
                                : launch_grid<MODE, D, ROWS, false, ORDER_PLAIN, 1>(a, g, stream);
     }
   }
-  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + 2 * BM - 1) / (2 * BM), a.causal || a.S % (2 * BM) != 0);
+  const CtaGrid g = cta_grid(head_bytes, a.B * a.Hq, (a.S + 2 * BM - 1) / (2 * BM), a.causal ? CAUSAL_TILES : a.S % (2 * BM) != 0);
   if constexpr (MODE != TC_SAGE) {
     if (a.mask != nullptr) return launch_grid<MODE, D, ROWS, true, ORDER_ARG>(a, g, stream);
   }

@@ -658,7 +658,7 @@ TrainExactPlan train_exact_plan(int B, int Hq, int Hkv, int S, int D, int causal
     const int tiles = (S + rows - 1) / rows;
     const CtaGrid plain{dim3((unsigned)tiles, (unsigned)heads, 1), 0};
     if (rows == BT && !causal) return plain;
-    const CtaGrid g = cta_grid(bytes, heads, tiles, causal || S % rows != 0);
+    const CtaGrid g = cta_grid(bytes, heads, tiles, causal ? CAUSAL_TILES : S % rows != 0);
     if (rows != BT || g.grouped) return g;
     return tiles <= 65535 ? CtaGrid{dim3(1, (unsigned)tiles, (unsigned)heads), 1} : plain;
   };

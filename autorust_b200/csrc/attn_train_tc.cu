@@ -488,7 +488,7 @@ cudaError_t launch_bwd_tc(const TrainBwdTcArgs& a, int split, cudaStream_t strea
   // bf16 bytes that stream past a tile: Q and dO of the group's heads, or the shared K and V
   const size_t head_bytes = (size_t)a.S * D * 4 * (DKV ? group : 1) / (DKV ? 1 : group);
   cudaLaunchConfig_t cfg = {};
-  const CtaGrid g = cta_grid(head_bytes, heads, tiles, a.causal || a.S % T != 0, split);
+  const CtaGrid g = cta_grid(head_bytes, heads, tiles, a.causal ? CAUSAL_TILES : a.S % T != 0, split);
   cfg.gridDim = g.grid;
   cfg.blockDim = dim3(C::NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;

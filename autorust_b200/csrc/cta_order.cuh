@@ -20,18 +20,21 @@ namespace ar {
 // Streamed operands of the heads that are walked together: a quarter of the 126 MB L2, whose two halves may each hold
 // a copy.  Heads beyond that would stream from memory once per tile instead of once per group.
 constexpr size_t HEAD_GROUP_BYTES = (size_t)32 << 20;
+enum { EVEN_TILES, PARTIAL_TILE, CAUSAL_TILES };  // how the tiles of a launch differ in weight
 
 struct CtaGrid {
   dim3 grid;
   int grouped;
 };
-// `bytes_per_head`: what every head streams past its tiles (K/V heads shared by a GQA group count once); `split`
-// neighbouring CTAs share a tile.  Launches of more than eight rounds of CTAs stay plain: their end weighs little.  So do
-// launches whose tiles all weigh the same (no causal mask, no partial tile): the order gains them nothing, and the heads
-// that run side by side should be few (bf16 D = 128, B=1 H=8 S=8192: 226 us plain, 231 grouped; H=32 840 and 854).
-inline CtaGrid cta_grid(size_t bytes_per_head, int heads, int tiles, bool uneven, int split = 1) {
+// `bytes_per_head`: what every head streams past its tiles (K/V heads shared by a GQA group count once); `split` neighbouring CTAs
+// share a tile.  Plain stay launches of more than eight rounds of CTAs, whose end weighs little, those whose tiles all weigh
+// the same, and those of one round with a partial tile: the order gains them nothing, and the heads that run side by side
+// should be few (bf16 D = 128, B=1 H=8 S=8192: 225 us plain, 231 grouped; H=32 831 and 852).  A causal launch of one round
+// is still better off with its heavy CTAs side by side (B=1 H=32/8 S=512: 14.8 us, 15.5 plain).
+inline CtaGrid cta_grid(size_t bytes_per_head, int heads, int tiles, int uneven, int split = 1) {
   int group = 1;
-  if (uneven && tiles > 1 && (long long)tiles * heads <= 8 * 148 && tiles <= 65535) {
+  const long long ctas = (long long)tiles * heads;
+  if (uneven && tiles > 1 && (uneven == CAUSAL_TILES || ctas * split > 148) && ctas <= 8 * 148 && tiles <= 65535) {
     const size_t fit = HEAD_GROUP_BYTES / (bytes_per_head ? bytes_per_head : 1);
     for (int d = fit < (size_t)heads ? (int)fit : heads; d > 1 && group == 1; d--)  // the largest divisor that fits
       if (heads % d == 0) group = d;
