@@ -13,7 +13,7 @@ MODE_EXACT_F32, MODE_TF32, MODE_BF16, MODE_SAGE_INT8, MODE_SAGE_FP8, MODE_SAGE_I
 DTYPE_F32, DTYPE_BF16 = 0, 1
 REPLICAS_MULTICAST = -1  # n_replicas: replicas[0] is one address of an NVLink multicast object
 
-PLAN_TRAIN_BACKWARD, PLAN_TRAIN_BACKWARD_TC = 0, 1  # paths of ar_attn_plan
+PLAN_TRAIN_BACKWARD, PLAN_TRAIN_BACKWARD_TC, PLAN_EXACT_FORWARD = 0, 1, 2  # paths of ar_attn_plan
 
 AR_OK = 0
 AR_ERR_UNSUPPORTED = -1

@@ -721,6 +721,12 @@ int ar_attn_plan(int path, int64_t B, int64_t Hq, int64_t Hkv, int64_t S, int64_
     put_grid(5, p.dkv.grid);
     return AR_OK;
   }
+  if (path == AR_PLAN_EXACT_FORWARD) {
+    const ar::ExactPlan p = ar::exact_forward_plan((int)B, (int)Hq, (int)S, (int)D, causal != 0);
+    plan[0] = p.rows;
+    plan[1] = p.plain;
+    return AR_OK;
+  }
   if (path == AR_PLAN_TRAIN_BACKWARD_TC) {
     const ar::TrainTcPlan p = ar::train_tc_plan((int)B, (int)Hq, (int)Hkv, (int)S, (int)D, causal != 0);
     plan[0] = p.small_dq;

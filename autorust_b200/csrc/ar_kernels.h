@@ -96,6 +96,11 @@ struct ExactArgs {
   int causal;
   float* lse = nullptr;  // [B*Hq, S]: when set, the rows' log-sum-exp is written as well (training forward)
 };
+// The form that such a call takes: rows of a CTA's tile; plain: 64 rows, one group, several CTAs per SM.
+struct ExactPlan {
+  int rows, plain;
+};
+ExactPlan exact_forward_plan(int B, int Hq, int S, int D, int causal);
 cudaError_t launch_attn_exact(const ExactArgs& a, cudaStream_t stream);
 
 // Training path (attn_train.cu): gradients of the exact f32 forward, from its saved log-sum-exp.

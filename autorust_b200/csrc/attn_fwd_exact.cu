@@ -41,11 +41,13 @@ struct ExactCfg {
   static_assert(GT * (RQ * OD * 4 + 2 * RQ) <= GROUP_FLOATS, "a group's result passes through its own tiles");
 };
 
-template <int D, int RQ, int TX, int TY, int GROUPS>
+// (CAUSAL is a template parameter so that the other kernel carries nothing of what a causal mask needs: as an argument it
+// cost that one 1 to 2 %.)
+template <int D, int RQ, int TX, int TY, int GROUPS, bool CAUSAL>
 __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     attn_fwd_exact_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                           float* __restrict__ O, const float* __restrict__ M, float* __restrict__ LSE, int N, int Hq,
-                          int Hkv, int grouped, int causal) {
+                          int Hkv, int grouped) {
   using C = ExactCfg<D, RQ, TX, TY, GROUPS>;
   constexpr int JK = C::JK, OD = C::OD, D4 = D / 4;
   extern __shared__ __align__(16) float smem_f[];
@@ -57,7 +59,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
   float* sP = sV + BK * D;
   const int bh = cta_head(grouped);
   int tile = cta_tile(grouped);
-  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
+  if (CAUSAL) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * C::BQ;
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
   };
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(C::GT) : "memory"); };
 
-  const int kend = causal ? min(N, q0 + C::BQ) : N;
+  const int kend = CAUSAL ? min(N, q0 + C::BQ) : N;
   const int tiles = (kend + BK - 1) / BK;
   for (int i = tid; i < C::BQ * D4; i += C::THREADS) {
     const int r = i / D4, c = i % D4;
@@ -128,19 +130,22 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     group_sync();  // the group is done with this K tile
     load_rows(sK, C::LDQ, kb, min(k0 + GROUPS * BK, N));  // (past the last tile: zeros, nothing is read)
     // Excluded keys get the finite sentinel, which a row whose visible keys all carry -1e30 counts along.  Under a causal
-    // mask a row counts them up to the end of the 64 keys its diagonal lies in; a tile that reaches further gives them
-    // no weight, so that such a row has the same value whatever tile height its call takes.
-    const bool bounds = k0 + BK > N || (causal && k0 + BK - 1 > q0);
+    // mask a row counts them up to the end of the 64 keys its diagonal lies in; a CTA whose rows reach over that end gives
+    // them no weight, so that such a row has the same value whatever tile height its call takes.
+    const bool past = BK % C::BQ != 0 && CAUSAL && k0 > q0;
+    const bool bounds = k0 + BK > N || (CAUSAL && k0 + BK - 1 > q0);
 #pragma unroll
     for (int i = 0; i < RQ; i++) {
       const int row = q0 + ty + TY * i;
+      // (tiles of 128 rows reach over the end by whole halves of their rows)
+      const float out = past && (C::BQ == 2 * BK ? TY * i < BK : row < k0) ? -INFINITY : NEG;
       float mx = m[i];
 #pragma unroll
       for (int jj = 0; jj < JK; jj++) {
         const int key = k0 + tx + TX * jj;
         float x = s[i][jj] * scale;
         if (M != nullptr && row < N && key < N) x += M[(size_t)row * N + key];
-        if (bounds && (key >= N || (causal && key > row))) x = causal && k0 > row ? -INFINITY : NEG;
+        if (bounds && (key >= N || (CAUSAL && key > row))) x = out;
         s[i][jj] = x;
         mx = fmaxf(mx, x);
       }
@@ -255,35 +260,38 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
 template <int D, int RQ, int TX, int TY, int GROUPS>
 cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
   using C = ExactCfg<D, RQ, TX, TY, GROUPS>;
-  auto kern = attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS>;
-  static bool configured[64] = {};
+  auto kern = a.causal ? attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, true> : attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, false>;
+  static bool configured[2][64] = {};
+  const int form = a.causal ? 1 : 0;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 64 && !configured[dev]) {
+  if (dev < 64 && !configured[form][dev]) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    configured[dev] = true;
+    configured[form][dev] = true;
   }
   const CtaGrid g = cta_grid((size_t)a.S * D * 8 / (size_t)(a.Hq / a.Hkv), a.B * a.Hq, (a.S + C::BQ - 1) / C::BQ,
                              a.causal ? CAUSAL_TILES : a.S % C::BQ != 0);
-  kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped,
-                                                     a.causal);
+  kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped);
   return cudaGetLastError();
 }
 
-// D = 64 without a causal mask, for calls whose tiles of 128 rows would leave a last round half empty: 4 x 4 scores per
-// thread on 64 rows, plain loads, two CTAs per SM that fill each other's waits.
-constexpr int PAIR_BQ = 64;
-constexpr int PAIR_SMEM = (PAIR_BQ * 68 + BK * 68 + BK * 64 + PAIR_BQ * (BK + 4)) * 4;
-__global__ void __launch_bounds__(256) attn_fwd_exact_pair_kernel(const float* __restrict__ Q, const float* __restrict__ K,
+// The plain form: 4 x 4 scores per thread on 64 rows, one group, plain loads; at D = 64 three CTAs of an SM fill each other's
+// waits.  It needs no key tiles to deal out, so it ends first for short sequences of many heads, and where larger tiles
+// would leave a last round half empty.
+constexpr int PLAIN_BQ = 64;
+template <int D>
+constexpr int PLAIN_SMEM = (PLAIN_BQ * (D + 4) + BK * (D + 4) + BK * D + PLAIN_BQ * (BK + 4)) * 4;
+template <int D>
+__global__ void __launch_bounds__(256) attn_fwd_exact_plain_kernel(const float* __restrict__ Q, const float* __restrict__ K,
                                                              const float* __restrict__ V, float* __restrict__ O,
                                                              const float* __restrict__ M, float* __restrict__ LSE,
                                                              int N, int Hq, int Hkv, int causal) {
-  constexpr int D = 64, LDQ = D + 4, LDP = BK + 4;  // padded rows (floats)
+  constexpr int LDQ = D + 4, LDP = BK + 4;  // padded rows (floats)
   extern __shared__ __align__(16) float smem_f[];
   float* sQ = smem_f;
-  float* sK = sQ + PAIR_BQ * LDQ;
+  float* sK = sQ + PLAIN_BQ * LDQ;
   float* sV = sK + BK * LDQ;
   float* sP = sV + BK * D;
   const int tid = threadIdx.x;
@@ -293,7 +301,7 @@ __global__ void __launch_bounds__(256) attn_fwd_exact_pair_kernel(const float* _
   const int b = bh / Hq;
   const int h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
-  const int q0 = blockIdx.x * PAIR_BQ;
+  const int q0 = blockIdx.x * PLAIN_BQ;
   const float* qb = Q + (size_t)bh * N * D;
   const float* kb = K + (size_t)kvbh * N * D;
   const float* vb = V + (size_t)kvbh * N * D;
@@ -301,7 +309,7 @@ __global__ void __launch_bounds__(256) attn_fwd_exact_pair_kernel(const float* _
   constexpr int D4 = D / 4;
   constexpr int OD = D / 64;  // float4 output groups per thread
 
-  for (int i = tid; i < PAIR_BQ * D4; i += 256) {
+  for (int i = tid; i < PLAIN_BQ * D4; i += 256) {
     const int r = i / D4, c = i - r * D4;
     float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (q0 + r < N) v4 = *(const float4*)(qb + (size_t)(q0 + r) * D + c * 4);
@@ -316,7 +324,7 @@ __global__ void __launch_bounds__(256) attn_fwd_exact_pair_kernel(const float* _
 #pragma unroll
     for (int dd = 0; dd < OD; dd++) o[i][dd] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  const int kend = causal ? min(N, q0 + PAIR_BQ) : N;
+  const int kend = causal ? min(N, q0 + PLAIN_BQ) : N;
   for (int k0 = 0; k0 < kend; k0 += BK) {
     __syncthreads();  // previous tile fully consumed (and sQ visible on the first pass)
     for (int i = tid; i < BK * D4; i += 256) {
@@ -427,56 +435,98 @@ __global__ void __launch_bounds__(256) attn_fwd_exact_pair_kernel(const float* _
   }
 }
 
-cudaError_t launch_exact_pair(const ExactArgs& a, cudaStream_t stream) {
+template <int D>
+cudaError_t launch_exact_plain(const ExactArgs& a, cudaStream_t stream) {
+  auto kern = attn_fwd_exact_plain_kernel<D>;
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(attn_fwd_exact_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAIN_SMEM<D>);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  attn_fwd_exact_pair_kernel<<<dim3((a.S + PAIR_BQ - 1) / PAIR_BQ, a.B * a.Hq, 1), 256, PAIR_SMEM, stream>>>(
+  kern<<<dim3((a.S + PLAIN_BQ - 1) / PLAIN_BQ, a.B * a.Hq, 1), 256, PLAIN_SMEM<D>, stream>>>(
       a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, a.causal);
   return cudaGetLastError();
 }
 
-// What a launch with tiles of `rows` rows costs, in rows of the large form: rounds of one CTA per SM -- under a causal
-// mask the average tile sees half of the keys and the rounds overlap, but none ends before its heaviest tile -- each as
-// long as its rows plus the part of a CTA that does not depend on them (loads, softmax, combination: about 8 rows).
-double launch_cost(const ExactArgs& a, int rows) {
-  const double ctas = (double)((a.S + rows - 1) / rows) * a.B * a.Hq;
-  const double rounds = a.causal ? fmax(1.0, 0.55 * ctas / 148.0) : ceil(ctas / 148.0);
-  return rounds * (rows + 8);
+// What a CTA of each form costs, in microseconds: cta + step * (its groups' turns) + tile * (its key tiles of 64), and
+// `launch` once per launch.  Fitted to the device times of every form at 302 shapes (D = 64 and 128, S = 50 to 2048, 2 to
+// 200 heads, causal and not); without a causal mask the fits are within 3 % in the mean, 11 % at worst.
+struct Form {
+  int rows, groups;
+  double launch, cta, step, tile;
+};
+constexpr Form FORMS_64[] = {{8, 4, 1.2, 1.9, 1.45, 0.77}, {12, 4, 1.2, 2.4, 1.8, 0.88}, {16, 4, 1.2, 2.5, 2.5, 0.92},
+                             {20, 4, 1.2, 2.8, 3.05, 1.0}, {24, 4, 1.5, 3.2, 3.5, 1.1},  {32, 4, 1.7, 3.6, 4.35, 1.25},
+                             {64, 2, 1.5, 2.1, 3.0, 3.1},  {128, 2, 2.3, 2.2, 5.4, 5.3}};
+constexpr Form FORMS_128[] = {{8, 2, 1.2, 2.3, 3.3, 0.6},   {12, 2, 1.2, 2.5, 4.45, 0.42}, {16, 2, 1.3, 2.6, 5.5, 0.36},
+                              {20, 2, 1.7, 3.05, 6.9, 0.2}, {24, 2, 1.9, 3.5, 7.1, 0.37},  {32, 2, 2.3, 3.6, 9.4, 0.2},
+                              {64, 2, 1.6, 3.1, 4.3, 5.8}};
+
+// Launch time of `ctas` CTAs of a form on 148 SMs.  Without a causal mask (or with one key tile) all CTAs weigh the same:
+// rounds.  Under a causal mask, heaviest first: no launch ends before its heaviest CTA, nor before the work is done, plus
+// a part of a mean CTA for the uneven end.
+double form_time(const Form& f, double tiles, double heads, int key_tiles, bool uneven) {
+  const double ctas = tiles * heads;
+  const int turns = (key_tiles + f.groups - 1) / f.groups;
+  const double heaviest = f.cta + f.step * turns + f.tile * key_tiles;
+  if (!uneven) return f.launch + ceil(ctas / 148.0) * heaviest;
+  const double full = key_tiles / f.groups, part = key_tiles % f.groups;  // mean turns of 1 .. key_tiles tiles
+  const double mean_turns = (f.groups * full * (full + 1) / 2 + part * (full + 1)) / key_tiles;
+  const double mean = f.cta + f.step * mean_turns + f.tile * 0.5 * (key_tiles + (f.rows > BK ? f.rows / BK : 1));
+  const double first = heaviest + (ctas > 148.0 ? f.cta : 0.0), work = ctas / 148.0 * mean + 0.3 * mean;
+  return f.launch + (first > work ? first : work);
+}
+// The same for the plain form; at D = 64 an SM holds three of its CTAs (5.9 us per key tile for one, 9.2 for two, 13 for
+// three).  Its tiles run in the order of their index, a causal launch ends on heavy ones.
+double plain_time(double tiles, double heads, int key_tiles, bool uneven, int D) {
+  const double ctas = tiles * heads;
+  if (D == 128) return form_time({PLAIN_BQ, 1, 1.0, 2.2, 0.0, 9.0}, tiles, heads, key_tiles, uneven);
+  auto together = [](double k, int n) { return n == 1 ? 2.7 + 5.9 * k : n == 2 ? 3.2 + 9.2 * k : 4.0 + 13.0 * k; };
+  if (!uneven) {
+    const double full = floor(ctas / 444.0);
+    const int rest = (int)ceil((ctas - 444.0 * full) / 148.0);
+    return 0.3 + full * together(key_tiles, 3) + (rest ? together(key_tiles, rest) : 0.0);
+  }
+  const int n = ctas <= 148.0 ? 1 : ctas <= 296.0 ? 2 : 3;
+  const double heaviest = together(key_tiles, n), work = ctas / 148.0 * together(0.5 * (key_tiles + 1), n) / n + 0.75 * heaviest / n;
+  return 0.3 + (heaviest > work ? heaviest : work);
 }
 
 }  // namespace
 
-cudaError_t launch_attn_exact(const ExactArgs& a, cudaStream_t stream) {
-  // The form that ends first.  Weights per row of a round, measured at S = 197 to 1024: 1 for the large form, 1.6 for the
-  // tiles of 8 to 32 rows that spread a small call over the chip, at D = 64 also 1.11 for 4 x 8 blocks on 64 rows, and
-  // for the 64-row form with two CTAs per SM 105 rows alone, 150 in pairs, 45.5 per half round beyond, the last one included
-  // (B=6 Hq=4 S=848: 189 us against 199 with 4 x 8 blocks; B=2 H=8 S=1024: 152 against 135 in the large form).
-  const int large = a.D == 64 ? 128 : 64;
-  int rows = large;
-  double cost = launch_cost(a, large);
-  auto offer = [&](int r, double c) {
-    if (c < cost) {
-      rows = r;
-      cost = c;
+// The form that ends first by these estimates.  Over the measured shapes the choice lies 0.3 % on average above the best
+// form and at most 2 % above the plain one, which used to serve every call.
+ExactPlan exact_forward_plan(int B, int Hq, int S, int D, int causal) {
+  const double heads = (double)B * Hq;
+  const int key_tiles = (S + BK - 1) / BK;
+  const bool uneven = causal && key_tiles > 1;
+  ExactPlan p{PLAIN_BQ, 1};
+  double least = plain_time((S + PLAIN_BQ - 1) / PLAIN_BQ, heads, key_tiles, uneven, D);
+  auto offer = [&](const Form& f) {
+    const double t = form_time(f, (S + f.rows - 1) / f.rows, heads, key_tiles, uneven);
+    if (t < least) {
+      least = t;
+      p = ExactPlan{f.rows, 0};
     }
   };
-  for (int r : {8, 12, 16, 20, 24, 32}) offer(r, 1.6 * launch_cost(a, r));
-  if (a.D == 64) offer(64, 1.11 * launch_cost(a, 64));
-  if (a.D == 64 && !a.causal) {
-    const double ctas = (double)((a.S + 63) / 64) * a.B * a.Hq;
-    offer(-64, ctas <= 148 ? 105.0 : ctas <= 296 ? 150.0 : 45.5 * 2.0 * ctas / 148.0);
-  }
-  if (rows == -64) return launch_exact_pair(a, stream);
+  if (D == 64)
+    for (const Form& f : FORMS_64) offer(f);
+  else
+    for (const Form& f : FORMS_128) offer(f);
+  return p;
+}
+
+cudaError_t launch_attn_exact(const ExactArgs& a, cudaStream_t stream) {
+  if (a.D != 64 && a.D != 128) return cudaErrorInvalidValue;
+  const ExactPlan p = exact_forward_plan(a.B, a.Hq, a.S, a.D, a.causal);
+  if (p.plain) return a.D == 64 ? launch_exact_plain<64>(a, stream) : launch_exact_plain<128>(a, stream);
 #define AR_EXACT(D_, G_)                                         \
   if (a.D == D_) {                                               \
-    switch (rows) {                                              \
+    switch (p.rows) {                                            \
       case 8: return launch_exact<D_, 2, 16, 4, G_>(a, stream);  \
       case 12: return launch_exact<D_, 3, 16, 4, G_>(a, stream); \
       case 16: return launch_exact<D_, 4, 16, 4, G_>(a, stream); \

@@ -291,8 +291,9 @@ int ar_add_layernorm(const void* x, const void* residual, const void* gamma, con
 /* Which form of its kernels a call of these sizes takes, for tests and profiles: fills plan[0 .. 7] and returns AR_OK; no
  * device is touched, nothing is launched.
  *   AR_PLAN_TRAIN_BACKWARD     rows of a tile of dQ and of dK/dV (64 or 128), the grid of dQ, the grid of dK/dV
- *   AR_PLAN_TRAIN_BACKWARD_TC  1 where dQ (dK/dV) takes two CTAs per SM, CTAs that share a key tile's query heads */
-enum ar_attn_plan_path { AR_PLAN_TRAIN_BACKWARD = 0, AR_PLAN_TRAIN_BACKWARD_TC = 1 };
+ *   AR_PLAN_TRAIN_BACKWARD_TC  1 where dQ (dK/dV) takes two CTAs per SM, CTAs that share a key tile's query heads
+ *   AR_PLAN_EXACT_FORWARD      rows of a tile, 1 for the plain form (the exact f32 forward, training included) */
+enum ar_attn_plan_path { AR_PLAN_TRAIN_BACKWARD = 0, AR_PLAN_TRAIN_BACKWARD_TC = 1, AR_PLAN_EXACT_FORWARD = 2 };
 int ar_attn_plan(int path, int64_t B, int64_t Hq, int64_t Hkv, int64_t S, int64_t D, int causal, int32_t* plan);
 
 /* Total kernel launches issued by this library since load (all kernels, prologue included). */

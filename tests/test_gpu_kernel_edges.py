@@ -7,7 +7,8 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from helpers import cosine, from_dev_bf16, max_abs, normal_qkv, sawtooth_mask, to_dev, to_dev_bf16
+from helpers import (EXACT_FORWARD_SHAPES, TRAINING_SHAPES, TRAINING_SHAPES_LARGE, cosine, from_dev_bf16, max_abs,
+                     normal_qkv, sawtooth_mask, to_dev, to_dev_bf16)
 
 pytestmark = pytest.mark.gpu
 
@@ -126,15 +127,14 @@ def test_mask_ring(ops, oracle_lib, mode, d, n, causal):
     assert ops.last_status(None) == 0
 
 
-@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 12, 12, 197), (1, 2, 2, 64), (1, 2, 2, 65), (2, 74, 74, 130),
-                                        (1, 148, 74, 257), (1, 2, 2, 1100)])
+@pytest.mark.parametrize("b,hq,hkv,n", EXACT_FORWARD_SHAPES)
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 def test_exact_tiles(ops, oracle_lib, b, hq, hkv, n, d, causal):
-    """Calls on both sides of the tile rule (16-row tiles for few rows, 128- or 64-row ones for many), the key groups
-    with more groups than tiles; 1e-5 of the largest value as for the exact mode elsewhere."""
+    """Every form of the tile rule (tests/test_plans.py), the key groups with more groups than tiles, with a mask at some
+    lengths; 1e-5 of the largest value as for the exact mode elsewhere."""
     q, k, v = normal_qkv(n, b, hq, hkv, n, d)
-    mask = sawtooth_mask(n) if n == 65 else None
+    mask = sawtooth_mask(n) if n in (17, 50, 65, 197, 257) else None
     got = ops.attn_forward("exact", *map(to_dev, (q, k, v)), None if mask is None else to_dev(mask), causal).cpu().numpy()
     want = oracle_lib.flash(0, q, k, v, mask, causal)
     assert np.all(np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1.0))
@@ -166,13 +166,12 @@ def test_exact_causal_rows_without_visible_keys(ops, n, d):
 
 
 @pytest.mark.parametrize("tc", [False, True])
-@pytest.mark.parametrize("b,hq,hkv,n", [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321), (1, 7, 1, 70),
-                                        (2, 8, 1, 200),
-                                        (5, 30, 30, 130)])
+@pytest.mark.parametrize("b,hq,hkv,n", TRAINING_SHAPES)
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 def test_training_steps(ops, oracle_lib, tc, b, hq, hkv, n, d, causal):
-    """Fewer steps than stages, ragged tiles, several query heads per K/V head, with and without a mask.  Exact: 2e-5 of
+    """Every form of both backwards without a causal mask (tests/test_plans.py), fewer steps than stages, ragged tiles,
+    several query heads per K/V head, with and without a mask.  Exact: 2e-5 of
     the largest entry, as the training tests hold it.  bf16 operands: 2e-2 of it (dP is a sum of D products of operands
     rounded to 2^-9, off by 2^-9 sqrt(2 D / 3) = 0.018 in the root mean square at D = 128, and a row of few visible keys
     passes that on to its dQ undamped), and a cosine of 0.9995."""
@@ -180,7 +179,7 @@ def test_training_steps(ops, oracle_lib, tc, b, hq, hkv, n, d, causal):
     rng = np.random.default_rng(n)
     q, k, v = normal_qkv(n, b, hq, hkv, n, d)
     d_o = rng.standard_normal(q.shape, dtype=np.float32)
-    mask = sawtooth_mask(n) if n == 129 else None
+    mask = sawtooth_mask(n) if n in (65, 127, 129) else None
     want = dict(zip(("o", "lse", "dq", "dk", "dv"), oracle_lib.attn_train(q, k, v, d_o, mask, causal)))
     tq, tk, tv, tdo = map(to_dev, (q, k, v, d_o))
     tm = None if mask is None else to_dev(mask)
@@ -195,4 +194,71 @@ def test_training_steps(ops, oracle_lib, tc, b, hq, hkv, n, d, causal):
             assert cosine(got.cpu().numpy(), w) >= 0.9995, name
     for x, y in zip(grads, again):  # no atomics: two launches give the same bits
         assert torch.equal(x, y)
+    assert ops.last_status(None) == 0
+
+
+@pytest.mark.parametrize("tc", [False, True])
+@pytest.mark.parametrize("b,hq,hkv,n", TRAINING_SHAPES_LARGE)
+@pytest.mark.parametrize("masked", [False, True])
+def test_training_steps_of_many_causal_heads(ops, tc, b, hq, hkv, n, masked):
+    """The forms that only large causal calls take (128-row exact tiles, two tensor-core CTAs per SM), against float64
+    autograd on the GPU; the bounds of test_training_steps."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v, d_o = (torch.randn(b, h, n, 64, device="cuda", generator=g) for h in (hq, hkv, hkv, hq))
+    mask = torch.randn(n, n, device="cuda", generator=g) if masked else None
+    o, lse = ops.train_forward(q, k, v, mask, True, tensor_cores=tc)
+    got = ops.train_backward(q, k, v, o, d_o, lse, mask, True, tensor_cores=tc)
+    qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
+    s = qd @ kd.transpose(-1, -2) / 8.0
+    if masked:
+        s = s + mask.double()
+    s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    (torch.softmax(s, -1) @ vd).backward(d_o.double())
+    for name, x, w in zip(("dq", "dk", "dv"), got, (qd.grad, kd.grad, vd.grad)):
+        bound = (2e-2 if tc else 2e-5) * max(1.0, w.abs().max().item())
+        assert (x.double() - w).abs().max().item() <= bound, name
+        assert torch.nn.functional.cosine_similarity(x.double().flatten(), w.flatten(), dim=0).item() >= 0.9995, name
+    assert ops.last_status(None) == 0
+
+
+@pytest.mark.parametrize("mode,b,hq,hkv,n", [("bf16", 1, 16, 16, 8200), ("sage", 1, 32, 32, 4100), ("sage_fp8", 1, 32, 32, 5000)])
+def test_heads_in_several_groups(ops, mode, b, hq, hkv, n):
+    """K and V of more heads than are walked together (32 MB), and a partial last tile: a grid of several groups.  Each head
+    alone, in a plain grid, gives the same bits; bf16 through strided views as well."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(b, h, n, 128, device="cuda", generator=g).to(torch.bfloat16) for h in (hq, hkv, hkv))
+    for causal in (False, True):
+        out = ops.attn_forward(mode, q, k, v, None, causal)
+        for h in (0, 1, hq // 2, hq - 1):
+            kv = h // (hq // hkv)
+            one = ops.attn_forward(mode, q[:, h:h + 1].contiguous(), *(t[:, kv:kv + 1].contiguous() for t in (k, v)), None, causal)
+            assert torch.equal(out[:, h:h + 1], one), (causal, h)
+        if mode == "bf16":
+            views = [t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v)]
+            assert torch.equal(out, ops.attn_forward_views(*views, None, causal))
+    assert ops.last_status(None) == 0
+
+
+@pytest.mark.parametrize("n,d", [(200, 64), (700, 128)])
+def test_captured_call_between_ticketed_ones(ops, n, d):
+    """Calls outside of a capture mark the shared status word with a ticket, a captured one clears it: replays between
+    such calls give the bits of the eager call and leave nothing behind."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(2, 80, n, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    want = ops.attn_forward("bf16", q, k, v)
+    out = torch.empty_like(q)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        ops.attn_forward("bf16", q, k, v, out=out)
+    for _ in range(3):
+        out.zero_()
+        assert torch.equal(ops.attn_forward("bf16", q, k, v), want)
+        graph.replay()
+        assert torch.equal(ops.attn_forward("bf16", q, k, v), want)
+        assert torch.equal(out, want)
     assert ops.last_status(None) == 0

@@ -5,6 +5,7 @@ from __future__ import annotations
 import pytest
 
 from autorust_b200 import _abi
+from helpers import EXACT_FORWARD_SHAPES, TRAINING_SHAPES, TRAINING_SHAPES_LARGE
 
 
 @pytest.fixture(scope="module", autouse=True)
@@ -51,6 +52,35 @@ def test_grids_are_grouped_only_where_tiles_differ():
     assert (heads_of_a_group * groups, tiles) == (148, 2) and heads_of_a_group > 1
     heads_of_a_group, tiles, groups = grid(1, 20, 20, 512, 64, True)
     assert (heads_of_a_group * groups, tiles) == (20, 8) and heads_of_a_group > 1
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("d,forms", [(64, {8, 12, 16, 20, 24, 32, 64, 128}), (128, {8, 12, 16, 20, 24, 32, 64})])
+def test_the_numerics_tests_reach_every_form_of_the_exact_forward(d, forms, causal):
+    plans = [_abi.plan(_abi.PLAN_EXACT_FORWARD, b, hq, hkv, n, d, causal)[:2] for b, hq, hkv, n in EXACT_FORWARD_SHAPES]
+    assert {rows for rows, plain in plans if not plain} == forms
+    assert [64, 1] in plans
+
+
+def test_the_numerics_tests_reach_every_form_of_the_backwards():
+    exact = lambda shapes, causal: {tuple(_abi.plan(_abi.PLAN_TRAIN_BACKWARD, *s, 64, causal)[:2]) for s in shapes}
+    assert exact(TRAINING_SHAPES, False) == {(64, 64), (64, 128), (128, 64), (128, 128)}
+    assert (128, 128) in exact(TRAINING_SHAPES_LARGE, True) and (64, 64) in exact(TRAINING_SHAPES, True)
+    for causal in (False, True):
+        fast = [_abi.plan(_abi.PLAN_TRAIN_BACKWARD_TC, *s, 64, causal)[:3] for s in TRAINING_SHAPES + TRAINING_SHAPES_LARGE]
+        assert [0, 0, 1] in fast and [1, 1, 1] in fast and any(split > 1 for _, _, split in fast)
+        fast = [_abi.plan(_abi.PLAN_TRAIN_BACKWARD_TC, *s, 128, causal)[:3] for s in TRAINING_SHAPES]
+        assert [0, 0, 1] in fast and any(split > 1 for _, _, split in fast)
+
+
+def test_exact_forward_form_of_many_short_and_many_long_heads():
+    """The forms that were measured ahead: the plain one for many heads of one key tile (48 heads of S=50, causal: 8.6 us
+    against 14.2 with 12-row tiles), 128-row tiles for large calls, tiles of 16 to 24 rows for one image's layer."""
+    form = lambda *sizes: _abi.plan(_abi.PLAN_EXACT_FORWARD, *sizes)[:2]
+    for d in (64, 128):
+        assert form(1, 200, 200, 50, d, True) == [64, 1]
+    assert form(8, 32, 32, 2048, 64, False) == [128, 0]
+    assert form(1, 12, 12, 197, 64, False)[0] in (16, 20, 24)
 
 
 def test_exact_backward_forms_of_causal_calls():
