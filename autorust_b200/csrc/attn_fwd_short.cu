@@ -16,10 +16,10 @@
 //   TMEM (256 columns): S [0, 256); P (bf16, two per column) overwrites [0, 128) as S is read; O takes [128, 192) once
 //   all of S has been read.
 //
-// Bound: latency.  Measured, B=64 H=12 S=197 on strided views: 45.8 us in the form with two key steps that this replaces, 29.5 us
-// here against 11.8 us for its 77 MB; the MUFU unit and the issue slots are about a third busy.  An item's chain is 7700
-// cycles: maximum 1070, exponentials 2800 (a quarter of them on the FMA pipe), P V with its hand-overs 1350, from O
-// read to the next scores 2300, and two CTAs per SM are what TMEM holds.
+// Bound: latency.  Measured, B=64 H=12 S=197 on strided views: 42.5 us in the key loop's one-tile form, 31.4 us here against
+// 11.8 us for its 77 MB (29.4 with the cubic in every whole chunk: what the accuracy costs); the MUFU unit and the issue
+// slots are about a third busy.  An item's chain is about 8000 cycles: maximum 1070, exponentials 3100, P V with its
+// hand-overs 1350, from O read to the next scores 2300, and two CTAs per SM are what TMEM holds.
 #include "ar_kernels.h"
 #include "ar_ptx.cuh"
 #include "softmax_math.cuh"
