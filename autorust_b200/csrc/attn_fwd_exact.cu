@@ -41,13 +41,14 @@ struct ExactCfg {
   static_assert(GT * (RQ * OD * 4 + 2 * RQ) <= GROUP_FLOATS, "a group's result passes through its own tiles");
 };
 
-// (CAUSAL is a template parameter so that the other kernel carries nothing of what a causal mask needs: as an argument it
-// cost that one 1 to 2 %.)
-template <int D, int RQ, int TX, int TY, int GROUPS, bool CAUSAL>
+// CAUSAL: the mask is known when the kernel is compiled (NO, YES) for the forms whose tiles reach over the end of a row's 64
+// keys (see `past`): what that takes cost the 128-row form 2 to 5 % without a mask.  The others are told at run time.
+enum { CAUSAL_NO, CAUSAL_YES, CAUSAL_ARG };
+template <int D, int RQ, int TX, int TY, int GROUPS, int CAUSAL>
 __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     attn_fwd_exact_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                           float* __restrict__ O, const float* __restrict__ M, float* __restrict__ LSE, int N, int Hq,
-                          int Hkv, int grouped) {
+                          int Hkv, int grouped, int causal_arg) {
   using C = ExactCfg<D, RQ, TX, TY, GROUPS>;
   constexpr int JK = C::JK, OD = C::OD, D4 = D / 4;
   extern __shared__ __align__(16) float smem_f[];
@@ -59,7 +60,8 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
   float* sP = sV + BK * D;
   const int bh = cta_head(grouped);
   int tile = cta_tile(grouped);
-  if (CAUSAL) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
+  const bool causal = CAUSAL == CAUSAL_ARG ? causal_arg != 0 : CAUSAL == CAUSAL_YES;
+  if (causal) tile = cta_tiles(grouped) - 1 - tile;  // the last query tile sees the most keys
   const int b = bh / Hq, h = bh - b * Hq;
   const int kvbh = b * Hkv + h / (Hq / Hkv);
   const int q0 = tile * C::BQ;
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
   };
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(C::GT) : "memory"); };
 
-  const int kend = CAUSAL ? min(N, q0 + C::BQ) : N;
+  const int kend = causal ? min(N, q0 + C::BQ) : N;
   const int tiles = (kend + BK - 1) / BK;
   for (int i = tid; i < C::BQ * D4; i += C::THREADS) {
     const int r = i / D4, c = i % D4;
@@ -132,8 +134,8 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
     // Excluded keys get the finite sentinel, which a row whose visible keys all carry -1e30 counts along.  Under a causal
     // mask a row counts them up to the end of the 64 keys its diagonal lies in; a CTA whose rows reach over that end gives
     // them no weight, so that such a row has the same value whatever tile height its call takes.
-    const bool past = BK % C::BQ != 0 && CAUSAL && k0 > q0;
-    const bool bounds = k0 + BK > N || (CAUSAL && k0 + BK - 1 > q0);
+    const bool past = BK % C::BQ != 0 && causal && k0 > q0;
+    const bool bounds = k0 + BK > N || (causal && k0 + BK - 1 > q0);
 #pragma unroll
     for (int i = 0; i < RQ; i++) {
       const int row = q0 + ty + TY * i;
@@ -145,7 +147,7 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
         const int key = k0 + tx + TX * jj;
         float x = s[i][jj] * scale;
         if (M != nullptr && row < N && key < N) x += M[(size_t)row * N + key];
-        if (bounds && (key >= N || (CAUSAL && key > row))) x = out;
+        if (bounds && (key >= N || (causal && key > row))) x = out;
         s[i][jj] = x;
         mx = fmaxf(mx, x);
       }
@@ -260,7 +262,8 @@ __global__ void __launch_bounds__(TX* TY* GROUPS, 1)
 template <int D, int RQ, int TX, int TY, int GROUPS>
 cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
   using C = ExactCfg<D, RQ, TX, TY, GROUPS>;
-  auto kern = a.causal ? attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, true> : attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, false>;
+  auto kern = attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, BK % C::BQ == 0 ? CAUSAL_ARG : CAUSAL_NO>;
+  if (BK % C::BQ != 0 && a.causal) kern = attn_fwd_exact_kernel<D, RQ, TX, TY, GROUPS, BK % C::BQ == 0 ? CAUSAL_ARG : CAUSAL_YES>;
   static bool configured[2][64] = {};
   const int form = a.causal ? 1 : 0;
   int dev = 0;
@@ -273,7 +276,8 @@ cudaError_t launch_exact(const ExactArgs& a, cudaStream_t stream) {
   }
   const CtaGrid g = cta_grid((size_t)a.S * D * 8 / (size_t)(a.Hq / a.Hkv), a.B * a.Hq, (a.S + C::BQ - 1) / C::BQ,
                              a.causal ? CAUSAL_TILES : a.S % C::BQ != 0);
-  kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped);
+  kern<<<g.grid, C::THREADS, C::SMEM_BYTES, stream>>>(a.q, a.k, a.v, a.out, a.mask, a.lse, a.S, a.Hq, a.Hkv, g.grouped,
+                                                     a.causal);
   return cudaGetLastError();
 }
 

@@ -589,11 +589,12 @@ cudaError_t configure() {
 
 // The 128-row tiles do their rows about 5 % faster than the 64-row ones, of which an SM holds two: the form whose
 // rounds come to fewer rows per SM (B=6 Hq=4 S=848: dQ 2 x 128 against 3 x 64, a step 7 % slower in the wide form).
-// Under a causal mask they want more than four rounds: their heaviest tiles, twice as long, end the launch (96 heads of
+// Under a causal mask, where rounds overlap, it is the rows altogether that count (352 heads of S=405, of which 128-row tiles
+// walk 512: 1700 us the training step, 1625 with 64 rows), and they want more than four rounds: their heaviest tiles, twice as long, end the launch (96 heads of
 // S=700: 764 us against 702 with 64 rows; 96 of S=848, 4.5 rounds: 1110 against 1230).
 bool worth_it(int S, int heads, int causal) {
   const long long w = (long long)((S + 127) / 128) * heads, n = (long long)((S + 63) / 64) * heads;
-  if (causal) return w > 4 * 148 + 74;
+  if (causal) return w > 4 * 148 + 74 && w * 128 * 20 <= n * 64 * 21;
   return ((w + 147) / 148) * 128 * 20 <= ((n + 147) / 148) * 64 * 21;
 }
 }  // namespace wide

@@ -97,4 +97,4 @@ EXACT_FORWARD_SHAPES = [(1, 2, 1, 1), (1, 12, 12, 197), (1, 2, 2, 64), (1, 2, 2,
                         (1, 24, 24, 300), (1, 60, 60, 100), (1, 148, 148, 197), (1, 150, 75, 17)]
 TRAINING_SHAPES = [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321), (1, 7, 1, 70), (2, 8, 1, 200),
                    (5, 30, 30, 130), (1, 148, 74, 127), (1, 148, 74, 130), (2, 48, 48, 65)]
-TRAINING_SHAPES_LARGE = [(1, 660, 660, 130), (2, 148, 148, 257)]
+TRAINING_SHAPES_LARGE = [(1, 700, 700, 127), (2, 170, 170, 250)]

@@ -87,7 +87,7 @@ def test_exact_backward_forms_of_causal_calls():
     """Under a causal mask the 128-row kernels want more than four rounds of CTAs (200 heads of S=197: 297 us against 229
     with 64 rows; 96 heads of S=848: 1110 against 1230)."""
     rows = lambda *sizes: _abi.plan(_abi.PLAN_TRAIN_BACKWARD, *sizes, 64, True)[:2]
-    for heads, n in ((200, 197), (200, 256), (200, 300), (96, 500), (96, 700), (48, 848)):
+    for heads, n in ((200, 197), (200, 256), (200, 300), (96, 500), (96, 700), (48, 848), (352, 405)):
         assert rows(1, heads, heads, n) == [64, 64]
     for heads, n in ((96, 848), (200, 500), (200, 512)):
         assert rows(1, heads, heads, n) == [128, 128]
