@@ -94,7 +94,7 @@ def to_dev(a: np.ndarray):
 # ---- shapes (B, Hq, Hkv, S) that reach every form of the dispatch rules; tests/test_plans.py holds them to that ----
 EXACT_FORWARD_SHAPES = [(1, 2, 1, 1), (1, 12, 12, 197), (1, 2, 2, 64), (1, 2, 2, 65), (2, 74, 74, 130), (1, 148, 74, 257),
                         (1, 2, 2, 1100), (1, 60, 60, 17), (1, 30, 30, 50), (1, 96, 48, 17), (1, 40, 40, 65), (1, 30, 15, 257),
-                        (1, 24, 24, 300), (1, 60, 60, 100), (1, 148, 148, 197), (1, 150, 75, 17)]
+                        (1, 24, 24, 300), (1, 60, 60, 100), (1, 148, 148, 197), (1, 150, 75, 17), (1, 60, 30, 50)]
 TRAINING_SHAPES = [(1, 2, 1, 1), (1, 4, 2, 63), (1, 4, 2, 64), (1, 2, 2, 129), (1, 6, 2, 321), (1, 7, 1, 70), (2, 8, 1, 200),
                    (5, 30, 30, 130), (1, 148, 74, 127), (1, 148, 74, 130), (2, 48, 48, 65)]
 TRAINING_SHAPES_LARGE = [(1, 700, 700, 127), (2, 170, 170, 250)]
