@@ -80,6 +80,7 @@ def test_exact_forward_form_of_many_short_and_many_long_heads():
     for d in (64, 128):
         assert form(1, 200, 200, 50, d, True) == [64, 1]
     assert form(8, 32, 32, 2048, 64, False) == [128, 0]
+    assert form(16, 16, 16, 188, 128, False) == [64, 0]   # 174 us; the plain one 217
     assert form(1, 12, 12, 197, 64, False)[0] in (16, 20, 24)
 
 
